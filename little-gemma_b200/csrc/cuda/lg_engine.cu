@@ -89,6 +89,12 @@ WMat build_wmat(Engine *e, std::vector<const struct gguf_tensor *> parts, bool i
     W.ws = dalloc<uint2>(tiles * 8);
     if (W.fmt != LG_FMT_Q4_0) W.wd = dalloc<uint2>(tiles * 8);
     if (W.fmt == LG_FMT_I8M) W.wm = dalloc<uint4>(tiles * 8);
+    if (W.fmt <= LG_FMT_Q4_K) {                              // what the wide matmul's weight copies read
+        auto rows_map = [&](const void *p, int bytes) { return tiled_map(p, CU_TENSOR_MAP_DATA_TYPE_INT32, (long long)W.nkp * bytes / 4, W.n_row_tiles,
+                                                                         (long long)W.nkp * bytes, 2 * bytes / 4, 8, CU_TENSOR_MAP_SWIZZLE_NONE); };
+        W.tq = rows_map(W.wq, 512); W.ts = rows_map(W.ws, 64);
+        if (W.wd) W.td = rows_map(W.wd, 64);
+    }
     const int nsb = W.k / 32;
 
     // file bytes of one part on the device (dense parts: re-encoded as q8_0 first)
@@ -206,12 +212,8 @@ template <int FMT> void gemv_attr_f() {
     gemv_attr<2, 1, FMT, LG_EPI_GATE>(); gemv_attr<2, 2, FMT, LG_EPI_GATE>();
 }
 // Opt every kernel into large dynamic shared memory once, outside any stream capture.
-template <int NT, int FMT, int EPI> void pf_attr() {
-    LG_CHECK(cudaFuncSetAttribute(lg_pf_gemm_kernel<NT, FMT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pf_smem_bytes<NT, FMT>()));
-}
-template <int NT> void pf_attr_n() {
-    pf_attr<NT, LG_FMT_Q4_0, LG_PF_STORE>(); pf_attr<NT, LG_FMT_Q4_0, LG_PF_GEGLU>();
-    pf_attr<NT, LG_FMT_Q4_K, LG_PF_STORE>(); pf_attr<NT, LG_FMT_Q4_K, LG_PF_GEGLU>();
+template <int FMT, int EPI> void pf_attr() {
+    LG_CHECK(cudaFuncSetAttribute(lg_pf_gemm_kernel<FMT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, LG_PF_SMEM_MAX));
 }
 // cudaFuncSetAttribute applies to the current device only, so the opt-in is tracked per device.
 template <int HD> void attn_cluster_attr() {
@@ -231,7 +233,7 @@ void set_kernel_attributes() {
     LG_CHECK(cudaFuncSetAttribute(lg_attn_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATTN_SMEM_MAX));
     LG_CHECK(cudaFuncSetAttribute(lg_attn_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATTN_SMEM_MAX));
     attn_cluster_attr<64>(); attn_cluster_attr<128>(); attn_cluster_attr<256>(); attn_cluster_attr<512>();
-    pf_attr_n<64>(); pf_attr_n<128>(); pf_attr_n<256>();
+    pf_attr<LG_FMT_Q4_0, LG_PF_STORE>(); pf_attr<LG_FMT_Q4_0, LG_PF_GEGLU>(); pf_attr<LG_FMT_Q4_K, LG_PF_STORE>(); pf_attr<LG_FMT_Q4_K, LG_PF_GEGLU>();
     LG_CHECK(cudaFuncSetAttribute(lg_attn_deep_kernel<128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATTN_SMEM_MAX));
     LG_CHECK(cudaFuncSetAttribute(lg_attn_deep_kernel<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATTN_SMEM_MAX));
     LG_CHECK(cudaFuncSetAttribute(lg_attn_deep_kernel<256, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATTN_SMEM_MAX));
@@ -479,39 +481,35 @@ CUtensorMap kv_tensor_map(const __half *ptr, int kv_dim, int seq, int S) {
     return tiled_map(ptr, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, kv_dim, seq, (long long)kv_dim * 2, 64, S);
 }
 
-template <int NT, int FMT> void launch_pf_nt(Engine *e, const CUtensorMap &tm, const LgPfGemmArgs &a, int epi, dim3 grid) {
-    const size_t sm = pf_smem_bytes<NT, FMT>();
-    if (epi == LG_PF_GEGLU) launch_k(e, (lg_pf_gemm_kernel<NT, FMT, LG_PF_GEGLU>), grid, dim3(LG_PF_THREADS), sm, tm, a);
-    else launch_k(e, (lg_pf_gemm_kernel<NT, FMT, LG_PF_STORE>), grid, dim3(LG_PF_THREADS), sm, tm, a);
-}
-
-// out[tok][ldo] (f32) = W x X^T for n_tok <= 256 tokens; X is f16 [x_rows >= token tile][W.k], 16-byte aligned.
-// epi == LG_PF_GEGLU: W holds interleaved gate/up rows and act[tok][ld_act] (f16) receives gelu(gate)*up.
-// k slices of the wide matmul for a matrix with few rows (each slice writes its own plane of `out`)
-int pf_kslices(const Engine *e, const WMat &W, int max_ks) {
-    const int ctas = (W.n_row_tiles + 7) / 8;
+// The tokens of a block are shared out evenly over the fewest tiles of at most 256 (a multiple of 16 each: N of the multiply).
+int pf_token_tiles(int n_tok) { return (n_tok + LG_PF_NT - 1) / LG_PF_NT; }
+// k slices of the wide matmul for a matrix with few rows (each slice writes its own plane of `out`): doubled while all slices'
+// items still fit the SMs once and a slice keeps 8 k blocks.  All planes together stay within LG_PF_MAXN rows.
+int pf_kslices(const Engine *e, const WMat &W, int n_tok, int max_ks) {
+    const int items = (W.n_row_tiles + 7) / 8 * pf_token_tiles(n_tok);
     int ks = 1;
-    while (ks < max_ks && ctas * ks * 2 <= e->sm_count && W.nkp / (ks * 2) >= 8) ks *= 2;
+    while (ks < max_ks && items * ks * 2 <= e->sm_count && W.nkp / (ks * 2) >= 8 && ks * 2 * n_tok <= LG_PF_MAXN) ks *= 2;
     return ks;
 }
 
+// out[tok][ldo] (f32) = W x X^T for n_tok <= LG_PF_MAXN tokens; X is f16 [x_rows][W.k], 16-byte aligned.
+// epi == LG_PF_GEGLU: W holds interleaved gate/up rows and act[tok][ld_act] (f16) receives gelu(gate)*up.
 void launch_pf_gemm(Engine *e, const WMat &W, const __half *X, int x_rows, int n_tok, float *out, __half *act, int ld_act, int epi,
                     int ks = 1) {
-    if (n_tok < 1 || n_tok > LG_PF_MAXN) { fprintf(stderr, "lg_b200: wide matmul takes 1..%d tokens\n", LG_PF_MAXN); exit(1); }
-    const int nt = n_tok > 128 ? 256 : n_tok > 64 ? 128 : 64;
-    if (x_rows < nt) { fprintf(stderr, "lg_b200: activation block of %d rows is smaller than the token tile %d\n", x_rows, nt); exit(1); }
-    CUtensorMap tm = act_tensor_map(X, W.k, x_rows, nt);
+    if (n_tok < 1 || n_tok > LG_PF_MAXN || n_tok > x_rows) { fprintf(stderr, "lg_b200: wide matmul takes 1..%d tokens\n", std::min(LG_PF_MAXN, x_rows)); exit(1); }
     LgPfGemmArgs a{};
-    a.wq = W.wq; a.ws = W.ws; a.wd = W.wd; a.nkp = W.nkp; a.n_row_tiles = W.n_row_tiles; a.n_tok = n_tok;
+    a.tok_tiles = pf_token_tiles(n_tok);
+    a.nt = ((n_tok + a.tok_tiles - 1) / a.tok_tiles + 15) & ~15;
+    CUtensorMap tm = act_tensor_map(X, W.k, x_rows, a.nt);
+    a.nkp = W.nkp; a.n_row_tiles = W.n_row_tiles; a.n_tok = n_tok;
     a.out = out; a.ldo = W.ldo; a.n_rows = W.ldo; a.act = act; a.ld_act = ld_act; a.err = e->err;
-    a.part_stride = (size_t)LG_PF_MAXN * W.ldo;
-    dim3 grid((W.n_row_tiles + 7) / 8, 1, epi == LG_PF_GEGLU ? 1 : ks);
-    const bool k4 = W.fmt == LG_FMT_Q4_K;
-    switch (nt) {
-    case 64:  if (k4) launch_pf_nt<64, LG_FMT_Q4_K>(e, tm, a, epi, grid); else launch_pf_nt<64, LG_FMT_Q4_0>(e, tm, a, epi, grid); break;
-    case 128: if (k4) launch_pf_nt<128, LG_FMT_Q4_K>(e, tm, a, epi, grid); else launch_pf_nt<128, LG_FMT_Q4_0>(e, tm, a, epi, grid); break;
-    default:  if (k4) launch_pf_nt<256, LG_FMT_Q4_K>(e, tm, a, epi, grid); else launch_pf_nt<256, LG_FMT_Q4_0>(e, tm, a, epi, grid); break;
-    }
+    a.kslices = epi == LG_PF_GEGLU ? 1 : ks; a.part_stride = (size_t)n_tok * W.ldo;
+    a.rs = pf_raw_stages(a.nt, W.fmt);
+    const dim3 grid(std::min(e->sm_count, (W.n_row_tiles + 7) / 8 * a.tok_tiles * a.kslices));
+    const size_t sm = pf_smem_bytes(a.nt, W.fmt);
+    auto *kernel = W.fmt == LG_FMT_Q4_K ? (epi == LG_PF_GEGLU ? lg_pf_gemm_kernel<LG_FMT_Q4_K, LG_PF_GEGLU> : lg_pf_gemm_kernel<LG_FMT_Q4_K, LG_PF_STORE>)
+                                        : (epi == LG_PF_GEGLU ? lg_pf_gemm_kernel<LG_FMT_Q4_0, LG_PF_GEGLU> : lg_pf_gemm_kernel<LG_FMT_Q4_0, LG_PF_STORE>);
+    launch_k(e, kernel, grid, dim3(LG_PF_THREADS), sm, tm, W.tq, W.ts, W.td, a);
 }
 
 void launch_attn(Engine *e, LgAttnArgs a, int n_tiles_max) {
@@ -1037,8 +1035,8 @@ void prefill_alloc(Engine *e) {
     b.a_attn = dalloc<__half>((size_t)LG_PF_MAXN * max_attn);
     b.a_ff = dalloc<__half>((size_t)LG_PF_MAXN * max_ff);
     b.x = dalloc<float>((size_t)LG_PF_MAXN * ne);
-    b.qkv = dalloc<float>((size_t)PF_MAX_KS * LG_PF_MAXN * max_qkv);
-    b.o = dalloc<float>((size_t)PF_MAX_KS * LG_PF_MAXN * max_o);
+    b.qkv = dalloc<float>((size_t)LG_PF_MAXN * max_qkv);
+    b.o = dalloc<float>((size_t)LG_PF_MAXN * max_o);
     b.toks = dalloc<int>(LG_PF_MAXN);
     b.pos = dalloc<int>(LG_PF_MAXN / LG_MAXM);
     b.rope_local = dalloc<float2>((size_t)LG_PF_MAXN * max_hd / 2);
@@ -1062,7 +1060,7 @@ void prefill_alloc(Engine *e) {
 void launch_norm_pf(Engine *e, int n_tok, float *x, int n, float eps, const float *add, int n_parts, int ld_add, const float *add_w,
                     float out_scale, const float *norm_w, __half *yh, bool row_itself = false) {
     LgNormArgs a{};
-    a.x = x; a.ldx = n; a.add_src = add; a.n_parts = n_parts; a.part_stride = (size_t)LG_PF_MAXN * ld_add; a.ld_add = ld_add; a.add_w = add_w; a.out_scale = out_scale;
+    a.x = x; a.ldx = n; a.add_src = add; a.n_parts = n_parts; a.part_stride = (size_t)n_tok * ld_add; a.ld_add = ld_add; a.add_w = add_w; a.out_scale = out_scale;
     a.norm_w = norm_w; a.n = n; a.eps = eps; a.yh = (norm_w || row_itself) ? yh : nullptr; a.ldyh = n;   // row_itself: the f16 row is x, not a norm of it
     int threads = n >= 2048 ? 1024 : (n >= 512 ? 512 : 256);
     launch_k(e, lg_norm_kernel, dim3(n_tok), dim3(threads), (size_t)(2 * n + 32) * 4, a);
@@ -1102,12 +1100,12 @@ void enqueue_prefill_block(Engine *e, const struct kvcache *kv, int n, int only 
         const int gqa = H / w.nkv;
         static const int block_attn = env_int("LG_PREFILL_BLOCK_ATTN", 1);
         const bool whole = block_attn && (hd == 64 || hd == 128 || hd == 256) && LG_PFA_Q % gqa == 0;
-        const int ks_q = whole ? pf_kslices(e, w.qkv, 2) : 1, ks_o = pf_kslices(e, w.o, PF_MAX_KS), ks_d = pf_kslices(e, w.down, PF_MAX_KS);
+        const int ks_q = whole ? pf_kslices(e, w.qkv, n, 2) : 1, ks_o = pf_kslices(e, w.o, n, PF_MAX_KS), ks_d = pf_kslices(e, w.down, n, PF_MAX_KS);
         if (only & C_QKV) launch_pf_gemm(e, w.qkv, b.a_ne, LG_PF_MAXN, n, b.qkv, nullptr, 0, LG_PF_STORE, ks_q);
         if ((only & C_ATTN) && whole) {
             // the whole block at once: rows to the cache + f16 queries, then the tiled online-softmax kernel
             LgPfPrepArgs pa{};
-            pa.qkv = b.qkv; pa.ld = w.qkv.ldo; pa.n_parts = ks_q; pa.part_stride = (size_t)LG_PF_MAXN * w.qkv.ldo; pa.has_v = w.has_v; pa.owns_kv = w.owns_kv; pa.q_norm = w.q_norm; pa.k_norm = w.k_norm;
+            pa.qkv = b.qkv; pa.ld = w.qkv.ldo; pa.n_parts = ks_q; pa.part_stride = (size_t)n * w.qkv.ldo; pa.has_v = w.has_v; pa.owns_kv = w.owns_kv; pa.q_norm = w.q_norm; pa.k_norm = w.k_norm;
             pa.eps = c->rms_eps; pa.rope = w.local ? b.rope_local : b.rope_global;
             pa.kc = (__half *)kv->k[src]; pa.vc = (__half *)kv->v[src]; pa.seq = kv->seq[src]; pa.kv_dim = kv->kv_dim[src];
             pa.H = H; pa.Hkv = w.nkv; pa.pos = b.pos; pa.q_hi = b.q_hi; pa.q_lo = b.q_lo;
@@ -1978,7 +1976,7 @@ int lg_bench_prefill_pass(struct model *m, int n, int classes) {
         if (n < 1 || !e->kv_bound || e->fam->bench_block(e, e->kv_bound, n, 0, classes) != 0) return -1;
         return (int)(e->launches - before);
     }
-    if (n < 1 || n > LG_PF_MAXN || !e->kv_bound || !prefill_wide_ok(e)) return -1;
+    if (n < 1 || n > LG_PF_OP_MAXN || !e->kv_bound || !prefill_wide_ok(e)) return -1;
     prefill_alloc(e);
     enqueue_prefill_block(e, e->kv_bound, n, classes);
     return (int)(e->launches - before);

@@ -59,6 +59,7 @@ struct WMat {
     uint4 *wq = nullptr; uint2 *ws = nullptr; uint2 *wd = nullptr; uint4 *wm = nullptr;      // tiles, scales (see lg_kernels.cuh)
     int fmt = 0, m = 0, k = 0, nkp = 0, n_row_tiles = 0, ldo = 0;
     size_t file_bytes = 0;
+    CUtensorMap tq{}, ts{}, td{};             // q4 formats: wq / ws / wd as rows of tiles, boxes of 8 row tiles x 2 tile positions
 };
 
 struct Panel { LgPanel p{}; };
@@ -219,11 +220,12 @@ inline const struct gguf_tensor *find_t(const struct gguf_context *g, int L, con
 }
 inline int env_int(const char *name, int fb) { const char *v = getenv(name); return v && v[0] ? atoi(v) : fb; }
 
-// Descriptor of a row-major matrix [rows][cols] for tiled copies: boxes of box_c columns (one 128-byte swizzle row) x box_r rows.
+// Descriptor of a row-major matrix [rows][cols] for tiled copies: boxes of box_c columns (one 128-byte row where swizzled) x box_r rows.
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-inline CUtensorMap tiled_map(const void *ptr, CUtensorMapDataType type, long long cols, long long rows, long long row_bytes, int box_c, int box_r) {
+inline CUtensorMap tiled_map(const void *ptr, CUtensorMapDataType type, long long cols, long long rows, long long row_bytes, int box_c, int box_r,
+                             CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
     static EncodeTiledFn fn = nullptr;
     if (!fn) {
         void *p = nullptr;
@@ -238,7 +240,7 @@ inline CUtensorMap tiled_map(const void *ptr, CUtensorMapDataType type, long lon
     cuuint32_t box[2] = {(cuuint32_t)box_c, (cuuint32_t)box_r};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = fn(&map, type, 2, (void *)ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                    swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { fprintf(stderr, "lg_b200: cuTensorMapEncodeTiled failed (%d) for %lld x %lld\n", (int)r, rows, cols); exit(1); }
     return map;
 }

@@ -1,49 +1,59 @@
 // lg_prefill.cuh -- the wide (prompt) matmul on the 5th-generation tensor cores.
 //
-// out[tok][row] = sum_k W[row][k] * X[tok][k] for a block of up to 256 prompt tokens at once.
+// out[tok][row] = sum_k W[row][k] * X[tok][k] for a block of up to LG_PF_MAXN prompt tokens at once.
 // W is the same tile-major q4 matrix the decode step streams (16 rows x 64 columns per 512-byte
 // tile, nibbles stored as two's-complement q-8); X is an f16 row-major activation block.  The
 // weights are expanded to f16 on the fly -- d*(q-8) rounded once to f16, i.e. the f16 rounding of
-// the exact dequantised value -- so each weight byte leaves HBM once per token block and the
-// multiply-accumulate runs as tcgen05.mma (kind::f16, f32 accumulate in tensor memory).
+// the exact dequantised value -- and the multiply-accumulate runs as tcgen05.mma (kind::f16, f32 accumulate).
 //
-// One CTA owns 128 weight rows (8 row tiles = the 128 TMEM lanes) x NT tokens (TMEM columns) and
-// walks k in blocks of 64 (one tile position = one 128-byte swizzle row of f16):
-//   warp 8 (one thread)  streams the raw q4 tiles + scales of two k blocks per stage with bulk copies;
-//   warp 9 (one thread)  loads the X block [NT tokens x 64] with a tiled TMA copy (128-byte swizzle);
-//   warps 0-7            expand a raw k block to the f16 A operand [128 rows x 64] (one row tile per
-//                        warp) in the same swizzled K-major layout, then fence it to the async proxy;
-//   warp 10 (one thread) issues four tcgen05.mma (M=128, N=NT, K=16) per k block and commits the
-//                        stage back to the producers; after the last block it commits the accumulator;
-//   warps 0-7            read the accumulator with tcgen05.ld (lane quarter = warp % 4, column half =
-//                        warp / 4) and store f32 rows, or apply GeGLU on interleaved gate/up rows and
-//                        store the f16 input of the down projection.
-// blockIdx.z cuts k into slices whose partial sums go to separate planes of `out` (matrices with
-// few rows would otherwise fill a fraction of the SMs); the consumer adds the planes.
-// Every mbarrier wait is bounded; a timeout raises LG_ERR_MBAR_TIMEOUT, the CTA stops waiting,
-// drains its own copies, frees its tensor memory and returns.
+// Persistent: a CTA takes work items (128 weight rows x one token tile x one k slice) blockIdx.x, + gridDim.x, ...  Token
+// tiles are equal shares of the block (a.nt <= 256 tokens each, a multiple of 16), the items of one row block side by side,
+// so its weights leave HBM once and the other token tiles find them in L2.  Per step of two k blocks (128 columns):
+//   warp DQ     (one thread) streams the raw q4 tiles + scales, one tiled copy each (8 row tiles x 2 positions);
+//   warp DQ + 1 (one thread) loads the X block [nt tokens x 64] twice with tiled TMA copies (128-byte swizzle);
+//   warps 0..DQ-1 expand: three groups of four warps take the steps in turn, a warp the two row tiles of its 32 tensor-memory
+//               lanes, and write the f16 A operand straight into tensor memory.  A tile's lane order -- lane (g, t) holds columns
+//               4t..4t+3 and 16+4t..16+4t+3 of rows g and g+8 -- is the register order of tcgen05.st.16x256b: nothing is shuffled;
+//   warp DQ + 2 issues eight tcgen05.mma (M = 128, N = the tile's tokens, K = 16), A from tensor memory, B from shared memory,
+//               and commits the stage back to both producers;
+//   warps 0..DQ-1 then read the accumulator with tcgen05.ld (lane quarter = warp % 4, the columns shared out over the groups) and
+//               store f32 rows, or apply GeGLU on interleaved gate/up rows and store the f16 input of the down projection.
+// Tensor memory: columns [0, 256) accumulator, [256, 448) three A stages of 64 columns.
+// What bounds it: the issuing warp (0.32 us per k block of 128 rows x 240 tokens where the products alone take 0.25) and, per item,
+// the epilogue.  12B-class q4_0, 928 tokens in one block: gate/up + GeGLU 168 us (1305 TFLOP/s), down 76 (1432), o 29 (1010),
+// qkv 51 (1139).  Against A expanded into shared memory, one CTA per 128 rows x 256 tokens and 16 bulk copies per weight stage
+// (four launches): 355, 109, 109 (with k slices) and 96 us.  On the way: one copy per row tile instead of a tiled copy kept the copy thread
+// at 115 cycles a copy and every k block at 0.53 us whatever the tile; a barrier pair per k block and operand cost 0.10 us.
+// k slices leave their partial sums in separate planes of `out` (matrices with few rows would otherwise fill a fraction of the
+// SMs); the consumer adds the planes.
+// Every mbarrier wait is bounded; a timeout raises LG_ERR_MBAR_TIMEOUT, the role stops waiting, drains its own copies, and the
+// CTA frees its tensor memory and returns.
 #pragma once
 #include <cuda.h>
 #include "lg_kernels.cuh"
 
 #define LG_PF_BM 128
 #define LG_PF_BK 64
-#define LG_PF_A_STAGES 4        // expanded weight (A operand) stages: a multiple of LG_PF_GROUPS, so a stage belongs to ONE
-                                // expand group and its empty-barrier phases are observed in order by the same threads
-                                // (a parity wait cannot tell "two completions behind" from "done")
+#define LG_PF_NT 256            // most tokens of a tile (accumulator columns)
+#define LG_PF_GROUPS 3          // groups of four expand warps, on steps in turn
+#define LG_PF_STAGES 3          // operand stages (A in tensor memory, X in shared memory) behind one pair of barriers: one per group,
+                                // so that a stage's phases are observed in order by the same threads
 #define LG_PF_SMEM_MAX 232448   // 227 KB: the most dynamic shared memory a CTA can have
-#define LG_PF_DQ_WARPS 8
-#define LG_PF_GROUPS 4          // expand-warp groups working on different k blocks
+#define LG_PF_DQ_WARPS (4 * LG_PF_GROUPS)
 #define LG_PF_THREADS ((LG_PF_DQ_WARPS + 3) * 32)
-#define LG_PF_MAXN 256
+#define LG_PF_MAXN 1024         // tokens of a block: as many as a sliding-window ring has spare rows
+#define LG_PF_OP_MAXN 256       // tokens the kernel-level entry points take
+#define LG_PF_MAX_RAW 15
 
 enum { LG_PF_STORE = 0, LG_PF_GEGLU = 1 };
 
 struct LgPfGemmArgs {
-    const uint4 *wq; const uint2 *ws; const uint2 *wd;
     int nkp, n_row_tiles;
-    int n_tok;                  // valid tokens of the block (columns beyond are computed and dropped)
-    float *out; int ldo;        // STORE: out[slice][tok][ldo], slice = blockIdx.z
+    int n_tok;                  // valid tokens of the block
+    int nt, tok_tiles;          // tokens per tile (the X copy's box), tiles
+    int kslices;
+    int rs;                     // raw stages: a multiple of LG_PF_GROUPS
+    float *out; int ldo;        // STORE: out[slice][tok][ldo]
     size_t part_stride;         // floats between the planes of two k slices
     int n_rows;                 // rows >= n_rows are padding and are not stored
     __half *act; int ld_act;    // GEGLU: act[tok][ld_act], element j = gelu(gate_j) * up_j
@@ -51,23 +61,16 @@ struct LgPfGemmArgs {
 };
 
 // raw stage: 8 row tiles x 2 tile positions of nibbles, then their scales, then (q4_K) their {d,dmin}
-template <int FMT> __host__ __device__ constexpr int pf_raw_stage_bytes() {
-    return 8 * 2 * (512 + 64 + (FMT == LG_FMT_Q4_K ? 64 : 0));
+__host__ __device__ constexpr int pf_raw_stage_bytes(int fmt) { return 8 * 2 * (512 + 64 + (fmt == LG_FMT_Q4_K ? 64 : 0)); }
+// raw stages: as many as fit beside the X stages, at most 15 -- the bytes in flight from HBM per SM
+__host__ __device__ constexpr int pf_raw_stages(int nt, int fmt) {
+    const int n = (LG_PF_SMEM_MAX - 1024 - 512 - LG_PF_STAGES * nt * 256) / pf_raw_stage_bytes(fmt);
+    return (n > LG_PF_MAX_RAW ? LG_PF_MAX_RAW : n) / LG_PF_GROUPS * LG_PF_GROUPS;
 }
-template <int NT> __host__ __device__ constexpr int pf_a_stages() { return LG_PF_A_STAGES; }
-// activation (B operand) stages (3 stages with a deeper raw ring measured slower at a 256-wide token tile)
-template <int NT> __host__ __device__ constexpr int pf_b_stages() { return 4; }
-// raw q4 stages of two k blocks each: as many as fit beside the operand stages, at most 8 -- the bytes in flight
-// from HBM per SM, which is what keeps the weight stream moving
-template <int NT, int FMT> __host__ __device__ constexpr int pf_raw_stages() {
-    int left = LG_PF_SMEM_MAX - 1024 - 512 - pf_a_stages<NT>() * LG_PF_BM * 128 - pf_b_stages<NT>() * NT * 128;
-    int n = left / pf_raw_stage_bytes<FMT>();
-    return n > 8 ? 8 : n;
+__host__ __device__ constexpr size_t pf_smem_bytes(int nt, int fmt) {
+    return 1024 + (size_t)LG_PF_STAGES * nt * 256 + (size_t)pf_raw_stages(nt, fmt) * pf_raw_stage_bytes(fmt) + 512;
 }
-template <int NT, int FMT> __host__ __device__ constexpr size_t pf_smem_bytes() {
-    return 1024 + (size_t)pf_a_stages<NT>() * LG_PF_BM * 128 + (size_t)pf_b_stages<NT>() * NT * 128
-         + (size_t)pf_raw_stages<NT, FMT>() * pf_raw_stage_bytes<FMT>() + 512;
-}
+static_assert(pf_raw_stages(LG_PF_NT, LG_FMT_Q4_K) >= LG_PF_GROUPS, "a raw stage per group");
 
 // two stored nibbles (bytes b0,b1 of `n`, already q = stored ^ 8) -> half2 (q0-8, q1-8) * d
 __device__ __forceinline__ uint32_t pf_pair_q4_0(uint32_t n, uint32_t sel, __half2 d2) {
@@ -86,216 +89,250 @@ __device__ __forceinline__ uint32_t pf_pair_q4_K(uint32_t n, uint32_t sel, __hal
     return *(uint32_t *)&h;
 }
 
-template <int NT, int FMT, int EPI>
-__global__ void __launch_bounds__(LG_PF_THREADS) lg_pf_gemm_kernel(const __grid_constant__ CUtensorMap tmx, LgPfGemmArgs a) {
+// a CTA's work item `it`: token tiles fastest, then row blocks, then k slices
+struct PfItem { int rt0, tok0, n, slice, kb_lo, nkb; };
+__device__ __forceinline__ PfItem pf_item(const LgPfGemmArgs &a, int it) {
+    PfItem w;
+    const int tt = it % a.tok_tiles, rest = it / a.tok_tiles, row_blocks = (a.n_row_tiles + 7) >> 3;
+    w.rt0 = (rest % row_blocks) * 8; w.slice = rest / row_blocks;
+    w.tok0 = tt * a.nt; w.n = min(a.nt, a.n_tok - w.tok0);
+    w.kb_lo = (int)((long long)a.nkp * w.slice / a.kslices);
+    w.nkb = (int)((long long)a.nkp * (w.slice + 1) / a.kslices) - w.kb_lo;
+    return w;
+}
+// a ring position and the parity of the pass it is in
+struct PfRing {
+    int s = 0; uint32_t ph = 0;
+    __device__ __forceinline__ void next(int n) { if (++s == n) { s = 0; ph ^= 1; } }
+};
+
+template <int FMT, int EPI>
+__global__ void __launch_bounds__(LG_PF_THREADS, 1) lg_pf_gemm_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmq,
+                                                                       const __grid_constant__ CUtensorMap tms, const __grid_constant__ CUtensorMap tmd, LgPfGemmArgs a) {
     extern __shared__ unsigned char pf_smem_raw[];
-    constexpr int STA = pf_a_stages<NT>(), STB = pf_b_stages<NT>(), RS = pf_raw_stages<NT, FMT>(), RAW = pf_raw_stage_bytes<FMT>();
-    constexpr int A_BYTES = LG_PF_BM * 128, B_BYTES = NT * 128;
+    constexpr int ST = LG_PF_STAGES, NG = LG_PF_GROUPS, RAW = pf_raw_stage_bytes(FMT), DQ = LG_PF_DQ_WARPS;
+    static_assert(ST == NG, "a stage belongs to one expand group");
     constexpr int RAW_SC = 16 * 512, RAW_DD = RAW_SC + 16 * 64;
-    unsigned char *base = (unsigned char *)(((uintptr_t)pf_smem_raw + 1023) & ~(uintptr_t)1023);
-    unsigned char *sA = base, *sB = sA + STA * A_BYTES, *sRaw = sB + STB * B_BYTES;
+    const int RS = a.rs, B_BYTES = a.nt * 128;
+    unsigned char *sB = (unsigned char *)(((uintptr_t)pf_smem_raw + 1023) & ~(uintptr_t)1023), *sRaw = sB + ST * 2 * B_BYTES;
     uint64_t *bars = (uint64_t *)(sRaw + RS * RAW);
-    static_assert(STA == STB, "an operand stage is one A tile and one B tile behind the same pair of barriers");
-    // full[s]: the expand group's arrivals + the activation copy's bytes; empty[s]: one commit frees both tiles
-    uint64_t *raw_full = bars, *raw_empty = raw_full + RS, *full = raw_empty + RS, *empty = full + STA, *acc_full = empty + STA;
-    uint32_t *tmem_slot = (uint32_t *)(acc_full + 1);
+    // full[s]: the group's four warps + the bytes of the X copies; empty[s]: one commit frees both operands
+    uint64_t *raw_full = bars, *raw_empty = raw_full + RS, *full = raw_empty + RS, *empty = full + ST, *acc_full = empty + ST, *acc_empty = acc_full + 1;
+    uint32_t *tmem_slot = (uint32_t *)(acc_empty + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rt0 = blockIdx.x * 8, tok0 = blockIdx.y * NT;
-    const int kb_lo = (int)((long long)a.nkp * blockIdx.z / gridDim.z), kb_hi = (int)((long long)a.nkp * (blockIdx.z + 1) / gridDim.z);
-    const int nkb = kb_hi - kb_lo, n_raw = (nkb + 1) >> 1;     // this CTA's k blocks: kb_lo + [0, nkb)
-    constexpr int DQT = LG_PF_DQ_WARPS * 32;
+    const int n_items = ((a.n_row_tiles + 7) >> 3) * a.tok_tiles * a.kslices;
 
-    pdl_launch();
     if (threadIdx.x == 0) {
-        for (int i = 0; i < RS; i++) { mbar_init(raw_full + i, 1); mbar_init(raw_empty + i, 2 * DQT / LG_PF_GROUPS); }
-        for (int i = 0; i < STA; i++) { mbar_init(full + i, DQT / LG_PF_GROUPS + 1); mbar_init(empty + i, 1); }
-        mbar_init(acc_full, 1);
+        for (int i = 0; i < RS; i++) { mbar_init(raw_full + i, 1); mbar_init(raw_empty + i, 4); }
+        for (int i = 0; i < ST; i++) { mbar_init(full + i, 5); mbar_init(empty + i, 1); }
+        mbar_init(acc_full, 1); mbar_init(acc_empty, DQ);
     }
-    if (warp == LG_PF_DQ_WARPS + 2) {        // tensor memory: NT f32 columns x 128 lanes
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(tmem_slot)), "r"(NT) : "memory");
+    if (warp == DQ + 2) {        // tensor memory: 256 accumulator columns, 3 x 64 columns of weights
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(tmem_slot)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = *tmem_slot, tmem_a = tmem + LG_PF_NT;
+    pdl_launch();                // only now: a dependant must not take tensor memory a CTA of this grid still waits for
 
-    if (warp == LG_PF_DQ_WARPS) {
+    if (warp == DQ) {
         // ---------------- raw weight producer ----------------
         if (lane == 0) {
             bool ok = true;
+            PfRing q;
             int issued = 0;
-            for (int r = 0; r < n_raw && ok; r++) {
-                const int rs = r % RS;
-                if (r >= RS && !mbar_wait(raw_empty + rs, ((r / RS) & 1) ^ 1)) { atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 2); ok = false; break; }
-                const int np = min(2, nkb - 2 * r);
-                unsigned char *st = sRaw + rs * RAW;
-                mbar_expect_tx(raw_full + rs, 8u * np * (512 + 64 + (FMT == LG_FMT_Q4_K ? 64 : 0)));
-                #pragma unroll
-                for (int ti = 0; ti < 8; ti++) {
-                    const int rt = min(rt0 + ti, a.n_row_tiles - 1);
-                    const size_t tile = (size_t)rt * a.nkp + kb_lo + 2 * r;
-                    bulk_g2s(st + ti * 1024, a.wq + tile * 32, np * 512, raw_full + rs);
-                    bulk_g2s(st + RAW_SC + ti * 128, a.ws + tile * 8, np * 64, raw_full + rs);
-                    if (FMT == LG_FMT_Q4_K) bulk_g2s(st + RAW_DD + ti * 128, a.wd + tile * 8, np * 64, raw_full + rs);
+            for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
+                const PfItem w = pf_item(a, it);
+                for (int k = 0; k < w.nkb; k += 2) {
+                    if (issued >= RS && !mbar_wait(raw_empty + q.s, q.ph ^ 1)) { atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 2); ok = false; break; }
+                    // boxes of 8 row tiles x 2 positions; what lies past the matrix arrives as zeros, what lies past the slice unused
+                    unsigned char *st = sRaw + q.s * RAW;
+                    mbar_expect_tx(raw_full + q.s, RAW);
+                    tma_load_2d(st, &tmq, (w.kb_lo + k) * 128, w.rt0, raw_full + q.s);
+                    tma_load_2d(st + RAW_SC, &tms, (w.kb_lo + k) * 16, w.rt0, raw_full + q.s);
+                    if (FMT == LG_FMT_Q4_K) tma_load_2d(st + RAW_DD, &tmd, (w.kb_lo + k) * 16, w.rt0, raw_full + q.s);
+                    issued++;
+                    q.next(RS);
                 }
-                issued = r + 1;
             }
             if (!ok)      // drain: the copies already issued must land before the CTA's shared memory is released
                 for (int r = max(0, issued - RS); r < issued; r++) mbar_wait(raw_full + r % RS, (r / RS) & 1);
         }
-    } else if (warp == LG_PF_DQ_WARPS + 1) {
+    } else if (warp == DQ + 1) {
         // ---------------- activation producer ----------------
         if (lane == 0) {
             pdl_wait();
             bool ok = true;
+            PfRing q;
             int issued = 0;
-            for (int kb = 0; kb < nkb && ok; kb++) {
-                const int s = kb % STB;
-                if (kb >= STB && !mbar_wait(empty + s, ((kb / STB) & 1) ^ 1)) { atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 4); ok = false; break; }
-                mbar_expect_tx(full + s, B_BYTES);
-                tma_load_2d(sB + s * B_BYTES, &tmx, (kb_lo + kb) * LG_PF_BK, tok0, full + s);
-                issued = kb + 1;
-            }
-            if (!ok)
-                for (int kb = max(0, issued - STB); kb < issued; kb++) mbar_wait(full + kb % STB, (kb / STB) & 1);
-        }
-    } else if (warp == LG_PF_DQ_WARPS + 2) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(LG_PF_BM >> 4) << 24);
-            // This one thread is the pipeline's pacemaker: everything it does per k block is a serial chain of dependent
-            // instructions, so the loop is unrolled over the stages (static stage index: descriptors and barrier
-            // addresses live in registers) and carries as little arithmetic as possible.
-            uint64_t adesc[STA], bdesc[STB];
-            uint32_t ufull[STA], uempty[STA];
-            #pragma unroll
-            for (int st = 0; st < STA; st++) {
-                adesc[st] = umma_desc_k128(smem_u32(sA + st * A_BYTES)); bdesc[st] = umma_desc_k128(smem_u32(sB + st * B_BYTES));
-                ufull[st] = smem_u32(full + st); uempty[st] = smem_u32(empty + st);
-            }
-            bool ok = true;
-            uint32_t ph = 0, acc = 0;
-            for (int kb0 = 0; kb0 < nkb && ok; kb0 += STA, ph ^= 1) {
-                #pragma unroll
-                for (int st = 0; st < STA; st++) {
-                    if (kb0 + st >= nkb || !ok) break;
-                    if (!mbar_wait_u32(ufull[st], ph)) { atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 8); ok = false; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    #pragma unroll
-                    for (int j = 0; j < LG_PF_BK / 16; j++) { umma_f16(tmem, adesc[st] + 2 * j, bdesc[st] + 2 * j, idesc, acc); acc = 1u; }
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(uempty[st]) : "memory");
+            for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
+                const PfItem w = pf_item(a, it);
+                for (int k = 0; k < w.nkb; k += 2) {
+                    if (issued >= ST && !mbar_wait(empty + q.s, q.ph ^ 1)) { atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 4); ok = false; break; }
+                    const int np = min(2, w.nkb - k);
+                    mbar_expect_tx(full + q.s, np * B_BYTES);
+                    for (int h = 0; h < np; h++)
+                        tma_load_2d(sB + (2 * q.s + h) * B_BYTES, &tmx, (w.kb_lo + k + h) * LG_PF_BK, w.tok0, full + q.s);
+                    issued++;
+                    q.next(ST);
                 }
             }
-            umma_commit(acc_full);                   // arrives when every MMA above has completed
+            if (!ok)      // drain; the group's warps may never arrive: the waits are bounded, and far longer than any copy
+                for (int r = max(0, issued - ST); r < issued; r++) mbar_wait(full + r % ST, (r / ST) & 1);
+        }
+    } else if (warp == DQ + 2) {
+        // ---------------- MMA issuer ----------------
+        // The whole warp walks the loop and one elected thread issues (a lane-0 branch around the loop cost 10 %).  It never waits
+        // in a long item: what it does between two steps' products bounds the kernel (a wait that is over costs about 100
+        // cycles, a step's products 1024), so the next step's barrier is looked at before this step's products are issued.
+        bool ok = true, ready = false;
+        PfRing q;
+        uint32_t aph = 0;                            // parity of the accumulator's next release
+        const uint64_t bdesc0 = umma_desc_k128(smem_u32(sB));
+        const uint32_t bstep = (uint32_t)B_BYTES >> 4;
+        for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
+            const PfItem w = pf_item(a, it);
+            const uint32_t idesc = (1u << 4) | ((uint32_t)((w.n + 15) >> 4) << 18) | ((uint32_t)(LG_PF_BM >> 4) << 24);
+            if (it != (int)blockIdx.x) {
+                ok = mbar_wait(acc_empty, aph);
+                aph ^= 1;
+            }
+            for (int k = 0; k < w.nkb; k += 2) {
+                if (ok && !ready) ok = mbar_wait(full + q.s, q.ph);
+                if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t ad = tmem_a + q.s * 64, done = smem_u32(empty + q.s);
+                const uint64_t bd = bdesc0 + 2 * q.s * bstep;
+                q.next(ST);
+                ready = mbar_test(full + q.s, q.ph);
+                if (elect_one()) {
+                    #pragma unroll
+                    for (int j = 0; j < 4; j++) umma_f16_ta(tmem, ad + 8 * j, bd + 2 * j, idesc, k | j);
+                    if (k + 1 < w.nkb) {
+                        #pragma unroll
+                        for (int j = 0; j < 4; j++) umma_f16_ta(tmem, ad + 32 + 8 * j, bd + bstep + 2 * j, idesc, 1);
+                    }
+                    umma_commit_u32(done);
+                }
+                __syncwarp();
+            }
+            if (!ok && lane == 0) atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 8);
+            if (elect_one()) umma_commit(acc_full);  // arrives when every MMA above has completed
+            __syncwarp();
         }
     } else {
-        // ---------------- expand q4 -> f16 A operand (one row tile per warp), then the epilogue ----------------
-        // The expand warps form LG_PF_GROUPS groups; group gi takes the k blocks kb = gi (mod LG_PF_GROUPS), so
-        // several k blocks are being expanded at once and a group's latency chain (wait, expand, proxy fence,
-        // arrive) overlaps the other groups'.  Within a group the warps split the 8 row tiles.
-        // All shared-memory traffic of this loop uses explicit shared-space addresses (32-bit).
-        constexpr int NG = LG_PF_GROUPS, WPG = LG_PF_DQ_WARPS / NG, TPW = 8 / WPG;   // warps per group, tiles per warp
-        static_assert(STA % NG == 0, "a stage must belong to one expand group");
-        const int g = lane >> 2, t = lane & 3;
-        const int gi = warp / WPG, wi = warp % WPG;
+        // ---------------- expand q4 -> f16 A operand in tensor memory, then the epilogue ----------------
+        const int g = lane >> 2, lq = warp & 3, grp = warp >> 2;        // lane quarter, expand group
         const uint32_t raw0 = smem_u32(sRaw) + lane * 16;
         const uint32_t rsc0 = smem_u32(sRaw) + RAW_SC + g * 8, rdd0 = smem_u32(sRaw) + RAW_DD + g * 8;
-        // row ti*16 + g (+8): 8-row group (2 ti) (+1), row-in-group g; 16-byte chunk c of a row sits at c ^ g
-        const uint32_t dst0 = smem_u32(sA) + g * 128 + (t & 1) * 8;
-        uint32_t coff[4];                                                            // [sub-block][low / high nibbles]
-        #pragma unroll
-        for (int i = 0; i < 4; i++) coff[i] = (uint32_t)(((4 * (i >> 1) + (t >> 1) + 2 * (i & 1)) ^ g) << 4);
+        const uint32_t lanes = (uint32_t)(lq * 32) << 16;
         bool ok = true;
-        for (int kb = gi; kb < nkb; kb += NG) {
-            const int s = kb % STA, r = kb >> 1, rs = r % RS, half = kb & 1;
-            if (ok && !mbar_wait(raw_full + rs, (r / RS) & 1)) { ok = false; atomicOr(a.err, 32); }
-            if (ok && kb >= STA && !mbar_wait(empty + s, ((kb / STA) & 1) ^ 1)) { ok = false; atomicOr(a.err, 64); }
-            if (!ok) break;
-            #pragma unroll
-            for (int q = 0; q < TPW; q++) {
-                const int ti = wi * TPW + q;                                         // row tile of the CTA's 8
-                const uint32_t roff = rs * RAW + ti * 1024 + half * 512, soff = rs * RAW + ti * 128 + half * 64;
-                uint4 w; uint2 sc, dd = make_uint2(0, 0);
-                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "r"(raw0 + roff));
-                asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(sc.x), "=r"(sc.y) : "r"(rsc0 + soff));
-                if (FMT == LG_FMT_Q4_K) asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(dd.x), "=r"(dd.y) : "r"(rdd0 + soff));
-                const uint32_t dstS = dst0 + s * A_BYTES + (2 * ti) * 1024;
+        int step = 0;                                // steps of the items before this one and of this one so far
+        int rs = grp; uint32_t rph = 0, sph = 1;     // this group's raw stage and its parity; parity of the operand stage's release
+        uint32_t cph = 0;
+        for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
+            const PfItem w = pf_item(a, it);
+            for (int k = 0; k < w.nkb; k += 2, step++) {
+                if (step % NG != grp) continue;
+                const int np = min(2, w.nkb - k);
+                if (!mbar_wait(raw_full + rs, rph)) { ok = false; atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 32); }
+                if (ok && step >= ST && !mbar_wait(empty + grp, sph)) { ok = false; atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 64); }
+                sph ^= 1;
+                if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 #pragma unroll
-                for (int sbk = 0; sbk < 2; sbk++)
+                for (int h = 0; h < 2; h++) {
+                    if (h >= np) break;
                     #pragma unroll
-                    for (int h8 = 0; h8 < 2; h8++) {
-                        const uint32_t word = sbk ? (h8 ? w.w : w.z) : (h8 ? w.y : w.x);
-                        const uint32_t sw = sbk ? sc.y : sc.x;
-                        const uint32_t lo = (word & 0x0F0F0F0Fu) ^ 0x08080808u, hi = ((word >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;
-                        uint2 vlo, vhi;
-                        if (FMT == LG_FMT_Q4_0) {
-                            uint32_t dbits;                                           // the row's scale in both halves
-                            asm("prmt.b32 %0, %1, %1, %2;" : "=r"(dbits) : "r"(sw), "r"(h8 ? 0x3232u : 0x1010u));
-                            const __half2 d2 = *(const __half2 *)&dbits;
-                            vlo = make_uint2(pf_pair_q4_0(lo, 0x4140u, d2), pf_pair_q4_0(lo, 0x4342u, d2));
-                            vhi = make_uint2(pf_pair_q4_0(hi, 0x4140u, d2), pf_pair_q4_0(hi, 0x4342u, d2));
-                        } else {
-                            const uint32_t sm = h8 ? (sw >> 16) : (sw & 0xffff);
-                            const float2 dm = __half22float2(*(const __half2 *)(h8 ? &dd.y : &dd.x));
-                            const __half2 dsc2 = __float2half2_rn(dm.x * (float)(sm & 0xff));
-                            const __half2 ndm2 = __float2half2_rn(-dm.y * (float)(sm >> 8));
-                            vlo = make_uint2(pf_pair_q4_K(lo, 0x4140u, dsc2, ndm2), pf_pair_q4_K(lo, 0x4342u, dsc2, ndm2));
-                            vhi = make_uint2(pf_pair_q4_K(hi, 0x4140u, dsc2, ndm2), pf_pair_q4_K(hi, 0x4342u, dsc2, ndm2));
-                        }
-                        const uint32_t rowa = dstS + h8 * 1024;
-                        asm volatile("st.shared.v2.u32 [%0], {%1,%2};" :: "r"(rowa + coff[2 * sbk]), "r"(vlo.x), "r"(vlo.y) : "memory");
-                        asm volatile("st.shared.v2.u32 [%0], {%1,%2};" :: "r"(rowa + coff[2 * sbk + 1]), "r"(vhi.x), "r"(vhi.y) : "memory");
+                    for (int j = 0; j < 2; j++) {
+                        const int ti = lq * 2 + j;                                         // row tile of the CTA's 8
+                        const uint32_t roff = rs * RAW + ti * 1024 + h * 512, soff = rs * RAW + ti * 128 + h * 64;
+                        uint4 wv; uint2 sc, dd = make_uint2(0, 0);
+                        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(wv.x), "=r"(wv.y), "=r"(wv.z), "=r"(wv.w) : "r"(raw0 + roff));
+                        asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(sc.x), "=r"(sc.y) : "r"(rsc0 + soff));
+                        if (FMT == LG_FMT_Q4_K) asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(dd.x), "=r"(dd.y) : "r"(rdd0 + soff));
+                        uint32_t v[16];                                                    // [16 columns][row g: 2, row g + 8: 2]
+                        #pragma unroll
+                        for (int sbk = 0; sbk < 2; sbk++)
+                            #pragma unroll
+                            for (int h8 = 0; h8 < 2; h8++) {
+                                const uint32_t word = sbk ? (h8 ? wv.w : wv.z) : (h8 ? wv.y : wv.x);
+                                const uint32_t sw = sbk ? sc.y : sc.x;
+                                const uint32_t lo = (word & 0x0F0F0F0Fu) ^ 0x08080808u, hi = ((word >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;
+                                uint32_t *vl = v + 8 * sbk + 2 * h8, *vh = vl + 4;
+                                if (FMT == LG_FMT_Q4_0) {
+                                    uint32_t dbits;                                        // the row's scale in both halves
+                                    asm("prmt.b32 %0, %1, %1, %2;" : "=r"(dbits) : "r"(sw), "r"(h8 ? 0x3232u : 0x1010u));
+                                    const __half2 d2 = *(const __half2 *)&dbits;
+                                    vl[0] = pf_pair_q4_0(lo, 0x4140u, d2); vl[1] = pf_pair_q4_0(lo, 0x4342u, d2);
+                                    vh[0] = pf_pair_q4_0(hi, 0x4140u, d2); vh[1] = pf_pair_q4_0(hi, 0x4342u, d2);
+                                } else {
+                                    const uint32_t sm = h8 ? (sw >> 16) : (sw & 0xffff);
+                                    const float2 dm = __half22float2(*(const __half2 *)(h8 ? &dd.y : &dd.x));
+                                    const __half2 dsc2 = __float2half2_rn(dm.x * (float)(sm & 0xff));
+                                    const __half2 ndm2 = __float2half2_rn(-dm.y * (float)(sm >> 8));
+                                    vl[0] = pf_pair_q4_K(lo, 0x4140u, dsc2, ndm2); vl[1] = pf_pair_q4_K(lo, 0x4342u, dsc2, ndm2);
+                                    vh[0] = pf_pair_q4_K(hi, 0x4140u, dsc2, ndm2); vh[1] = pf_pair_q4_K(hi, 0x4342u, dsc2, ndm2);
+                                }
+                            }
+                        tmem_st_16x256b_x4(tmem_a + grp * 64 + h * 32 + lanes + ((uint32_t)j << 20), v);
                     }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(raw_empty + rs);
+                tmem_wait_st();
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full + grp);
+                rs += NG;
+                if (rs >= RS) { rs = grp; rph ^= 1; }
             }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");           // generic-proxy stores -> visible to the MMA
-            mbar_arrive(full + s);
-            mbar_arrive(raw_empty + rs);           // every expand thread arrives once per k block it takes
-        }
-        if (!ok && lane == 0) atomicOr(a.err, LG_ERR_MBAR_TIMEOUT);
 
-        // ---------------- epilogue: lane l of warp w holds accumulator row 32 (w % 4) + l ----------------
-        if (ok) { ok = mbar_wait(acc_full, 0); if (!ok) atomicOr(a.err, 128); }
-        if (!ok && lane == 0) atomicOr(a.err, LG_ERR_MBAR_TIMEOUT);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (ok) {
-            const int lq = warp & 3, ch = warp >> 2;                     // TMEM lane quarter, column half
-            const int lrow = lq * 32 + lane;                            // row within the CTA's 128
-            const int rt = rt0 + (lrow >> 4);
-            float *outp = a.out + (size_t)blockIdx.z * a.part_stride;
-            for (int c0 = ch * (NT / 2); c0 < (ch + 1) * (NT / 2); c0 += 32) {
-                if (tok0 + c0 >= a.n_tok) break;                          // uniform per CTA
+            // ---------------- epilogue: lane l of warp w holds accumulator row 32 (w % 4) + l ----------------
+            if (ok && !mbar_wait(acc_full, cph)) { ok = false; atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 128); }
+            cph ^= 1;
+            if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int lrow = lq * 32 + lane, rt = w.rt0 + (lrow >> 4);       // row within the CTA's 128
+            float *outp = a.out + (size_t)w.slice * a.part_stride + (size_t)w.tok0 * a.ldo + w.rt0 * 16 + lrow;
+            const bool row_ok = rt < a.n_row_tiles && w.rt0 * 16 + lrow < a.n_rows;
+            for (int c0 = grp * 32; c0 < w.n; c0 += NG * 32) {               // uniform per warp
                 uint32_t v[32];
-                tmem_ld32(tmem + ((uint32_t)(lq * 32) << 16) + c0, v);
+                tmem_ld32(tmem + lanes + c0, v);
                 if (EPI == LG_PF_STORE) {
-                    const int row = rt0 * 16 + lrow;
-                    if (rt < a.n_row_tiles && row < a.n_rows) {
+                    if (row_ok) {
                         #pragma unroll
                         for (int j = 0; j < 32; j++)
-                            if (tok0 + c0 + j < a.n_tok) outp[(size_t)(tok0 + c0 + j) * a.ldo + row] = __uint_as_float(v[j]);
+                            if (c0 + j < w.n) outp[(size_t)(c0 + j) * a.ldo] = __uint_as_float(v[j]);
                     }
                 } else {
-                    // tile rows 0-7 are gate rows, rows 8-15 the matching up rows: lane l pairs with lane l+8
-                    const int r16 = lrow & 15;
+                    // tile rows 0-7 are gate rows, rows 8-15 the matching up rows: lane l pairs with lane l + 8.  Of two tokens
+                    // the gate lane takes the even one and the up lane the odd one: one exchange, one GeLU and one store each.
+                    const int r16 = lrow & 15, upper = r16 >> 3;
+                    __half *ap = a.act + (size_t)(w.tok0 + c0 + upper) * a.ld_act + rt * 8 + (r16 & 7);
                     #pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        const float mine = __uint_as_float(v[j]);
-                        const float other = __shfl_xor_sync(0xffffffffu, mine, 8);
-                        if (r16 < 8 && rt < a.n_row_tiles && tok0 + c0 + j < a.n_tok) {
-                            const float y = __fmul_rn(gelu_tanh(mine), other);
-                            a.act[(size_t)(tok0 + c0 + j) * a.ld_act + rt * 8 + r16] = __float2half_rn(y);
-                        }
+                    for (int j = 0; j < 32; j += 2) {
+                        const float e = __uint_as_float(v[j]), o = __uint_as_float(v[j + 1]);
+                        const float got = __shfl_xor_sync(0xffffffffu, upper ? e : o, 8);
+                        const float gate = upper ? got : e, up = upper ? o : got;
+                        if (rt < a.n_row_tiles && c0 + j + upper < w.n)
+                            ap[(size_t)j * a.ld_act] = __float2half_rn(__fmul_rn(gelu_tanh(gate), up));
                     }
                 }
             }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty);
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == LG_PF_DQ_WARPS + 2) {
+    if (warp == DQ + 2) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(NT) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512) : "memory");
     }
 }
 

@@ -1,0 +1,42 @@
+"""GPU tests of the wide matmul's persistent form: an odd number of k blocks (a last step of one), row blocks with fewer than
+eight row tiles, and prompts of several token tiles."""
+import numpy as np
+import pytest
+
+from tests.conftest import model_files, synth_module
+from tests.test_gpu_prefill import _weights
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,k", [(16, 64), (48, 192), (272, 320), (2048, 448)])
+@pytest.mark.parametrize("n", [1, 17, 241, 256])
+def test_odd_k_blocks_and_ragged_rows(lg, port_built, m, k, n):
+    s = synth_module()
+    rng = np.random.default_rng(m + k + n)
+    raw, t, w = _weights(s, rng, "q4_0", m, k)
+    x = rng.standard_normal((n, k)).astype(np.float32)
+    got = lg.prefill_matmul(t, raw, m, k, x)
+    want = x.astype(np.float16).astype(np.float64) @ w.astype(np.float64).T
+    # one f16 rounding per weight (2^-11 relative) and f32 sums
+    bound = 2.0 ** -11 * (np.abs(x) @ np.abs(w.T)) + 1e-5 * np.abs(want).max()
+    assert (np.abs(got - want) <= bound).all()
+
+
+@pytest.mark.parametrize("n", [257, 521, 1024, 1101])
+def test_token_tiles_do_not_change_a_prompt(lg, n):
+    """One call (tiles of equal shares, one block of up to 1024) against calls of 200 tokens (one tile each, other k slices)."""
+    s = synth_module()
+    tp, _ = model_files("mid")
+    out = []
+    for step in (n, 200):
+        with lg.Session(tp, None, 1280) as g:
+            toks = s.prompt_ids(n + 1, g.n_vocab, seed=31)
+            for i in range(0, n, step):
+                g.prefill(toks[i:min(n, i + step)], i)
+            rows = [np.concatenate(g.kv_row(layer, p, 512)) for layer in range(2) for p in (0, 199, n - 40, n - 1)]
+            out.append((rows, g.forward(int(toks[n]), n)))
+    for a, b in zip(*[o[0] for o in out]):
+        assert np.abs(a - b).max() <= 1e-2 * max(1.0, np.abs(b).max())
+    a, b = out[0][1], out[1][1]
+    assert np.abs(a - b).max() / (b.max() - b.min()) <= 1e-2
