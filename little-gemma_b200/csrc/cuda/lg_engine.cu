@@ -1099,7 +1099,7 @@ void enqueue_prefill_block(Engine *e, const struct kvcache *kv, int n, int only 
         const int hd = w.hd, src = w.src;
         const int gqa = H / w.nkv;
         static const int block_attn = env_int("LG_PREFILL_BLOCK_ATTN", 1);
-        const bool whole = block_attn && (hd == 64 || hd == 128 || hd == 256) && LG_PFA_Q % gqa == 0;
+        const bool whole = block_attn && (hd == 64 || hd == 128 || hd == 256) && 32 % gqa == 0;
         const int ks_q = whole ? pf_kslices(e, w.qkv, n, 2) : 1, ks_o = pf_kslices(e, w.o, n, PF_MAX_KS), ks_d = pf_kslices(e, w.down, n, PF_MAX_KS);
         if (only & C_QKV) launch_pf_gemm(e, w.qkv, b.a_ne, LG_PF_MAXN, n, b.qkv, nullptr, 0, LG_PF_STORE, ks_q);
         if ((only & C_ATTN) && whole) {
@@ -1110,19 +1110,20 @@ void enqueue_prefill_block(Engine *e, const struct kvcache *kv, int n, int only 
             pa.kc = (__half *)kv->k[src]; pa.vc = (__half *)kv->v[src]; pa.seq = kv->seq[src]; pa.kv_dim = kv->kv_dim[src];
             pa.H = H; pa.Hkv = w.nkv; pa.pos = b.pos; pa.q_hi = b.q_hi; pa.q_lo = b.q_lo;
             LgPfAttnArgs fa{};
-            fa.q_hi = b.q_hi; fa.q_lo = b.q_lo; fa.kc = pa.kc; fa.vc = pa.vc; fa.seq = pa.seq; fa.kv_dim = pa.kv_dim;
-            fa.H = H; fa.Hkv = w.nkv; fa.n = n; fa.window = w.local ? c->sliding_window : 0; fa.pos = b.pos;
-            fa.out = b.a_attn; fa.ld_out = H * hd;
+            fa.seq = pa.seq; fa.H = H; fa.Hkv = w.nkv; fa.n = n; fa.window = w.local ? c->sliding_window : 0; fa.pos = b.pos;
+            fa.out = b.a_attn; fa.ld_out = H * hd; fa.err = e->err;
+            const CUtensorMap tqh = act_tensor_map(b.q_hi, hd, n * H, LG_PFA_Q), tql = act_tensor_map(b.q_lo, hd, n * H, LG_PFA_Q);
+            const CUtensorMap tk = kv_tensor_map(pa.kc, pa.kv_dim, pa.seq, LG_PFA_S), tv = kv_tensor_map(pa.vc, pa.kv_dim, pa.seq, LG_PFA_S);
             const int qb = LG_PFA_Q / gqa;
-            dim3 grid(w.nkv, (n + qb - 1) / qb);
+            const dim3 grid((n + qb - 1) / qb, w.nkv);
             dim3 prep_grid(n, (H + (w.owns_kv ? 2 * w.nkv : 0) + 7) / 8);           // one head vector per warp
             switch (hd) {
             case 64:  launch_k(e, lg_pf_qkv_prep_kernel<64>, prep_grid, dim3(256), 0, pa);
-                      launch_k(e, lg_pf_attn_kernel<64>, grid, dim3(256), pf_attn_smem<64>(), fa); break;
+                      launch_k(e, lg_pf_attn_kernel<64>, grid, dim3(LG_PFA_THREADS), pf_attn_smem<64>(), tqh, tql, tk, tv, fa); break;
             case 128: launch_k(e, lg_pf_qkv_prep_kernel<128>, prep_grid, dim3(256), 0, pa);
-                      launch_k(e, lg_pf_attn_kernel<128>, grid, dim3(256), pf_attn_smem<128>(), fa); break;
+                      launch_k(e, lg_pf_attn_kernel<128>, grid, dim3(LG_PFA_THREADS), pf_attn_smem<128>(), tqh, tql, tk, tv, fa); break;
             default:  launch_k(e, lg_pf_qkv_prep_kernel<256>, prep_grid, dim3(256), 0, pa);
-                      launch_k(e, lg_pf_attn_kernel<256>, grid, dim3(256), pf_attn_smem<256>(), fa); break;
+                      launch_k(e, lg_pf_attn_kernel<256>, grid, dim3(LG_PFA_THREADS), pf_attn_smem<256>(), tqh, tql, tk, tv, fa); break;
             }
         } else if (only & C_ATTN)
             for (int g0 = 0; g0 < n; g0 += LG_MAXM) {

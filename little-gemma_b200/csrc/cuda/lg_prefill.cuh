@@ -365,7 +365,7 @@ __global__ void lg_f32_to_f16_rows(const float *__restrict__ src, int ld_src, __
 // attention of a prompt block: all query rows of the block in one launch per layer
 // ---------------------------------------------------------------------------------------------
 // Step 1 (lg_pf_qkv_prep_kernel): per token, per-head RMSNorm + NeoX RoPE of the raw projection
-// rows.  Queries go to an f16 hi + lo pair [tok][H][hd]; K (norm + rope) and V (plain norm) rows go
+// rows.  Queries go to an f16 hi + lo pair [kv head][tok][query heads of it][hd]; K (norm + rope) and V (plain norm) rows go
 // to the f16 cache of the owning layer (round to nearest even) at row (pos % seq).  The cache ring
 // of a sliding-window layer has more spare rows than a block has tokens, so writing the whole block
 // first does not overwrite a row an earlier query of the block still attends to.
@@ -378,7 +378,7 @@ struct LgPfPrepArgs {
     __half *kc, *vc; int seq, kv_dim;
     int H, Hkv;
     const int *pos;                      // position of the block's first token
-    __half *q_hi, *q_lo;                 // [n][H][hd]
+    __half *q_hi, *q_lo;                 // [Hkv][n][H / Hkv][hd]
 };
 
 template <int HD>
@@ -411,7 +411,9 @@ __global__ void __launch_bounds__(256) lg_pf_qkv_prep_kernel(LgPfPrepArgs a) {
         }
         if (j < a.H) {
             head_norm_rope<HD>(src, s_qn, rope, a.eps, lane, v0, v1);
-            __half *dh = a.q_hi + ((size_t)tok * a.H + j) * HD, *dl = a.q_lo + ((size_t)tok * a.H + j) * HD;
+            const int gqa = a.H / a.Hkv;
+            const size_t qrow = ((size_t)(j / gqa) * gridDim.x + tok) * gqa + j % gqa;
+            __half *dh = a.q_hi + qrow * HD, *dl = a.q_lo + qrow * HD;
             #pragma unroll
             for (int e = 0; e < PER; e++) {
                 const int i = lane * PER + e;
@@ -431,185 +433,251 @@ __global__ void __launch_bounds__(256) lg_pf_qkv_prep_kernel(LgPfPrepArgs a) {
     }
 }
 
-// Step 2 (lg_pf_attn_kernel): one CTA = one KV head x LG_PFA_Q query rows (LG_PFA_Q / gqa consecutive
-// tokens x the gqa query heads of that KV head).  It walks the keys of its causal / sliding window
-// in tiles of 64 with an online softmax: S = Q K^T and O += P V on mma.sync.m16n8k16 (f16 operands,
-// f32 accumulate), Q and P as f16 hi + lo pairs like the decode kernel, scale 1.0.  The normalised
-// rows are written as f16 -- the o-projection's input.
+// Step 2 (lg_pf_attn_kernel): one CTA = one KV head x 128 query rows (the TMEM lanes; 128 / gqa consecutive tokens x the gqa
+// query heads of that KV head), longest rows first.  It walks the keys of its causal / sliding window in tiles of 64 with an
+// online softmax, S = Q K^T and O += P V on tcgen05 (f16 operands, f32 accumulation in tensor memory), Q and P as f16 hi + lo
+// pairs like the decode kernel, scale 1.0.
+//   warp 4  copies the two query blocks, then key and value tiles in the order the products take them, through three slots;
+//           rows behind the last position written so far hold whatever was there: their values are zeroed in the last tile;
+//   warp 5  issues the products: S(i + 1) into one of two 64-column buffers while tile i is in its softmax, then O += P(i) V
+//           with P from tensor memory and V as it lies in the cache (an MN-major operand);
+//   warps 0-3  one query row per thread: scores from tensor memory, softmax in f32, the weights back over the scores.  O is
+//           rescaled only when a row's maximum has grown by more than 2^LG_PFA_SLACK since the one in use (until then weights
+//           are merely larger than 1), which needs the previous product to have finished.
+// Scores of two tiles may be finished before the first one's weights are used, so the buffers have barriers of their own.
+// What bounds it: the products of a row block's tiles and the softmax between them, about 1.7 us a tile of 64 keys at head size 256
+// (the products alone: 1.1 us).  12B-class layer, 928 tokens from position 0: 35 us (mma.sync, 32 rows per CTA: 165); E4B-class
+// layer, 48 tokens behind 701: 18 us (52).
 struct LgPfAttnArgs {
-    const __half *q_hi, *q_lo;           // [n][H][hd]
-    const __half *kc, *vc; int seq, kv_dim;
-    int H, Hkv, n;
+    int seq, H, Hkv, n;
     int window;                          // <= 0: full causal
     const int *pos;
     __half *out; int ld_out;             // [n][ld_out], head hq at column hq*hd
+    int *err;
 };
-#define LG_PFA_Q 32
+#define LG_PFA_Q 128
 #define LG_PFA_S 64
+#define LG_PFA_SLOTS 3
+#define LG_PFA_THREADS 192
+#define LG_PFA_SLACK 8.0f
+template <int HD> constexpr size_t pf_attn_smem() { return 1024 + (size_t)HD / 64 * (2 * LG_PFA_Q + LG_PFA_SLOTS * LG_PFA_S) * 128 + 256; }
 
 template <int HD>
-__global__ void __launch_bounds__(256) lg_pf_attn_kernel(LgPfAttnArgs a) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    constexpr int NQ = LG_PFA_Q, S = LG_PFA_S, LDH = HD + 8, LDP = S + 8, LDS = S + 4;
-    __half *qhi = (__half *)smem, *qlo = qhi + NQ * LDH;
-    __half *sk = qlo + NQ * LDH;                              // two buffers of [K tile | V tile], each [S][LDH]
-    float *sc = (float *)(sk + 4 * S * LDH);                  // [NQ][LDS]
-    __half *phi = (__half *)(sc + NQ * LDS), *plo = phi + NQ * LDP;
-    float *row_m = (float *)(plo + NQ * LDP), *row_l = row_m + NQ, *row_a = row_l + NQ;
-    pdl_launch(); pdl_wait();
-
-    const int kvh = blockIdx.x, gqa = a.H / a.Hkv, qb = NQ / gqa;           // qb tokens per CTA
-    const int t0 = blockIdx.y * qb;
-    if (t0 >= a.n) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const int pos0 = *a.pos;
-    const int nt = min(qb, a.n - t0);                                       // valid tokens of this CTA
-    const int p_first = pos0 + t0, p_last = pos0 + t0 + nt - 1;
-    const int lo_first = a.window > 0 ? max(0, p_first - a.window + 1) : 0;
-
-    // queries: row r = (token r / gqa, head kvh*gqa + r % gqa)
-    constexpr int CH = HD / 8;
-    for (int i = threadIdx.x; i < NQ * CH; i += 256) {
-        const int r = i / CH, c = i % CH, tok = t0 + r / gqa, hq = kvh * gqa + r % gqa;
-        uint4 vh = make_uint4(0, 0, 0, 0), vl = vh;
-        if (r / gqa < nt) {
-            vh = *(const uint4 *)(a.q_hi + ((size_t)tok * a.H + hq) * HD + c * 8);
-            vl = *(const uint4 *)(a.q_lo + ((size_t)tok * a.H + hq) * HD + c * 8);
-        }
-        *(uint4 *)(qhi + (size_t)r * LDH + c * 8) = vh;
-        *(uint4 *)(qlo + (size_t)r * LDH + c * 8) = vl;
+__global__ void __launch_bounds__(LG_PFA_THREADS, 1)
+lg_pf_attn_kernel(const __grid_constant__ CUtensorMap tmqh, const __grid_constant__ CUtensorMap tmql, const __grid_constant__ CUtensorMap tmk,
+                  const __grid_constant__ CUtensorMap tmv, LgPfAttnArgs a) {
+    extern __shared__ __align__(16) unsigned char pfa_smem[];
+    constexpr int NB = HD / 64, S = LG_PFA_S, SL = LG_PFA_SLOTS, Q_BLK = LG_PFA_Q * 128, T_BLK = S * 128, SLOT = NB * T_BLK;
+    constexpr uint32_t TCOLS = 2 * S + HD <= 256 ? 256 : 512;            // scores / weights twice 64 columns, output HD
+    unsigned char *sQ = (unsigned char *)(((uintptr_t)pfa_smem + 1023) & ~(uintptr_t)1023), *sT = sQ + 2 * NB * Q_BLK;
+    uint64_t *qfull = (uint64_t *)(sT + SL * SLOT), *full = qfull + 1, *empty = full + SL, *sfull = empty + SL /* two */,
+             *pready = sfull + 2 /* two */, *odone = pready + 2 /* two */, *vfix = odone + 2;
+    uint32_t *tmem_slot = (uint32_t *)(vfix + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        mbar_init(qfull, 1); mbar_init(vfix, 1);
+        for (int i = 0; i < SL; i++) { mbar_init(full + i, 1); mbar_init(empty + i, 1); }
+        for (int i = 0; i < 2; i++) { mbar_init(sfull + i, 1); mbar_init(pready + i, 4); mbar_init(odone + i, 1); }
     }
-    for (int r = threadIdx.x; r < NQ; r += 256) { row_m[r] = -INFINITY; row_l[r] = 0.0f; }
+    if (warp == 5) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(tmem_slot)), "r"(TCOLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tmem_slot, tO = tmem + 2 * S;
+    pdl_launch();                        // only now: a dependant must not take tensor memory a CTA of this grid still waits for
+    pdl_wait();
 
-    // warp roles: m-tile mt (16 query rows) x slice hf of the tile's keys (scores) or of the head dims (output)
-    constexpr int MT = NQ / 16, WK = 8 / MT, KPW = S / WK, NKT = KPW / 8;
-    const int mt = warp % MT, hf = warp / MT;
-    constexpr int DW = HD / WK, NT = DW / 8;                   // output dims per warp, 8-wide n tiles
-    static_assert(NT % 2 == 0 && NKT >= 1, "tile split");
-    float o[NT][4];
-    #pragma unroll
-    for (int n2 = 0; n2 < NT; n2++) o[n2][0] = o[n2][1] = o[n2][2] = o[n2][3] = 0.0f;
+    const int kvh = blockIdx.y, gqa = a.H / a.Hkv, qb = LG_PFA_Q / gqa;                 // qb tokens per CTA
+    const int t0 = (gridDim.x - 1 - blockIdx.x) * qb, nt = min(qb, a.n - t0);           // its valid tokens
+    const int pos0 = *a.pos, p_last = pos0 + t0 + nt - 1;
+    const int k_first = (a.window > 0 ? max(0, pos0 + t0 - a.window + 1) : 0) / S * S;
+    const int n_tiles = (p_last - k_first) / S + 1;
+    const int v_stale = pos0 + a.n - (k_first + (n_tiles - 1) * S);                     // first unwritten row of the last tile
 
-    // K/V tiles are double-buffered: tile i+1 streams in (cp.async) while tile i is being used
-    auto load_tile = [&](int k0, int buf) {
-        __half *bk = sk + (size_t)buf * 2 * S * LDH, *bv = bk + S * LDH;
-        for (int i = threadIdx.x; i < S * CH; i += 256) {
-            const int key = i / CH, c = i % CH, p = k0 + key;
-            __half *dk = bk + (size_t)key * LDH + c * 8, *dv = bv + (size_t)key * LDH + c * 8;
-            if (p <= p_last) {
-                const size_t off = (size_t)(p % a.seq) * a.kv_dim + (size_t)kvh * HD + c * 8;
-                cp_async16(dk, a.kc + off);
-                cp_async16(dv, a.vc + off);
-            } else {
-                *(uint4 *)dk = make_uint4(0, 0, 0, 0);
-                *(uint4 *)dv = make_uint4(0, 0, 0, 0);
+    if (warp == 4) {
+        bool ok = true;
+        int issued = 0;
+        PfRing q;
+        if (lane == 0) {
+            mbar_expect_tx(qfull, 2 * NB * Q_BLK);
+            const int row = (kvh * a.n + t0) * gqa;
+            for (int c = 0; c < NB; c++) {
+                tma_load_2d(sQ + c * Q_BLK, &tmqh, c * 64, row, qfull);
+                tma_load_2d(sQ + (NB + c) * Q_BLK, &tmql, c * 64, row, qfull);
+            }
+            // K0, K1, V0, K2, V1, ..
+            for (int u = 0; u < 2 * n_tiles; u++) {
+                const bool is_v = u == 2 * n_tiles - 1 || (u >= 2 && !(u & 1));
+                const int i = u == 0 ? 0 : is_v ? (u == 2 * n_tiles - 1 ? n_tiles - 1 : u / 2 - 1) : (u + 1) / 2;
+                if (issued >= SL && !mbar_wait(empty + q.s, q.ph ^ 1)) { atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 4); ok = false; break; }
+                mbar_expect_tx(full + q.s, SLOT);
+                const int r = (k_first + i * S) % a.seq;
+                for (int c = 0; c < NB; c++) tma_load_2d(sT + q.s * SLOT + c * T_BLK, is_v ? &tmv : &tmk, kvh * HD + c * 64, r, full + q.s);
+                issued++;
+                if (u != 2 * n_tiles - 1) q.next(SL);
+            }
+            if (!ok) {           // own copies in flight land before the CTA ends
+                mbar_wait(qfull, 0);
+                for (int r = max(0, issued - SL); r < issued; r++) mbar_wait(full + r % SL, (r / SL) & 1);
             }
         }
-    };
-    const int k_first = (lo_first / S) * S;
-    load_tile(k_first, 0);
-    int buf = 0;
-    for (int k0 = k_first; k0 <= p_last; k0 += S, buf ^= 1) {
-        cp_async_wait_all();
-        __syncthreads();                                        // tile k0 has landed; the other buffer and P are no longer read
-        if (k0 + S <= p_last) load_tile(k0 + S, buf ^ 1);
-        const __half *sk_t = sk + (size_t)buf * 2 * S * LDH, *sv_t = sk_t + S * LDH;
-
-        // ---- scores of 16 rows x KPW keys per warp ----
-        {
-            float c0[NKT][4];
-            #pragma unroll
-            for (int n2 = 0; n2 < NKT; n2++) c0[n2][0] = c0[n2][1] = c0[n2][2] = c0[n2][3] = 0.0f;
-            const __half *qa_hi = qhi + (size_t)(mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDH + (lane >> 4) * 8;
-            const __half *qa_lo = qlo + (size_t)(mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDH + (lane >> 4) * 8;
-            const __half *kb = sk_t + (size_t)(hf * KPW + (lane & 7)) * LDH + (lane >> 3) * 8;
-            #pragma unroll 2
-            for (int d0 = 0; d0 < HD; d0 += 32) {
-                uint32_t ah[4], al[4], ah2[4], al2[4];
-                ldsm_x4(ah, qa_hi + d0); ldsm_x4(al, qa_lo + d0);
-                ldsm_x4(ah2, qa_hi + d0 + 16); ldsm_x4(al2, qa_lo + d0 + 16);
-                #pragma unroll
-                for (int n2 = 0; n2 < NKT; n2++) {
-                    uint32_t b[4];
-                    ldsm_x4(b, kb + (size_t)n2 * 8 * LDH + d0);
-                    mma_f16(c0[n2], ah, b[0], b[1]); mma_f16(c0[n2], al, b[0], b[1]);
-                    mma_f16(c0[n2], ah2, b[2], b[3]); mma_f16(c0[n2], al2, b[2], b[3]);
+        if (v_stale < S) {
+            const int slot = __shfl_sync(0xffffffffu, q.s, 0), ph = __shfl_sync(0xffffffffu, (int)q.ph, 0);
+            ok = __shfl_sync(0xffffffffu, (int)ok, 0) && mbar_wait(full + slot, ph);
+            if (__all_sync(0xffffffffu, ok)) {
+                for (int c = lane; c < NB * (S - v_stale) * 8; c += 32) {       // a row's 16-byte chunks stay within its 128 bytes
+                    const int b = c / ((S - v_stale) * 8), rest = c % ((S - v_stale) * 8);
+                    *(uint4 *)(sT + slot * SLOT + b * T_BLK + v_stale * 128 + rest * 16) = make_uint4(0, 0, 0, 0);
                 }
+                fence_async_shared();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(vfix);
             }
-            #pragma unroll
-            for (int h2 = 0; h2 < 2; h2++) {
-                const int r = mt * 16 + g + h2 * 8;
-                const int pj = pos0 + t0 + r / gqa;
-                const int lo = a.window > 0 ? max(0, pj - a.window + 1) : 0;
-                const bool rv = r / gqa < nt;
+        }
+    } else if (warp == 5) {
+        // f32 accumulator, f16 x f16; N = keys of a tile / value columns
+        const uint32_t fmt = (1u << 4) | ((uint32_t)(LG_PFA_Q >> 4) << 24);
+        const uint32_t idS = fmt | ((uint32_t)(S >> 3) << 17), idO = fmt | ((uint32_t)(HD >> 3) << 17) | LG_UMMA_B_MN;
+        const uint64_t qd = umma_desc_k128(smem_u32(sQ)), kd0 = umma_desc_k128(smem_u32(sT)), vd0 = umma_desc_mn128(smem_u32(sT), T_BLK);
+        PfRing q;
+        bool ok = mbar_wait(qfull, 0);
+        auto scores = [&](int i) {
+            if (!__all_sync(0xffffffffu, mbar_wait(full + q.s, q.ph))) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t tS = tmem + (i & 1) * S;
+            const uint64_t kd = kd0 + q.s * (SLOT >> 4);
+            if (elect_one()) {
                 #pragma unroll
-                for (int n2 = 0; n2 < NKT; n2++)
+                for (int part = 0; part < 2; part++)
                     #pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        const int key = hf * KPW + n2 * 8 + t * 2 + e, p = k0 + key;
-                        sc[r * LDS + key] = (rv && p >= lo && p <= pj) ? c0[n2][h2 * 2 + e] : -INFINITY;
-                    }
+                    for (int c = 0; c < NB; c++)
+                        #pragma unroll
+                        for (int j = 0; j < 4; j++)
+                            umma_f16(tS, qd + (part * NB + c) * (Q_BLK >> 4) + 2 * j, kd + c * (T_BLK >> 4) + 2 * j, idS, part | c | j);
+                umma_commit(empty + q.s);
+                umma_commit(sfull + (i & 1));
             }
-        }
-        __syncthreads();
-
-        // ---- online softmax: warp w owns NQ/8 consecutive rows ----
-        for (int r = warp * (NQ / 8); r < (warp + 1) * (NQ / 8); r++) {
-            const float s0 = sc[r * LDS + lane], s1 = sc[r * LDS + lane + 32];
-            const float m_old = row_m[r];
-            const float m_new = fmaxf(m_old, warp_max(fmaxf(s0, s1)));
-            const float e0 = s0 == -INFINITY ? 0.0f : expf(s0 - m_new), e1 = s1 == -INFINITY ? 0.0f : expf(s1 - m_new);
-            const __half h0 = __float2half_rn(e0), h1 = __float2half_rn(e1);
-            phi[r * LDP + lane] = h0; phi[r * LDP + lane + 32] = h1;
-            plo[r * LDP + lane] = __float2half_rn(e0 - __half2float(h0));
-            plo[r * LDP + lane + 32] = __float2half_rn(e1 - __half2float(h1));
-            const float sum = warp_sum(e0 + e1);
-            if (lane == 0) {
-                const float alpha = m_old == -INFINITY ? 0.0f : expf(m_old - m_new);     // m_new == -inf: nothing seen yet
-                row_a[r] = alpha;
-                row_l[r] = row_l[r] * alpha + sum;
-                row_m[r] = m_new;
-            }
-        }
-        __syncthreads();
-
-        // ---- O = alpha O + P V: 16 rows x DW dims per warp ----
-        {
-            const float a0 = row_a[mt * 16 + g], a1 = row_a[mt * 16 + g + 8];
-            #pragma unroll
-            for (int n2 = 0; n2 < NT; n2++) { o[n2][0] *= a0; o[n2][1] *= a0; o[n2][2] *= a1; o[n2][3] *= a1; }
-            const __half *pa_hi = phi + (size_t)(mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDP + (lane >> 4) * 8;
-            const __half *pa_lo = plo + (size_t)(mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDP + (lane >> 4) * 8;
-            #pragma unroll
-            for (int kk = 0; kk < S; kk += 16) {
-                uint32_t ah[4], al[4];
-                ldsm_x4(ah, pa_hi + kk); ldsm_x4(al, pa_lo + kk);
-                const __half *vb = sv_t + (size_t)(kk + (lane & 7) + ((lane >> 3) & 1) * 8) * LDH + hf * DW + (lane >> 4) * 8;
+            __syncwarp();
+            q.next(SL);
+            return true;
+        };
+        ok = __all_sync(0xffffffffu, ok) && scores(0);
+        for (int i = 0; i < n_tiles && ok; i++) {
+            if (i + 1 < n_tiles) ok = scores(i + 1);
+            ok = ok && mbar_wait(pready + (i & 1), (i >> 1) & 1) && mbar_wait(full + q.s, q.ph);
+            if (ok && i == n_tiles - 1 && v_stale < S) ok = mbar_wait(vfix, 0);
+            if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t tP = tmem + (i & 1) * S;
+            const uint64_t vd = vd0 + q.s * (SLOT >> 4);
+            if (elect_one()) {
                 #pragma unroll
-                for (int n2 = 0; n2 < NT; n2 += 2) {
-                    uint32_t b[4];
-                    ldsm_x4_t(b, vb + n2 * 8);
-                    mma_f16(o[n2], ah, b[0], b[1]); mma_f16(o[n2], al, b[0], b[1]);
-                    mma_f16(o[n2 + 1], ah, b[2], b[3]); mma_f16(o[n2 + 1], al, b[2], b[3]);
+                for (int j = 0; j < 4; j++) umma_f16_ta(tO, tP + 8 * j, vd + j * 128, idO, i | j);
+                #pragma unroll
+                for (int j = 0; j < 4; j++) umma_f16_ta(tO, tP + 32 + 8 * j, vd + j * 128, idO, 1u);
+                umma_commit(empty + q.s);
+                umma_commit(odone + (i & 1));
+            }
+            __syncwarp();
+            q.next(SL);
+        }
+        if (!ok && lane == 0) atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 8);
+    } else {
+        const int r = threadIdx.x, tok = t0 + r / gqa, hq = kvh * gqa + r % gqa;
+        const bool rv = r / gqa < nt;
+        const int pj = rv ? pos0 + tok : -1, lo = rv && a.window > 0 ? max(0, pj - a.window + 1) : 0;       // keys lo .. pj
+        // every row of the warp sees keys all_lo .. all_hi
+        const int all_lo = __reduce_max_sync(0xffffffffu, lo), all_hi = __reduce_min_sync(0xffffffffu, pj);
+        const uint32_t lanes = (uint32_t)(warp * 32) << 16;
+        float m = -INFINITY, l = 0.0f;
+        bool ok = true;
+        for (int i = 0; i < n_tiles; i++) {
+            const int k0 = k_first + i * S;
+            ok = __all_sync(0xffffffffu, mbar_wait(sfull + (i & 1), (i >> 1) & 1));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t tS = tmem + lanes + (i & 1) * S;
+            uint32_t s0[32], s1[32];
+            tmem_ld32(tS, s0);
+            tmem_ld32(tS + 32, s1);
+            float mx = -INFINITY;
+            if (k0 < all_lo || k0 + S - 1 > all_hi) {
+                #pragma unroll
+                for (int j = 0; j < 32; j++) {
+                    const int k = k0 + j;
+                    if (k < lo || k > pj) s0[j] = 0xff800000u;
+                    if (k + 32 < lo || k + 32 > pj) s1[j] = 0xff800000u;
                 }
             }
+            #pragma unroll
+            for (int j = 0; j < 32; j++) mx = fmaxf(mx, fmaxf(__uint_as_float(s0[j]), __uint_as_float(s1[j])));
+            const float mt = mx * LG_LOG2E;
+            const bool grow = mt > m + LG_PFA_SLACK;             // from -inf: as soon as the row sees a key
+            if (__any_sync(0xffffffffu, grow)) {
+                const float m_new = fmaxf(m, mt), alpha = m == -INFINITY ? 0.0f : exp2f(m - m_new);
+                if (i) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(odone + ((i - 1) & 1), ((i - 1) >> 1) & 1));
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    for (int c = 0; c < HD; c += 32) {
+                        uint32_t o[32];
+                        tmem_ld32(tO + lanes + c, o);
+                        #pragma unroll
+                        for (int j = 0; j < 32; j++) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
+                        tmem_st32(tO + lanes + c, o);
+                    }
+                    tmem_wait_st();
+                }
+                l *= alpha; m = m_new;
+            }
+            const float mu = m == -INFINITY ? 0.0f : m;          // nothing seen yet: every weight is 2^-inf
+            #pragma unroll
+            for (int half = 0; half < 2; half++) {
+                uint32_t hi[16], lw[16];
+                #pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    const float x = __uint_as_float(half ? s1[2 * j] : s0[2 * j]), y = __uint_as_float(half ? s1[2 * j + 1] : s0[2 * j + 1]);
+                    const float p = ex2(fmaf(x, LG_LOG2E, -mu)), w = ex2(fmaf(y, LG_LOG2E, -mu));
+                    l += p + w;
+                    const __half2 h = __floats2half2_rn(p, w);
+                    const float2 f = __half22float2(h);
+                    const __half2 d = __floats2half2_rn(p - f.x, w - f.y);
+                    hi[j] = *(const uint32_t *)&h; lw[j] = *(const uint32_t *)&d;
+                }
+                tmem_st16(tS + 16 * half, hi);
+                tmem_st16(tS + 32 + 16 * half, lw);
+            }
+            tmem_wait_st();
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(pready + (i & 1));
         }
+        ok = __all_sync(0xffffffffu, ok && mbar_wait(odone + ((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1));
+        if (!ok && lane == 0) atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 32);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+        if (ok)
+            for (int c = 0; c < HD; c += 32) {
+                uint32_t o[32];
+                tmem_ld32(tO + lanes + c, o);
+                if (rv) {
+                    uint4 *dst = (uint4 *)(a.out + (size_t)tok * a.ld_out + (size_t)hq * HD + c);
+                    #pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        auto two = [&](int k) { const __half2 h = __floats2half2_rn(__uint_as_float(o[8 * j + k]) * inv, __uint_as_float(o[8 * j + k + 1]) * inv); return *(const uint32_t *)&h; };
+                        dst[j] = make_uint4(two(0), two(2), two(4), two(6));
+                    }
+                }
+                __syncwarp();
+            }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
     __syncthreads();
-    #pragma unroll
-    for (int h2 = 0; h2 < 2; h2++) {
-        const int r = mt * 16 + g + h2 * 8;
-        if (r / gqa < nt) {
-            const float l = row_l[r], inv = l > 0.0f ? 1.0f / l : 0.0f;
-            __half *dst = a.out + (size_t)(t0 + r / gqa) * a.ld_out + (size_t)(kvh * gqa + r % gqa) * HD + hf * DW;
-            #pragma unroll
-            for (int n2 = 0; n2 < NT; n2++)
-                *(__half2 *)(dst + n2 * 8 + t * 2) = __floats2half2_rn(o[n2][h2 * 2] * inv, o[n2][h2 * 2 + 1] * inv);
-        }
+    if (warp == 5) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(TCOLS) : "memory");
     }
-}
-
-template <int HD> constexpr size_t pf_attn_smem() {
-    return (size_t)2 * LG_PFA_Q * (HD + 8) * 2 + (size_t)4 * LG_PFA_S * (HD + 8) * 2 + (size_t)LG_PFA_Q * (LG_PFA_S + 4) * 4
-         + (size_t)2 * LG_PFA_Q * (LG_PFA_S + 8) * 2 + 3 * LG_PFA_Q * 4;
 }

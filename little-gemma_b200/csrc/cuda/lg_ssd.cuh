@@ -16,15 +16,6 @@
 #define LG_SSD_Q 128
 #define LG_SSD_OUT_THREADS 448
 
-// MN-major operand, 128-byte swizzle: rows of the contraction of 128 bytes (64 elements), 8-row groups 1024 bytes apart, blocks of 64
-// columns `block` bytes apart
-__device__ __forceinline__ uint64_t umma_desc_mn128(uint32_t saddr, uint32_t block) {
-    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(block >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-#define LG_UMMA_A_MN (1u << 15)     // instruction descriptor: A / B stored MN-major
-#define LG_UMMA_B_MN (1u << 16)
-__device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
 struct LgSsdArgs {
     const float *dt; int ld_dt;                  // raw step sizes [token][..]
     const float *dt_bias, *a_log, *d;

@@ -40,3 +40,36 @@ def test_token_tiles_do_not_change_a_prompt(lg, n):
         assert np.abs(a - b).max() <= 1e-2 * max(1.0, np.abs(b).max())
     a, b = out[0][1], out[1][1]
     assert np.abs(a - b).max() / (b.max() - b.min()) <= 1e-2
+
+
+@pytest.mark.parametrize("name,n,step", [("tiny", 1500, 200), ("tiny", 1500, 64), ("mid", 330, 129)])
+def test_prompt_attention_tiles_and_ring(lg, name, n, step):
+    """Key tiles behind a wrapped sliding-window ring, first tiles that some rows do not see, query blocks that end inside a tile:
+    one call against calls of `step` tokens."""
+    s = synth_module()
+    tp, _ = model_files(name)
+    out = []
+    for st in (n, step):
+        with lg.Session(tp, None, 2048) as g:
+            toks = s.prompt_ids(n + 1, g.n_vocab, seed=32)
+            for i in range(0, n, st):
+                g.prefill(toks[i:min(n, i + st)], i)
+            out.append(g.forward(int(toks[n]), n))
+    assert np.abs(out[0] - out[1]).max() / (out[1].max() - out[1].min()) <= 1e-2
+
+
+@pytest.mark.parametrize("name", ["tiny", "mid"])
+@pytest.mark.parametrize("n", [33, 65, 100])
+def test_rows_behind_the_prompt_do_not_matter(lg, name, n):
+    """A prompt over a cache that an earlier, longer one has filled gives the bits of a fresh cache."""
+    s = synth_module()
+    tp, _ = model_files(name)
+    out = []
+    for used in (False, True):
+        with lg.Session(tp, None, 512) as g:
+            if used:
+                g.prefill(s.prompt_ids(400, g.n_vocab, seed=33), 0)
+            toks = s.prompt_ids(n + 1, g.n_vocab, seed=34)
+            g.prefill(toks[:n], 0)
+            out.append(g.forward(int(toks[n]), n))
+    assert np.array_equal(out[0].view(np.uint32), out[1].view(np.uint32))
