@@ -1059,9 +1059,18 @@ void prefill_alloc(Engine *e) {
 // x += norm(add)*add_w (optional), x *= out_scale; yh = norm(x)*norm_w as f16 rows.  One CTA per token.
 void launch_norm_pf(Engine *e, int n_tok, float *x, int n, float eps, const float *add, int n_parts, int ld_add, const float *add_w,
                     float out_scale, const float *norm_w, __half *yh, bool row_itself = false) {
+    __half *out = (norm_w || row_itself) ? yh : nullptr;                     // row_itself: the f16 row is x, not a norm of it
+    if (n % 4 == 0 && n <= 8192) {
+        // two groups of four elements a thread, four beyond 4096 elements
+        LgPfNormArgs a{x, add, n_parts, (size_t)n_tok * ld_add, ld_add, add_w, out_scale, norm_w, out, n, eps};
+        const int t = std::min(512, (n / 8 + 31) & ~31);
+        if (n <= 8 * t) launch_k(e, lg_pf_norm_kernel<2>, dim3(n_tok), dim3(t), 0, a);
+        else launch_k(e, lg_pf_norm_kernel<4>, dim3(n_tok), dim3(t), 0, a);
+        return;
+    }
     LgNormArgs a{};
     a.x = x; a.ldx = n; a.add_src = add; a.n_parts = n_parts; a.part_stride = (size_t)n_tok * ld_add; a.ld_add = ld_add; a.add_w = add_w; a.out_scale = out_scale;
-    a.norm_w = norm_w; a.n = n; a.eps = eps; a.yh = (norm_w || row_itself) ? yh : nullptr; a.ldyh = n;   // row_itself: the f16 row is x, not a norm of it
+    a.norm_w = norm_w; a.n = n; a.eps = eps; a.yh = out; a.ldyh = n;
     int threads = n >= 2048 ? 1024 : (n >= 512 ? 512 : 256);
     launch_k(e, lg_norm_kernel, dim3(n_tok), dim3(threads), (size_t)(2 * n + 32) * 4, a);
 }

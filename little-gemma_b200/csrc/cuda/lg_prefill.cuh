@@ -353,6 +353,83 @@ __global__ void lg_inject_rows(float *__restrict__ x, int ldx, const float *__re
     for (int i = threadIdx.x; i < n; i += blockDim.x) x[(size_t)tok * ldx + i] = rows[(size_t)r * n + i];
 }
 
+// The residual update and the norm of a prompt block's rows, one CTA per token with the row in registers (V groups of four
+// elements a thread), n a multiple of 4 and at most 4 V blockDim.x: x += rmsnorm(sum of the planes of add) * add_w, x *= out_scale;
+// yh = rmsnorm(x) * norm_w, or x itself, as f16.  Bound by memory traffic and the two sums over the block; 928 rows of 3840: 33 us with the row in shared
+// memory and three barriers per sum, 14 us now.
+struct LgPfNormArgs {
+    float *x;
+    const float *add; int n_parts; size_t part_stride; int ld_add;
+    const float *add_w; float out_scale;
+    const float *norm_w;
+    __half *yh;
+    int n; float eps;
+};
+__device__ __forceinline__ float pf_block_sum(float v, float *red) {        // red: one float per warp, a buffer of its own per sum
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    const int nw = blockDim.x >> 5;
+    return warp_sum((int)(threadIdx.x & 31) < nw ? red[threadIdx.x & 31] : 0.0f);
+}
+template <int V>
+__global__ void __launch_bounds__(512) lg_pf_norm_kernel(LgPfNormArgs a) {
+    __shared__ float red[2][32];
+    const int tok = blockIdx.x, n4 = a.n >> 2;
+    float4 aw[V], nw[V], x[V], o[V];
+    pdl_launch();
+    #pragma unroll
+    for (int k = 0; k < V; k++) {                          // the weights do not depend on the previous kernel
+        const int i = threadIdx.x + k * blockDim.x;
+        aw[k] = nw[k] = x[k] = o[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (i < n4 && a.add) aw[k] = ((const float4 *)a.add_w)[i];
+        if (i < n4 && a.norm_w) nw[k] = ((const float4 *)a.norm_w)[i];
+    }
+    pdl_wait();
+    float4 *row = (float4 *)(a.x + (size_t)tok * a.n);
+    const float *src = a.add + (size_t)tok * a.ld_add;
+    float ss = 0.0f;
+    #pragma unroll
+    for (int k = 0; k < V; k++) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i >= n4) continue;
+        x[k] = row[i];
+        if (!a.add) continue;
+        for (int p = 0; p < a.n_parts; p++) {
+            const float4 t = ((const float4 *)(src + (size_t)p * a.part_stride))[i];
+            o[k].x += t.x; o[k].y += t.y; o[k].z += t.z; o[k].w += t.w;
+        }
+        ss += o[k].x * o[k].x + o[k].y * o[k].y + o[k].z * o[k].z + o[k].w * o[k].w;
+    }
+    if (a.add) {
+        const float s = 1.0f / sqrtf(pf_block_sum(ss, red[0]) / (float)a.n + a.eps);
+        auto upd = [&](float x, float o, float w) { return __fmul_rn(__fadd_rn(x, __fmul_rn(__fmul_rn(o, s), w)), a.out_scale); };
+        #pragma unroll
+        for (int k = 0; k < V; k++) {
+            const int i = threadIdx.x + k * blockDim.x;
+            if (i >= n4) continue;
+            x[k] = make_float4(upd(x[k].x, o[k].x, aw[k].x), upd(x[k].y, o[k].y, aw[k].y), upd(x[k].z, o[k].z, aw[k].z), upd(x[k].w, o[k].w, aw[k].w));
+            row[i] = x[k];
+        }
+    }
+    if (!a.yh) return;
+    float s = 1.0f;
+    if (a.norm_w) {
+        ss = 0.0f;
+        #pragma unroll
+        for (int k = 0; k < V; k++) ss += x[k].x * x[k].x + x[k].y * x[k].y + x[k].z * x[k].z + x[k].w * x[k].w;
+        s = 1.0f / sqrtf(pf_block_sum(ss, red[1]) / (float)a.n + a.eps);
+    }
+    auto y = [&](float x, float w) { return a.norm_w ? __fmul_rn(__fmul_rn(x, s), w) : x; };
+    #pragma unroll
+    for (int k = 0; k < V; k++) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i >= n4) continue;
+        const __half2 h0 = __floats2half2_rn(y(x[k].x, nw[k].x), y(x[k].y, nw[k].y)), h1 = __floats2half2_rn(y(x[k].z, nw[k].z), y(x[k].w, nw[k].w));
+        ((uint2 *)(a.yh + (size_t)tok * a.n))[i] = make_uint2(*(const uint32_t *)&h0, *(const uint32_t *)&h1);
+    }
+}
+
 // f32 rows -> f16 rows (the B operand of the wide matmul)
 __global__ void lg_f32_to_f16_rows(const float *__restrict__ src, int ld_src, __half *__restrict__ dst, int ld_dst, int n) {
     pdl_launch(); pdl_wait();
@@ -381,55 +458,68 @@ struct LgPfPrepArgs {
     __half *q_hi, *q_lo;                 // [Hkv][n][H / Hkv][hd]
 };
 
+// One head vector per warp, PER consecutive elements of each half a lane; the norm weights do not depend on the previous kernel
+// and are fetched before the wait.  Bound by its memory traffic (928 tokens of a 12B-class layer: 53 MB); wide loads and stores
+// instead of one element at a time: 22 -> 15 us.
+template <int N> struct PfVec;
+template <> struct PfVec<1> { typedef float F; typedef uint16_t H; };
+template <> struct PfVec<2> { typedef float2 F; typedef uint32_t H; };
+template <> struct PfVec<4> { typedef float4 F; typedef uint2 H; };
+template <int N> __device__ __forceinline__ void pf_load(const float *p, float (&v)[N]) { *(typename PfVec<N>::F *)v = *(const typename PfVec<N>::F *)p; }
+template <int N> __device__ __forceinline__ void pf_store(__half *p, const __half (&h)[N]) { *(typename PfVec<N>::H *)p = *(const typename PfVec<N>::H *)h; }
+
 template <int HD>
 __global__ void __launch_bounds__(256) lg_pf_qkv_prep_kernel(LgPfPrepArgs a) {
-    __shared__ float s_qn[HD], s_kn[HD];
-    __shared__ float s_row[8][HD];       // a warp's head vector with the k-slice planes added
-    pdl_launch();
-    for (int i = threadIdx.x; i < HD; i += 256) { s_qn[i] = a.q_norm[i]; s_kn[i] = a.k_norm ? a.k_norm[i] : 1.0f; }
-    pdl_wait();
-    __syncthreads();
     constexpr int PER = HD / 64, HALF = HD / 2;
-    const int tok = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tok = blockIdx.x, lane = threadIdx.x & 31, j = blockIdx.y * 8 + (threadIdx.x >> 5), i0 = lane * PER;
+    const int jj = j - a.H, isv = jj >= a.Hkv, kvh = isv ? jj - a.Hkv : jj;
+    const bool live = j < a.H + (a.owns_kv ? 2 * a.Hkv : 0);
+    const float *w = j < a.H ? a.q_norm : isv ? nullptr : a.k_norm;
+    alignas(16) float w0[PER], w1[PER], v0[PER], v1[PER];
+    #pragma unroll
+    for (int e = 0; e < PER; e++) w0[e] = w1[e] = 1.0f;
+    pdl_launch();
+    if (live && w) { pf_load(w + i0, w0); pf_load(w + i0 + HALF, w1); }
+    pdl_wait();
+    if (!live) return;
     const int p = *a.pos + tok;
-    const int jobs = a.H + (a.owns_kv ? 2 * a.Hkv : 0);
-    const float2 *rope = a.rope + (size_t)tok * HALF;
-    for (int j = blockIdx.y * 8 + warp; j < jobs; j += 8 * gridDim.y) {     // one head vector per warp
-        float v0[PER], v1[PER];
-        const int jj = j - a.H, isv = jj >= a.Hkv, kvh = isv ? jj - a.Hkv : jj;
-        const float *src = a.qkv + (size_t)tok * a.ld
-                         + (size_t)(j < a.H ? j : a.H + ((isv && a.has_v) ? a.Hkv : 0) + kvh) * HD;
-        if (a.n_parts > 1) {
-            __syncwarp();
-            for (int i = lane; i < HD; i += 32) {
-                float v = src[i];
-                for (int p = 1; p < a.n_parts; p++) v += src[(size_t)p * a.part_stride + i];
-                s_row[warp][i] = v;
-            }
-            __syncwarp();
-            src = s_row[warp];
+    const float *src = a.qkv + (size_t)tok * a.ld + (size_t)(j < a.H ? j : a.H + ((isv && a.has_v) ? a.Hkv : 0) + kvh) * HD + i0;
+    pf_load(src, v0); pf_load(src + HALF, v1);
+    float2 cs[PER];
+    #pragma unroll
+    for (int e = 0; e < PER; e++) cs[e] = isv ? make_float2(1.0f, 0.0f) : a.rope[(size_t)tok * HALF + i0 + e];
+    for (int q = 1; q < a.n_parts; q++) {                                   // the k-slice planes, in order
+        alignas(16) float t0[PER], t1[PER];
+        pf_load(src + (size_t)q * a.part_stride, t0); pf_load(src + (size_t)q * a.part_stride + HALF, t1);
+        #pragma unroll
+        for (int e = 0; e < PER; e++) { v0[e] += t0[e]; v1[e] += t1[e]; }
+    }
+    float ss = 0.0f;
+    #pragma unroll
+    for (int e = 0; e < PER; e++) ss += v0[e] * v0[e] + v1[e] * v1[e];
+    const float sc = 1.0f / sqrtf(warp_sum(ss) / (float)HD + a.eps);
+    alignas(8) __half h0[PER], h1[PER];
+    #pragma unroll
+    for (int e = 0; e < PER; e++) {
+        float x = __fmul_rn(__fmul_rn(v0[e], sc), w0[e]), y = __fmul_rn(__fmul_rn(v1[e], sc), w1[e]);
+        if (!isv) {
+            const float r0 = __fsub_rn(__fmul_rn(x, cs[e].x), __fmul_rn(y, cs[e].y));
+            y = __fadd_rn(__fmul_rn(x, cs[e].y), __fmul_rn(y, cs[e].x));
+            x = r0;
         }
-        if (j < a.H) {
-            head_norm_rope<HD>(src, s_qn, rope, a.eps, lane, v0, v1);
-            const int gqa = a.H / a.Hkv;
-            const size_t qrow = ((size_t)(j / gqa) * gridDim.x + tok) * gqa + j % gqa;
-            __half *dh = a.q_hi + qrow * HD, *dl = a.q_lo + qrow * HD;
-            #pragma unroll
-            for (int e = 0; e < PER; e++) {
-                const int i = lane * PER + e;
-                const __half h0 = __float2half_rn(v0[e]), h1 = __float2half_rn(v1[e]);
-                dh[i] = h0; dh[i + HALF] = h1;
-                dl[i] = __float2half_rn(v0[e] - __half2float(h0)); dl[i + HALF] = __float2half_rn(v1[e] - __half2float(h1));
-            }
-        } else {
-            head_norm_rope<HD>(src, isv ? nullptr : s_kn, isv ? nullptr : rope, a.eps, lane, v0, v1);
-            __half *dst = (isv ? a.vc : a.kc) + (size_t)(p % a.seq) * a.kv_dim + (size_t)kvh * HD;
-            #pragma unroll
-            for (int e = 0; e < PER; e++) {
-                dst[lane * PER + e] = __float2half_rn(v0[e]);
-                dst[lane * PER + e + HALF] = __float2half_rn(v1[e]);
-            }
-        }
+        v0[e] = x; v1[e] = y;
+        h0[e] = __float2half_rn(x); h1[e] = __float2half_rn(y);
+    }
+    if (j < a.H) {
+        const int gqa = a.H / a.Hkv;
+        const size_t qrow = (((size_t)(j / gqa) * gridDim.x + tok) * gqa + j % gqa) * HD + i0;
+        pf_store(a.q_hi + qrow, h0); pf_store(a.q_hi + qrow + HALF, h1);
+        #pragma unroll
+        for (int e = 0; e < PER; e++) { h0[e] = __float2half_rn(v0[e] - __half2float(h0[e])); h1[e] = __float2half_rn(v1[e] - __half2float(h1[e])); }
+        pf_store(a.q_lo + qrow, h0); pf_store(a.q_lo + qrow + HALF, h1);
+    } else {
+        __half *dst = (isv ? a.vc : a.kc) + (size_t)(p % a.seq) * a.kv_dim + (size_t)kvh * HD + i0;
+        pf_store(dst, h0); pf_store(dst + HALF, h1);
     }
 }
 
