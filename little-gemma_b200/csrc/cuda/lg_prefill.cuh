@@ -336,13 +336,16 @@ __global__ void __launch_bounds__(LG_PF_THREADS, 1) lg_pf_gemm_kernel(const __gr
     }
 }
 
-// y = gelu_tanh(gate) * up as f16 rows (per-layer-embedding gate of a prompt block)
+// y = gelu_tanh(sum of the planes of gate) * up as f16 rows (per-layer-embedding gate of a prompt block)
 __global__ void lg_pf_geglu_rows(const float *__restrict__ gate, const float *__restrict__ up, int ld_g, int ld_u, int n,
-                                 __half *__restrict__ out, int ld_out) {
+                                 __half *__restrict__ out, int ld_out, int n_parts, size_t part_stride) {
     pdl_launch(); pdl_wait();
     const int tok = blockIdx.y;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        out[(size_t)tok * ld_out + i] = __float2half_rn(__fmul_rn(gelu_tanh(gate[(size_t)tok * ld_g + i]), up[(size_t)tok * ld_u + i]));
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        float v = gate[(size_t)tok * ld_g + i];
+        for (int p = 1; p < n_parts; p++) v += gate[(size_t)p * part_stride + (size_t)tok * ld_g + i];
+        out[(size_t)tok * ld_out + i] = __float2half_rn(__fmul_rn(gelu_tanh(v), up[(size_t)tok * ld_u + i]));
+    }
 }
 
 // Media positions of a prompt block: x[tok] = rows[ridx[tok]] where ridx[tok] >= 0 (the row replaces the token embedding as it is)
