@@ -1076,9 +1076,9 @@ void launch_norm_pf(Engine *e, int n_tok, float *x, int n, float eps, const floa
 }
 
 // One block of n <= LG_PF_MAXN prompt tokens at positions pos0.. (ids in pf.toks, group positions in pf.pos):
-// fills the KV rows of every layer.  The layer matmuls see all n tokens at once; attention walks the block in
-// groups of LG_MAXM query rows with the decode step's kernel, so a group's keys include the rows of the groups
-// before it.  Models with per-layer embeddings take the narrow path instead.
+// fills the KV rows of every layer.  Matmuls and attention see all n tokens at once; layers whose head size or group the
+// block attention does not take (512; a group that does not divide 32) walk the block in groups of LG_MAXM query rows with
+// the decode step's kernel, so a group's keys include the rows of the groups before it.
 void enqueue_prefill_block(Engine *e, const struct kvcache *kv, int n, int only = C_ALL, bool media = false) {
     const struct config *c = &e->m->cfg;
     const int ne = c->n_embd, H = c->n_head, nl = c->n_layer;
