@@ -224,8 +224,7 @@ inline int env_int(const char *name, int fb) { const char *v = getenv(name); ret
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-inline CUtensorMap tiled_map(const void *ptr, CUtensorMapDataType type, long long cols, long long rows, long long row_bytes, int box_c, int box_r,
-                             CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
+inline EncodeTiledFn encode_tiled_fn() {
     static EncodeTiledFn fn = nullptr;
     if (!fn) {
         void *p = nullptr;
@@ -234,14 +233,30 @@ inline CUtensorMap tiled_map(const void *ptr, CUtensorMapDataType type, long lon
         if (!p || qr != cudaDriverEntryPointSuccess) { fprintf(stderr, "lg_b200: the driver has no cuTensorMapEncodeTiled\n"); exit(1); }
         fn = (EncodeTiledFn)p;
     }
+    return fn;
+}
+inline CUtensorMap tiled_map(const void *ptr, CUtensorMapDataType type, long long cols, long long rows, long long row_bytes, int box_c, int box_r,
+                             CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
     CUtensorMap map;
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
     cuuint32_t box[2] = {(cuuint32_t)box_c, (cuuint32_t)box_r};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(&map, type, 2, (void *)ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    CUresult r = encode_tiled_fn()(&map, type, 2, (void *)ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                   swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { fprintf(stderr, "lg_b200: cuTensorMapEncodeTiled failed (%d) for %lld x %lld\n", (int)r, rows, cols); exit(1); }
+    return map;
+}
+// The same of an array [row tiles][positions][bytes] (bytes <= 1024, a multiple of 16): boxes of box_t row tiles x box_p positions
+inline CUtensorMap tile_boxes_map(const void *ptr, int bytes, int positions, int row_tiles, int box_p, int box_t) {
+    CUtensorMap map;
+    cuuint64_t dims[3] = {(cuuint64_t)bytes / 4, (cuuint64_t)positions, (cuuint64_t)row_tiles};
+    cuuint64_t strides[2] = {(cuuint64_t)bytes, (cuuint64_t)bytes * positions};
+    cuuint32_t box[3] = {(cuuint32_t)bytes / 4, (cuuint32_t)box_p, (cuuint32_t)box_t};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = encode_tiled_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_INT32, 3, (void *)ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { fprintf(stderr, "lg_b200: cuTensorMapEncodeTiled failed (%d) for %d x %d tiles\n", (int)r, row_tiles, positions); exit(1); }
     return map;
 }
 

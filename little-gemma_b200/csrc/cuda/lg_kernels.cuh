@@ -364,6 +364,9 @@ __device__ __forceinline__ void mma_s8_k16(int (&c)[4], uint32_t a0, uint32_t a1
         : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(b0));
 }
 
+// A matrix's arrays as boxes of one ring stage (R row tiles x P positions)
+struct LgStageMaps { CUtensorMap q, s, d, m; };
+
 // The small-M matmul.  A CTA walks items = (group of R consecutive row tiles) x (its k slice,
 // blockIdx.y), item after item (blockIdx.x, +gridDim.x, ...).
 //   * One producer thread streams the items' weight tiles HBM -> shared memory with bulk copies
@@ -382,9 +385,8 @@ __device__ __forceinline__ void mma_s8_k16(int (&c)[4], uint32_t a0, uint32_t a1
 //     a thread-block cluster whose ranks 1.. send their sums into rank 0's shared memory (st.async, counted on an
 //     mbarrier of rank 0), so that rank 0 runs the epilogue on complete rows.
 // Dynamic shared memory: panel q | panel s | ring | warp partials | item sums | peers' sums (cluster) | mbarriers
-template <int R, int NP, int FMT, int EPI>
-__global__ void __launch_bounds__(LG_GEMV_THREADS)
-lg_gemv_kernel(LgGemvArgs a) {
+template <int R, int NP, int FMT, int EPI, bool TILED>
+__device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvArgs &a) {
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr int ST = gemv_stage_tiles<FMT>();
     constexpr int P = ST / R;                                // tile positions per stage
@@ -444,18 +446,30 @@ lg_gemv_kernel(LgGemvArgs a) {
                 for (int c = 0; c < n_chunks && ok; c++) {
                     if (!mbar_wait(empty + stage, phase ^ 1)) { atomicOr(a.err, LG_ERR_MBAR_TIMEOUT); ok = false; break; }
                     const int np = min(P, nkp_s - c * P);
-                    const uint32_t tile_bytes = (uint32_t)np * (TB + lg_tile_extra(FMT));
                     unsigned char *st = ring + (size_t)stage * STAGE;
-                    mbar_expect_tx(full + stage, R * tile_bytes);
-                    #pragma unroll
-                    for (int r = 0; r < R; r++) {
-                        const size_t tile = tile_base + (size_t)r * a.nkp + (size_t)c * P;
-                        bulk_g2s(st + (size_t)r * P * TB, a.wq + tile * (TB / 16), (uint32_t)np * TB, full + stage);
-                        bulk_g2s(st + SC_OFF + (size_t)r * P * 64, a.ws + tile * 8, (uint32_t)np * 64, full + stage);
-                        if (FMT != LG_FMT_Q4_0)
-                            bulk_g2s(st + DD_OFF + (size_t)r * P * 64, a.wd + tile * 8, (uint32_t)np * 64, full + stage);
-                        if (FMT == LG_FMT_I8M)
-                            bulk_g2s(st + MM_OFF + (size_t)r * P * 128, a.wm + tile * 8, (uint32_t)np * 128, full + stage);
+                    if (TILED && (np == P || kp1 == a.nkp)) {
+                        // a tiled copy per array: one of R row tiles x P positions takes as long to issue as one of a single
+                        // row tile (about 115 cycles).  Positions past the matrix arrive as zeros and are not read.
+                        const int kp = kp0 + c * P, rt = grp * R;
+                        mbar_expect_tx(full + stage, STAGE);
+                        tma_load_3d(st, &maps->q, 0, kp, rt, full + stage);
+                        tma_load_3d(st + SC_OFF, &maps->s, 0, kp, rt, full + stage);
+                        if (FMT != LG_FMT_Q4_0) tma_load_3d(st + DD_OFF, &maps->d, 0, kp, rt, full + stage);
+                        if (FMT == LG_FMT_I8M) tma_load_3d(st + MM_OFF, &maps->m, 0, kp, rt, full + stage);
+                    } else {
+                        // (the ragged end of a k slice too: the next slice's positions are not fetched for nothing)
+                        const uint32_t tile_bytes = (uint32_t)np * (TB + lg_tile_extra(FMT));
+                        mbar_expect_tx(full + stage, R * tile_bytes);
+                        #pragma unroll
+                        for (int r = 0; r < R; r++) {
+                            const size_t tile = tile_base + (size_t)r * a.nkp + (size_t)c * P;
+                            bulk_g2s(st + (size_t)r * P * TB, a.wq + tile * (TB / 16), (uint32_t)np * TB, full + stage);
+                            bulk_g2s(st + SC_OFF + (size_t)r * P * 64, a.ws + tile * 8, (uint32_t)np * 64, full + stage);
+                            if (FMT != LG_FMT_Q4_0)
+                                bulk_g2s(st + DD_OFF + (size_t)r * P * 64, a.wd + tile * 8, (uint32_t)np * 64, full + stage);
+                            if (FMT == LG_FMT_I8M)
+                                bulk_g2s(st + MM_OFF + (size_t)r * P * 128, a.wm + tile * 8, (uint32_t)np * 128, full + stage);
+                        }
                     }
                     if (++stage == NS) { stage = 0; phase ^= 1; }
                     if (!panel_sent && ++issued == early) {
@@ -773,6 +787,13 @@ lg_gemv_kernel(LgGemvArgs a) {
             if (a.amax_val2) a.amax_val2[(size_t)blockIdx.x * LG_MAXM + tok] = s2;
         }
     }
+}
+template <int R, int NP, int FMT, int EPI>
+__global__ void __launch_bounds__(LG_GEMV_THREADS) lg_gemv_kernel(LgGemvArgs a) { gemv_body<R, NP, FMT, EPI, false>(nullptr, a); }
+// the same with stages of several row tiles brought by tiled copies
+template <int R, int NP, int FMT, int EPI>
+__global__ void __launch_bounds__(LG_GEMV_THREADS) lg_gemv_tiled_kernel(const __grid_constant__ LgStageMaps maps, const __grid_constant__ LgGemvArgs a) {
+    gemv_body<R, NP, FMT, EPI, true>(&maps, a);
 }
 
 // Merge the per-CTA argmax candidates: out[tok] = index of the largest logit, lowest index on ties.
