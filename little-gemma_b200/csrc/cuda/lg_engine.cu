@@ -1668,9 +1668,12 @@ static void prefill_impl(struct model *m, struct kvcache *kv, const float *rows,
         std::vector<std::vector<int>> gpos_all, toks_all, ridx_all;
         std::vector<std::vector<float>> stage_all;
         while (n - i > LG_MAXM) {                                    // a last group of <= 8 tokens is cheaper on the verify path
-            const int real = std::min(LG_PF_MAXN, n - i);
-            const int b = (real + LG_MAXM - 1) / LG_MAXM * LG_MAXM;
-            if ((long long)pos0 + i + b > kv->max_seq) break;          // pad rows would wrap onto the cache's first rows: narrow path
+            int real = std::min(LG_PF_MAXN, n - i);
+            int b = (real + LG_MAXM - 1) / LG_MAXM * LG_MAXM;
+            if ((long long)pos0 + i + b > kv->max_seq) {               // pad rows would wrap onto the cache's first rows:
+                real = b = real / LG_MAXM * LG_MAXM;                   // whole groups only, the last 1 to 7 tokens take the narrow path
+                if (b <= LG_MAXM) break;
+            }
             gpos_all.emplace_back(LG_PF_MAXN / LG_MAXM);
             for (int g = 0; g < LG_PF_MAXN / LG_MAXM; g++) gpos_all.back()[g] = pos0 + i + g * LG_MAXM;
             toks_all.emplace_back(b);
