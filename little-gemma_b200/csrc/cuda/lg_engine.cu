@@ -21,7 +21,8 @@ using namespace lg;
 
 namespace {
 
-constexpr int RING_SPARE = 1024;             // ring rows beyond the window (covers the widest block written before its queries run)
+constexpr int RING_SPARE = 1024;             // ring rows beyond the window
+static_assert(LG_PF_MAXN <= RING_SPARE, "a prompt block is written whole before its queries run: it must not reach the first one's window");
 
 constexpr int LOG_CAP = 1 << 20;
 

@@ -41,7 +41,7 @@
 #define LG_PF_SMEM_MAX 232448   // 227 KB: the most dynamic shared memory a CTA can have
 #define LG_PF_DQ_WARPS (4 * LG_PF_GROUPS)
 #define LG_PF_THREADS ((LG_PF_DQ_WARPS + 3) * 32)
-#define LG_PF_MAXN 1024         // tokens of a block: as many as a sliding-window ring has spare rows
+#define LG_PF_MAXN 1024         // tokens of a block: at most the spare rows of a sliding-window ring (RING_SPARE)
 #define LG_PF_OP_MAXN 256       // tokens the kernel-level entry points take
 #define LG_PF_MAX_RAW 15
 
@@ -447,7 +447,7 @@ __global__ void lg_f32_to_f16_rows(const float *__restrict__ src, int ld_src, __
 // Step 1 (lg_pf_qkv_prep_kernel): per token, per-head RMSNorm + NeoX RoPE of the raw projection
 // rows.  Queries go to an f16 hi + lo pair [kv head][tok][query heads of it][hd]; K (norm + rope) and V (plain norm) rows go
 // to the f16 cache of the owning layer (round to nearest even) at row (pos % seq).  The cache ring
-// of a sliding-window layer has more spare rows than a block has tokens, so writing the whole block
+// of a sliding-window layer has at least as many spare rows as a block has tokens, so writing the whole block
 // first does not overwrite a row an earlier query of the block still attends to.
 struct LgPfPrepArgs {
     const float *qkv; int ld;            // [n][ld] = [q (H*hd) | k (Hkv*hd) | v (Hkv*hd)], the sum of n_parts planes
