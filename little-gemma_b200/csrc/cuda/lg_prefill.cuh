@@ -535,12 +535,13 @@ __global__ void __launch_bounds__(256) lg_pf_qkv_prep_kernel(LgPfPrepArgs a) {
 //   warp 5  issues the products: S(i + 1) into one of two 64-column buffers while tile i is in its softmax, then O += P(i) V
 //           with P from tensor memory and V as it lies in the cache (an MN-major operand);
 //   warps 0-3  one query row per thread: scores from tensor memory, softmax in f32, the weights back over the scores.  O is
-//           rescaled only when a row's maximum has grown by more than 2^LG_PFA_SLACK since the one in use (until then weights
+//           rescaled only when a row's maximum has grown by more than LG_PFA_SLACK since the one in use (until then weights
 //           are merely larger than 1), which needs the previous product to have finished.
 // Scores of two tiles may be finished before the first one's weights are used, so the buffers have barriers of their own.
-// What bounds it: the products of a row block's tiles and the softmax between them, about 1.7 us a tile of 64 keys at head size 256
-// (the products alone: 1.1 us).  12B-class layer, 928 tokens from position 0: 35 us (mma.sync, 32 rows per CTA: 165); E4B-class
-// layer, 48 tokens behind 701: 18 us (52).
+// What bounds it: the products of a row block's tiles and the softmax between them, about 1.8 us a tile of 64 keys at head size 256
+// (the products alone: 1.1 us).  In a serialised launch list: 12B-class layer, 928 tokens from position 0, 36.6 us (mma.sync, 32 rows
+// per CTA: 165); E4B-class layer, 48 tokens behind 701, 26 us on 4 CTAs.  The weights by ex2.approx of log2(e) s - m: 35.6 and 24.4 us,
+// but up to 2 % more error in a row's weights (scores within 0 .. 300 +- 16) and none below 2^-126; expf stays.
 struct LgPfAttnArgs {
     int seq, H, Hkv, n;
     int window;                          // <= 0: full causal
@@ -552,7 +553,7 @@ struct LgPfAttnArgs {
 #define LG_PFA_S 64
 #define LG_PFA_SLOTS 3
 #define LG_PFA_THREADS 192
-#define LG_PFA_SLACK 8.0f
+#define LG_PFA_SLACK 5.5f
 template <int HD> constexpr size_t pf_attn_smem() { return 1024 + (size_t)HD / 64 * (2 * LG_PFA_Q + LG_PFA_SLOTS * LG_PFA_S) * 128 + 256; }
 
 template <int HD>
@@ -707,10 +708,9 @@ lg_pf_attn_kernel(const __grid_constant__ CUtensorMap tmqh, const __grid_constan
             }
             #pragma unroll
             for (int j = 0; j < 32; j++) mx = fmaxf(mx, fmaxf(__uint_as_float(s0[j]), __uint_as_float(s1[j])));
-            const float mt = mx * LG_LOG2E;
-            const bool grow = mt > m + LG_PFA_SLACK;             // from -inf: as soon as the row sees a key
+            const bool grow = mx > m + LG_PFA_SLACK;             // from -inf: as soon as the row sees a key
             if (__any_sync(0xffffffffu, grow)) {
-                const float m_new = fmaxf(m, mt), alpha = m == -INFINITY ? 0.0f : exp2f(m - m_new);
+                const float m_new = fmaxf(m, mx), alpha = m == -INFINITY ? 0.0f : expf(m - m_new);
                 if (i) {
                     ok = __all_sync(0xffffffffu, mbar_wait(odone + ((i - 1) & 1), ((i - 1) >> 1) & 1));
                     if (!ok) break;
@@ -726,14 +726,14 @@ lg_pf_attn_kernel(const __grid_constant__ CUtensorMap tmqh, const __grid_constan
                 }
                 l *= alpha; m = m_new;
             }
-            const float mu = m == -INFINITY ? 0.0f : m;          // nothing seen yet: every weight is 2^-inf
+            const float mu = m == -INFINITY ? 0.0f : m;          // nothing seen yet: every weight is e^-inf
             #pragma unroll
             for (int half = 0; half < 2; half++) {
                 uint32_t hi[16], lw[16];
                 #pragma unroll
                 for (int j = 0; j < 16; j++) {
                     const float x = __uint_as_float(half ? s1[2 * j] : s0[2 * j]), y = __uint_as_float(half ? s1[2 * j + 1] : s0[2 * j + 1]);
-                    const float p = ex2(fmaf(x, LG_LOG2E, -mu)), w = ex2(fmaf(y, LG_LOG2E, -mu));
+                    const float p = expf(x - mu), w = expf(y - mu);
                     l += p + w;
                     const __half2 h = __floats2half2_rn(p, w);
                     const float2 f = __half22float2(h);
