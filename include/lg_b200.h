@@ -149,7 +149,7 @@ int  lg_gemv_host(int type, const void *blocks, int m, int k, const float *x, in
  * 0 (whole k range in one CTA), -2 (matrix shape cannot leave complete rows), -1 (bad arguments). */
 int  lg_matmul_resid_host(int type, const void *blocks, int m, int k, const float *act, int M, float *xres,
                           const float *add_w, float out_scale, const float *norm_w, float eps, float *y);
-/* The wide (prompt) matmul: out[tok][row] = W x[tok] for tok < n <= 256 at once, x rounded to f16,
+/* The wide (prompt) matmul: out[tok][row] = W x[tok] for tok < n <= 1024 at once, x rounded to f16,
  * weights expanded q4 -> f16 inside the kernel, tcgen05.mma with f32 accumulation.  With blocks_up
  * != NULL the two matrices are a gate/up pair and out[tok][row] = gelu_tanh(gate.x) * (up.x)
  * rounded to f16 (the fused epilogue the prompt pass uses).  Replaces the reference's wide-batch

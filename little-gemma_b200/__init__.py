@@ -176,7 +176,7 @@ def matmul_resid(ggml_type: int, raw: np.ndarray, m: int, k: int, act: np.ndarra
 
 
 def prefill_matmul(ggml_type: int, raw: np.ndarray, m: int, k: int, x: np.ndarray, raw_up: np.ndarray = None) -> np.ndarray:
-    """y[tok] = W x[tok] for up to 256 rows of x at once through the wide tcgen05 matmul (x rounded to f16).
+    """y[tok] = W x[tok] for up to 1024 rows of x at once through the wide tcgen05 matmul (x rounded to f16).
     With raw_up, raw/raw_up are a gate/up pair and y = gelu_tanh(gate x) * (up x), rounded to f16."""
     L = load()
     raw = np.ascontiguousarray(raw, dtype=np.uint8)

@@ -1,5 +1,5 @@
-"""GPU tests of the wide matmul's persistent form: an odd number of k blocks (a last step of one), row blocks with fewer than
-eight row tiles, and prompts of several token tiles."""
+"""GPU tests of the wide matmul's persistent form (an odd number of k blocks, so a last step of one; row blocks with fewer than
+eight row tiles; several items per CTA, several token tiles) and of prompts of several token tiles, key tiles and blocks."""
 import numpy as np
 import pytest
 
@@ -21,6 +21,32 @@ def test_odd_k_blocks_and_ragged_rows(lg, port_built, m, k, n):
     # one f16 rounding per weight (2^-11 relative) and f32 sums
     bound = 2.0 ** -11 * (np.abs(x) @ np.abs(w.T)) + 1e-5 * np.abs(want).max()
     assert (np.abs(got - want) <= bound).all()
+
+
+@pytest.mark.parametrize("wtype,k", [("q4_0", 448), ("q4_K", 512)])
+@pytest.mark.parametrize("n,geglu", [(257, False), (521, True), (1001, False), (1024, True)])
+def test_several_items_per_cta(lg, port_built, wtype, k, n, geglu):
+    """149 row blocks (the last of four row tiles) x 2 to 4 token tiles: two to five items for each of the 148 CTAs, so that the
+    accumulator is handed back between items and the rings of 3 stages run on through items of 4 steps."""
+    s = synth_module()
+    m = 19008
+    rng = np.random.default_rng(n + k)
+    x = rng.standard_normal((n, k)).astype(np.float32)
+    x16 = x.astype(np.float16).astype(np.float64)
+    if geglu:
+        (raw, t, wg), (raw_u, _, wu) = _weights(s, rng, wtype, m // 2, k), _weights(s, rng, wtype, m // 2, k)
+        got = lg.prefill_matmul(t, raw, m // 2, k, x, raw_up=raw_u)
+        g, u = (x16 @ v.astype(np.float64).T for v in (wg, wu))
+        want = 0.5 * g * (1.0 + np.tanh(0.7978845608028654 * (g + 0.044715 * g ** 3))) * u
+        assert np.abs(got - want).max() / np.abs(want).max() < 5e-3      # f16 output + f16 weights, as of one item
+        return
+    raw, t, w = _weights(s, rng, wtype, m, k)
+    got = lg.prefill_matmul(t, raw, m, k, x)
+    want = x16 @ w.astype(np.float64).T
+    if wtype == "q4_0":          # one f16 rounding per weight (2^-11 relative) and f32 sums
+        assert (np.abs(got - want) <= 2.0 ** -11 * (np.abs(x16) @ np.abs(w.T)) + 1e-5 * np.abs(want).max()).all()
+    else:                        # two f16 products and an f16 fma, as of one item
+        assert np.abs(got - want).max() / np.abs(want).max() < 4e-3
 
 
 @pytest.mark.parametrize("n", [257, 521, 1024, 1101])
