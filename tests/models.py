@@ -43,6 +43,9 @@ def shapes():
         "hd512": (s.TargetShape(n_layer=4, n_embd=512, n_head=4, n_head_kv=2, head_dim=256, head_dim_global=512, n_ff=1024,
                                 n_vocab=4096, window=64, local_per_global=1, ple=0, q_norm_scale=256 ** -0.5),
                   None, 26, 27),
+        # head size 128, a KV head per query head
+        "hd128": (s.TargetShape(n_layer=4, n_embd=512, n_head=4, n_head_kv=4, head_dim=128, n_ff=1024, n_vocab=4096, window=64,
+                                local_per_global=1, ple=0, q_norm_scale=128 ** -0.5), None, 28, 29),
         # a head whose 3 query heads the target's 2 KV heads do not divide: the device must turn drafting off, not exit
         "mid_oddhead": (s.TargetShape(n_layer=6, n_embd=512, n_head=8, n_head_kv=2, head_dim=256, n_ff=2048, n_vocab=8192,
                                       window=64, local_per_global=2, ple=0, q_norm_scale=256 ** -0.5),

@@ -122,3 +122,26 @@ def test_a_prompt_that_fills_its_cache(lg, n, pos0):
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
     a, b = out[0][1], out[1][1]              # the last 1 to 7 rows come from the narrow path in one of the two
     assert np.abs(a - b).max() / (b.max() - b.min()) <= 1e-2
+
+
+@pytest.mark.parametrize("n,step", [(45, 45), (300, 300), (300, 131)])
+def test_head_size_128_without_groups_matches_oracle(lg, port_built, n, step):
+    """128 tokens per attention CTA (one query head per KV head) in two column blocks, a window shorter than the prompt: most rows
+    do not see the first key tiles of their CTA."""
+    from oracle.pyref import PortOracle
+    s = synth_module()
+    tp, _ = model_files("hd128")
+    o = PortOracle(tp, None, 512, True, 4)
+    toks = s.prompt_ids(n + 3, o.n_vocab, seed=36)
+    o.prefill(toks[:n], 0)
+    with lg.Session(tp, None, 512) as g:
+        for i in range(0, n, step):
+            g.prefill(toks[i:min(n, i + step)], i)
+        for layer in range(4):
+            for pos in sorted({max(0, n - 60), n - 33, n - 9, n - 1}):          # the oracle's ring keeps the window's 64 rows
+                for a, b in zip(g.kv_row(layer, pos, 4 * 128), o.kv_row(layer, pos, 4 * 128)):
+                    assert np.abs(a - b).max() < 1e-2 * max(1.0, np.abs(b).max()), (layer, pos)
+        for i in range(n, n + 3):
+            want, got = o.forward(int(toks[i]), i), g.forward(int(toks[i]), i)
+            assert np.abs(got - want).max() / (want.max() - want.min()) <= 1e-2
+    o.close()
