@@ -288,7 +288,7 @@ def sweep(a, lg, synth, torch):
         print(json.dumps({"sweep_prefill": pf}), flush=True)
         lines.append(f"\nPrompt pass of {pf['tokens']} uniform-random tokens (model_prefill, host clock, synchronised): "
                      f"{pf['ms']:.1f} ms = {pf['tok_s']:.0f} tok/s" +
-                     (f"; the tcgen05 layer matmuls of one 256-token block: {pf['matmul_block']['ms']:.2f} ms = "
+                     (f"; the tcgen05 layer matmuls of its {pf['matmul_block']['tokens']}-token block: {pf['matmul_block']['ms']:.2f} ms = "
                       f"{pf['matmul_block']['achieved']:.0f} TFLOP/s = {pf['matmul_block']['frac']:.3f} of the measured sustained "
                       f"bf16 peak." if "matmul_block" in pf else "."))
     out = a.sweep_out or os.path.join(ROOT, "gpurun_out", f"sweep_{cfg}.md")
@@ -301,6 +301,7 @@ def sweep(a, lg, synth, torch):
 # the latent-attention design beside the block-quantised family
 # ---------------------------------------------------------------------------------------------
 C_QKV, C_O, C_GATEUP, C_DOWN, C_HEAD, C_EXPAND, C_NORM, C_ATTN, C_MISC, C_FUSED = 1, 2, 4, 8, 16, 32, 64, 256, 512, 1024
+PF_BLOCK = 1024         # most tokens of a wide prompt block of the block-quantised family (LG_PF_MAXN)
 
 
 def design_shapes(synth, name):
@@ -402,8 +403,9 @@ def design_model(a, lg, synth, torch, path, latent, shape, n_pf, depths, peaks):
             pairs = n * (n + 1) / 2
             fl = 2.0 * L * n * (sum(pf_par.values()) + ((kv_w + out_w) if latent else 0)) + L * pairs * pair
             r = {"prompt": {"ms": ms, "tok_s": n / ms * 1e3, "frac": fl / (ms * 1e-3) / tc}}
-            blk = min(n, 2048 if latent else 256)              # the family's own block
-            keys0 = 0 if latent else (n - 1) // 256 * 256      # where the block the class passes repeat sits
+            # where the block the class passes repeat sits (the q4 family: the prompt's last one), and its tokens
+            keys0 = 0 if latent else (n - 1) // PF_BLOCK * PF_BLOCK
+            blk = min(n, 2048) if latent else n - keys0
             if latent:
                 cl = dict(cls, expand=C_EXPAND)
                 pp = dict(pf_par, expand=kv_w + out_w)
@@ -428,7 +430,7 @@ def design(a, lg, synth, torch):
              "equal width, heads, feed-forward, layers and vocabulary.  `frac` = algorithmic bytes (decode) or operations (prefill) over device",
              f"time, of the measured copy bandwidth ({peaks.get('hbm_gbs')} GB/s) or sustained bf16 throughput ({peaks.get('bf16_tflops_sustained')} TFLOP/s).",
              "Kernel classes: device time per layer, all layers' launches of the class back to back, L2 overwritten before each pass; prefill",
-             "classes on one block (2048 tokens from position 0, or the q4 family's last block of 256).", ""]
+             f"classes on one block (2048 tokens from position 0, or the q4 family's last block of up to {PF_BLOCK}).", ""]
     out = {}
     for name in a.design_sizes.split(","):
         ls, ts = design_shapes(synth, name)
@@ -601,9 +603,14 @@ def load_peaks():
         return {}
 
 
+def block_of(n):
+    """Tokens of the first wide block of a prompt of n: padded to a multiple of 8."""
+    return min((n + 7) // 8 * 8, PF_BLOCK)
+
+
 def time_prefill(r, synth, torch, t_shape, peaks):
-    """model_prefill of a 929-token prompt (host call, wall clock, synchronised) and the wide tcgen05 matmuls of one
-    256-token block over all layers, event-timed, against the tensor peak."""
+    """model_prefill of a 929-token prompt (host call, wall clock, synchronised) and the wide tcgen05 matmuls of its
+    block over all layers, event-timed, against the tensor peak."""
     sess = r.sess
     n_pf = min(929, r.max_seq - 8)
     pf_prompt = synth.prompt_ids(n_pf, t_shape.n_vocab, seed=300 + RANK)
@@ -614,21 +621,22 @@ def time_prefill(r, synth, torch, t_shape, peaks):
     torch.cuda.synchronize()
     pf_s = time.perf_counter() - t0
     rec = {"tokens": n_pf, "ms": pf_s * 1e3, "tok_s": n_pf / pf_s}
-    if sess.prefill_pass(256, 0) > 0:
+    blk = block_of(n_pf)
+    if sess.prefill_pass(blk, 0) > 0:
         torch.cuda.synchronize()
         g0, g1 = r.ev(), r.ev()
         g0.record(r.stream)
         for _ in range(5):
-            n_pf_mm = sess.prefill_pass(256, 0)
+            n_pf_mm = sess.prefill_pass(blk, 0)
         g1.record(r.stream)
         g1.synchronize()
         pf_mm_ms = g0.elapsed_time(g1) / 5
         ne_, H_, Hkv_, nff_ = t_shape.n_embd, t_shape.n_head, t_shape.n_head_kv, t_shape.n_ff
         layer_params = sum(ne_ * (H_ + 2 * Hkv_) * t_shape.hd(l) + H_ * t_shape.hd(l) * ne_ + 3 * ne_ * nff_ for l in range(t_shape.n_layer))
-        tfl = 2.0 * layer_params * 256 / (pf_mm_ms * 1e-3) / 1e12
+        tfl = 2.0 * layer_params * blk / (pf_mm_ms * 1e-3) / 1e12
         tpeak = float(peaks.get("bf16_tflops_sustained", 1400.0))
         rec["matmul_block"] = {"bound": "tensor", "kernel": "lg_pf_gemm_kernel (tcgen05, f16 operands, f32 accumulate)",
-                               "tokens": 256, "launches": n_pf_mm, "ms": pf_mm_ms, "achieved": tfl, "unit": "TFLOP/s",
+                               "tokens": blk, "launches": n_pf_mm, "ms": pf_mm_ms, "achieved": tfl, "unit": "TFLOP/s",
                                "peak": tpeak, "frac": tfl / tpeak,
                                "peak_source": ("measured (MEASURED_PEAKS.json bf16_tflops_sustained: the pass is a few ms of "
                                                "back-to-back launches)" if peaks else "fallback 1400 TFLOP/s sustained")}
@@ -657,7 +665,7 @@ def main():
     ap.add_argument("--profile-step", action="store_true",
                     help="short path for profilers: load, prefill, W warm-up rounds, K rounds, exit")
     ap.add_argument("--profile-prefill", type=int, default=None, metavar="CLASSES",
-                    help="short path for profilers: load, model_prefill of 512 tokens, 3 wide prompt blocks of 256 tokens "
+                    help="short path for profilers: load, model_prefill of 929 tokens, 3 times its wide block "
                          "restricted to kernel classes (4 = gate/up matmul, 1023 = everything), exit")
     ap.add_argument("--design", default=None, choices=["mubopel", "baporax"], help="time a design beside its closest one instead of the benchmark line")
     ap.add_argument("--design-sizes", default="2b,8b,16b")
@@ -741,10 +749,11 @@ def main():
     sess, stream, first, pos0 = r.sess, r.stream, r.first, a.depth
 
     if a.profile_prefill is not None:
-        sess.prefill(synth.prompt_ids(min(512, r.max_seq - 8), V, seed=300), 0)
+        n_pf = min(929, r.max_seq - 8)
+        sess.prefill(synth.prompt_ids(n_pf, V, seed=300), 0)
         n_l = 0
         for _ in range(3):
-            n_l = sess.prefill_pass(256, a.profile_prefill)
+            n_l = sess.prefill_pass(block_of(n_pf), a.profile_prefill)
         torch.cuda.synchronize()
         print(json.dumps({"profile_prefill": a.profile_prefill, "launches_per_block": n_l, "config": base["config"]}), flush=True)
         r.close()

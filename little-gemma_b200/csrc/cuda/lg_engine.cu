@@ -2010,7 +2010,7 @@ int lg_bench_prefill_pass(struct model *m, int n, int classes) {
         if (n < 1 || !e->kv_bound || e->fam->bench_block(e, e->kv_bound, n, 0, classes) != 0) return -1;
         return (int)(e->launches - before);
     }
-    if (n < 1 || n > LG_PF_OP_MAXN || !e->kv_bound || !prefill_wide_ok(e)) return -1;
+    if (n < 1 || n > LG_PF_MAXN || !e->kv_bound || !prefill_wide_ok(e)) return -1;
     prefill_alloc(e);
     enqueue_prefill_block(e, e->kv_bound, n, classes);
     return (int)(e->launches - before);

@@ -42,7 +42,6 @@
 #define LG_PF_DQ_WARPS (4 * LG_PF_GROUPS)
 #define LG_PF_THREADS ((LG_PF_DQ_WARPS + 3) * 32)
 #define LG_PF_MAXN 1024         // tokens of a block: at most the spare rows of a sliding-window ring (RING_SPARE)
-#define LG_PF_OP_MAXN 256       // tokens lg_bench_prefill_pass takes
 #define LG_PF_MAX_RAW 15
 
 enum { LG_PF_STORE = 0, LG_PF_GEGLU = 1 };

@@ -145,3 +145,15 @@ def test_head_size_128_without_groups_matches_oracle(lg, port_built, n, step):
             want, got = o.forward(int(toks[i]), i), g.forward(int(toks[i]), i)
             assert np.abs(got - want).max() / (want.max() - want.min()) <= 1e-2
     o.close()
+
+
+def test_timing_pass_takes_the_block_a_prompt_runs(lg):
+    """The benchmark times the block that a prompt of its length runs, up to the largest one."""
+    import bench
+    s = synth_module()
+    tp, _ = model_files("mid")
+    with lg.Session(tp, None, 2048) as g:
+        g.prefill(s.prompt_ids(1024, g.n_vocab, seed=37), 0)
+        assert bench.block_of(929) == 936 and bench.block_of(5000) == bench.PF_BLOCK
+        assert g.prefill_pass(bench.block_of(929), 0) > 0 and g.prefill_pass(bench.PF_BLOCK, 0) > 0
+        assert g.prefill_pass(bench.PF_BLOCK + 1, 0) == -1
