@@ -317,9 +317,10 @@ void launch_gemv_t(Engine *e, const LgGemvArgs &a, const GemvPlan &p) {
     if (p.smem > GEMV_SMEM_MAX) { fprintf(stderr, "lg_b200: matmul slice needs %zu bytes of shared memory\n", p.smem); exit(1); }
     dim3 grid(p.gx, p.ks);
     if constexpr (R > 1) {
-        // Tiled copies where a CTA streams at least a full ring: they issue R times fewer copies, the first of which waits for
-        // its descriptor.  q4_K rounds of width 8 27.9 -> 27.5 ms, 12B-class q4_0 rounds 51.2 -> 50.8 ms; of shorter launches the
-        // descriptor costs more (the tiny model 1 % slower).
+        // Tiled copies where a CTA streams at least four stages (the deepest ring): they issue R times fewer copies, the first of
+        // which waits for its descriptor.  q4_K rounds of width 8 27.9 -> 27.5 ms, 12B-class q4_0 device-resident rounds 2.97 ->
+        // 2.94 ms; of shorter launches the descriptor costs more (the tiny model 1 % slower).  The boxes depend on R, so the
+        // descriptors are made per launch; launches are captured once into graphs.
         constexpr int P = gemv_stage_tiles<FMT>() / R;
         const int groups = (a.n_row_tiles + R - 1) / R;
         if ((groups + p.gx - 1) / p.gx * ((a.nkp / p.ks + P - 1) / P) >= 4) {

@@ -20,7 +20,7 @@
 //               store f32 rows, or apply GeGLU on interleaved gate/up rows and store the f16 input of the down projection.
 // Tensor memory: columns [0, 256) accumulator, [256, 448) three A stages of 64 columns.
 // What bounds it: the issuing warp (0.32 us per k block of 128 rows x 240 tokens where the products alone take 0.25) and, per item,
-// the epilogue.  12B-class q4_0, 928 tokens in one block: gate/up + GeGLU 168 us (1305 TFLOP/s), down 76 (1432), o 29 (1010),
+// the epilogue; gate/up keeps the tensor pipe busy for 67 % of the active cycles.  12B-class q4_0, 928 tokens in one block: gate/up + GeGLU 168 us (1305 TFLOP/s), down 76 (1432), o 29 (1010),
 // qkv 51 (1139).  Against A expanded into shared memory, one CTA per 128 rows x 256 tokens and 16 bulk copies per weight stage
 // (four launches): 355, 109, 109 (with k slices) and 96 us.  On the way: one copy per row tile instead of a tiled copy kept the copy thread
 // at 115 cycles a copy and every k block at 0.53 us whatever the tile; a barrier pair per k block and operand cost 0.10 us.

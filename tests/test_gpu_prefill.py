@@ -89,7 +89,7 @@ def test_prefill_matmul_geglu_epilogue(lg, port_built, wtype):
 
 @pytest.mark.parametrize("name,n", [("mid", 300), ("mid_k", 300), ("mid", 37)])
 def test_wide_prefill_matches_oracle(lg, port_built, name, n):
-    """model_prefill of n tokens (blocks of up to 256 on the tcgen05 path + a narrow tail): cache rows and the
+    """model_prefill of n tokens (blocks of up to 1024 on the tcgen05 path + a narrow tail): cache rows and the
     logits of the following step against the CPU oracle."""
     from oracle.pyref import PortOracle
     s = synth_module()
