@@ -63,6 +63,30 @@ __device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, ui
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+// two f32 operations in one instruction, each rounded as the scalar one
+__device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+
 // ---- bulk (TMA, non-tensor) global -> shared copy completed on an mbarrier --------------------
 // Bounded-wait probe: waits on an mbarrier nobody completes, for at most `polls` polls, then reports like the kernels do.
 __global__ void lg_wait_probe_kernel(int *err, int polls) {
@@ -380,6 +404,10 @@ struct LgStageMaps { CUtensorMap q, s, d, m; };
 //     fragment once and applies it to the R row tiles: A fragments are one conflict-free 16-byte
 //     shared load per lane, `mma.sync.m16n8k32.s8`, f32 scale-accumulate.  Partial sums of the
 //     warps are added in warp order.
+// Bound by the issue slots of its consumer warps and the hand-over between launches, not by HBM: the same matrix 48 times (in L2)
+// takes 12.6 us where 48 cold ones take 13.4 (12B-class gate/up, 66 MB), without the arithmetic 11.5.  Hence addresses of the shared
+// window (generic ones cost 64-bit arithmetic per load), packed f32 operations, and registers for two CTAs an SM (left to itself
+// the compiler stopped at 56 and spilled): 14.3 -> 13.0 us, down 8.9 -> 8.5, qkv 6.1 -> 5.6, o 4.25 -> 4.04.
 // Every wait is bounded; a timeout raises LG_ERR_MBAR_TIMEOUT and the kernel runs to its end.
 //   * k slices (gridDim.y > 1) either leave one partial result per slice for the consumer to add, or -- cl_ks -- form
 //     a thread-block cluster whose ranks 1.. send their sums into rank 0's shared memory (st.async, counted on an
@@ -511,6 +539,9 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
     if (!ok && threadIdx.x == 0) atomicOr(a.err, LG_ERR_MBAR_TIMEOUT);
     LG_STAMP(a.tag, 2);
     int stage = 0; uint32_t phase = 0;
+    // this lane's places in shared memory (addresses of the shared window: no 64-bit arithmetic in the loop)
+    const uint32_t b_lane = smem_u32(sq) + lane * 8, x_lane = smem_u32(ss) + t * 8;
+    const uint32_t w_lane = smem_u32(ring) + lane * 16, s_lane = smem_u32(ring) + SC_OFF + g * 8;
 
     for (int grp = blockIdx.x; grp < n_groups; grp += gridDim.x) {
         const int rt0 = grp * R;
@@ -526,16 +557,17 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
                 w_v[j] = live ? a.add_w[row] : 0.0f;
             }
         }
-        float acc[R][NP][2];
+        float2 acc[R][NP];                                   // rows g and g + 8 of token 4p + t
         #pragma unroll
         for (int r = 0; r < R; r++)
             #pragma unroll
-            for (int p = 0; p < NP; p++) acc[r][p][0] = acc[r][p][1] = 0.0f;
+            for (int p = 0; p < NP; p++) acc[r][p] = make_float2(0.0f, 0.0f);
 
         for (int c = 0; c < n_chunks; c++) {
             if (ok && !mbar_wait(full + stage, phase)) { ok = false; if (lane == 0) atomicOr(a.err, LG_ERR_MBAR_TIMEOUT); }
             const int np = min(P, nkp_s - c * P);
             const unsigned char *st = ring + (size_t)stage * STAGE;
+            const uint32_t st_w = w_lane + (uint32_t)stage * STAGE, st_s = s_lane + (uint32_t)stage * STAGE;
             for (int pp = warp % PW; pp < np; pp += PW) {
                 uint2 b[2][NP]; float2 xs[2][NP];
                 #pragma unroll
@@ -543,8 +575,9 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
                     #pragma unroll
                     for (int p = 0; p < NP; p++) {
                         const int sbl = (c * P + pp) * 2 + s;
-                        b[s][p] = *(const uint2 *)(sq + ((size_t)p * nsb_s + sbl) * 256 + lane * 8);
-                        xs[s][p] = ss[((size_t)p * nsb_s + sbl) * 4 + t];
+                        b[s][p] = lds64(b_lane + (uint32_t)(p * nsb_s + sbl) * 256);
+                        const uint2 xw = lds64(x_lane + (uint32_t)(p * nsb_s + sbl) * 32);
+                        xs[s][p] = make_float2(__uint_as_float(xw.x), __uint_as_float(xw.y));
                     }
                 #pragma unroll
                 for (int r = 0; r < R; r++) {
@@ -572,52 +605,51 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
                                     mma_s8_k16(cc, h ? w.z : w.x, h ? w.w : w.y, h ? b[s][p].y : b[s][p].x);
                                     const float v0 = (float)((cc[0] << 8) + cc[1]) * xs[s][p].x;
                                     const float v1 = (float)((cc[2] << 8) + cc[3]) * xs[s][p].x;
-                                    acc[r][p][0] = fmaf(v0, e0, acc[r][p][0]);
-                                    acc[r][p][1] = fmaf(v1, e1, acc[r][p][1]);
+                                    acc[r][p] = ffma2(make_float2(v0, v1), make_float2(e0, e1), acc[r][p]);
                                 }
                             }
                             if (FMT == LG_FMT_I8M) {
                                 const float m0 = -16.0f * __uint_as_float(s ? mm.z : mm.x), m1 = -16.0f * __uint_as_float(s ? mm.w : mm.y);
                                 #pragma unroll
                                 for (int p = 0; p < NP; p++) {
-                                    acc[r][p][0] = fmaf(m0, xs[s][p].y, acc[r][p][0]);
-                                    acc[r][p][1] = fmaf(m1, xs[s][p].y, acc[r][p][1]);
+                                    acc[r][p] = ffma2(make_float2(m0, m1), make_float2(xs[s][p].y, xs[s][p].y), acc[r][p]);
                                 }
                             }
                         }
                         continue;
                     }
                     // this lane's 16 bytes: {row g, row g+8} words of sub-block 0, then of sub-block 1
-                    const uint4 w = *(const uint4 *)(st + (size_t)(r * P + pp) * 512 + lane * 16);
-                    const uint2 sw2 = *(const uint2 *)(st + SC_OFF + (size_t)(r * P + pp) * 64 + g * 8);
-                    uint2 dd = make_uint2(0, 0);
-                    if (FMT == LG_FMT_Q4_K) dd = *(const uint2 *)(st + DD_OFF + (size_t)(r * P + pp) * 64 + g * 8);
+                    const uint4 w = lds128(st_w + (uint32_t)(r * P + pp) * 512);
+                    const uint2 sw2 = lds64(st_s + (uint32_t)(r * P + pp) * 64);
+                    float2 kd, km;                           // q4_K: d and -16 dmin of rows g and g + 8
+                    if (FMT == LG_FMT_Q4_K) {
+                        const uint2 dd = lds64(st_s + (DD_OFF - SC_OFF) + (uint32_t)(r * P + pp) * 64);
+                        const float2 r0 = __half22float2(*(const __half2 *)&dd.x), r1 = __half22float2(*(const __half2 *)&dd.y);
+                        kd = make_float2(r0.x, r1.x); km = make_float2(-16.0f * r0.y, -16.0f * r1.y);
+                    }
                     #pragma unroll
                     for (int s = 0; s < 2; s++) {
                         const uint32_t wg = s ? w.z : w.x, wh = s ? w.w : w.y, sw = s ? sw2.y : sw2.x;
                         uint32_t a0 = (wg << 4) & 0xF0F0F0F0u, a2 = wg & 0xF0F0F0F0u;
                         uint32_t a1 = (wh << 4) & 0xF0F0F0F0u, a3 = wh & 0xF0F0F0F0u;
-                        float d0, d1, m0 = 0.0f, m1 = 0.0f;
+                        float2 d, m = make_float2(0.0f, 0.0f);
                         if (FMT == LG_FMT_Q4_0) {
-                            float2 fd = __half22float2(*(const __half2 *)&sw);
-                            d0 = fd.x; d1 = fd.y;
+                            d = __half22float2(*(const __half2 *)&sw);
                         } else {
-                            float2 r0 = __half22float2(*(const __half2 *)&dd.x), r1 = __half22float2(*(const __half2 *)&dd.y);
-                            d0 = r0.x * (float)(sw & 0xff); m0 = 16.0f * (8.0f * d0 - r0.y * (float)((sw >> 8) & 0xff));
-                            d1 = r1.x * (float)((sw >> 16) & 0xff); m1 = 16.0f * (8.0f * d1 - r1.y * (float)(sw >> 24));
+                            // d sc and 16 (8 d sc - dmin m): products of 11 and 6 bits are exact, so only the difference rounds
+                            d = fmul2(kd, make_float2((float)(sw & 0xff), (float)((sw >> 16) & 0xff)));
+                            m = ffma2(km, make_float2((float)((sw >> 8) & 0xff), (float)(sw >> 24)), fmul2(d, make_float2(128.0f, 128.0f)));
                         }
                         #pragma unroll
                         for (int p = 0; p < NP; p++) {
                             int cc[4] = {0, 0, 0, 0};
                             mma_s8(cc, a0, a1, a2, a3, b[s][p].x, b[s][p].y);
-                            float v0 = (float)((cc[0] << 8) + cc[1]) * xs[s][p].x;      // row g,   token 4p+t
-                            float v1 = (float)((cc[2] << 8) + cc[3]) * xs[s][p].x;      // row g+8
-                            acc[r][p][0] = fmaf(v0, d0, acc[r][p][0]);
-                            acc[r][p][1] = fmaf(v1, d1, acc[r][p][1]);
-                            if (FMT == LG_FMT_Q4_K) {     // nibbles are stored as (q-8): add back (8 d sc - dmin m) * sum(x)
-                                acc[r][p][0] = fmaf(m0, xs[s][p].y, acc[r][p][0]);
-                                acc[r][p][1] = fmaf(m1, xs[s][p].y, acc[r][p][1]);
-                            }
+                            // rows g and g+8 of token 4p+t, side by side
+                            const float2 v = fmul2(make_float2((float)((cc[0] << 8) + cc[1]), (float)((cc[2] << 8) + cc[3])),
+                                                   make_float2(xs[s][p].x, xs[s][p].x));
+                            acc[r][p] = ffma2(v, d, acc[r][p]);
+                            if (FMT == LG_FMT_Q4_K)      // nibbles are stored as (q-8): add back (8 d sc - dmin m) * sum(x)
+                                acc[r][p] = ffma2(m, make_float2(xs[s][p].y, xs[s][p].y), acc[r][p]);
                         }
                     }
                 }
@@ -633,8 +665,8 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
         for (int r = 0; r < R; r++)
             #pragma unroll
             for (int p = 0; p < NP; p++) {
-                red[(warp * R * NP + r * NP + p) * 64 + t * 16 + g] = acc[r][p][0];
-                red[(warp * R * NP + r * NP + p) * 64 + t * 16 + g + 8] = acc[r][p][1];
+                red[(warp * R * NP + r * NP + p) * 64 + t * 16 + g] = acc[r][p].x;
+                red[(warp * R * NP + r * NP + p) * 64 + t * 16 + g + 8] = acc[r][p].y;
             }
         consumer_sync();
         float fs[SLOTS];
@@ -789,10 +821,10 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
     }
 }
 template <int R, int NP, int FMT, int EPI>
-__global__ void __launch_bounds__(LG_GEMV_THREADS) lg_gemv_kernel(LgGemvArgs a) { gemv_body<R, NP, FMT, EPI, false>(nullptr, a); }
+__global__ void __launch_bounds__(LG_GEMV_THREADS, 2) lg_gemv_kernel(LgGemvArgs a) { gemv_body<R, NP, FMT, EPI, false>(nullptr, a); }
 // the same with stages of several row tiles brought by tiled copies
 template <int R, int NP, int FMT, int EPI>
-__global__ void __launch_bounds__(LG_GEMV_THREADS) lg_gemv_tiled_kernel(const __grid_constant__ LgStageMaps maps, const __grid_constant__ LgGemvArgs a) {
+__global__ void __launch_bounds__(LG_GEMV_THREADS, 2) lg_gemv_tiled_kernel(const __grid_constant__ LgStageMaps maps, const __grid_constant__ LgGemvArgs a) {
     gemv_body<R, NP, FMT, EPI, true>(&maps, a);
 }
 
