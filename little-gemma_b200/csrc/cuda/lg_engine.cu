@@ -171,35 +171,41 @@ void free_wmat(WMat &W) { cudaFree(W.wq); cudaFree(W.ws); cudaFree(W.wd); cudaFr
 // launch helpers
 // ------------------------------------------------------------------------------------------
 
-struct GemvPlan { int r, ks, gx, ns, cl; size_t smem; };
-// dynamic shared memory of the small-M matmul: panel slice | ring | warp partials | item sums | peers' sums (cluster) | mbarriers
-size_t gemv_smem_bytes(int np, int nkp_slice, int r, int fmt, int ns, int cl_ks) {
+struct GemvPlan { int r, ks, gx, ns, cl, teams; size_t smem; };      // gx: teams along x (CTAs of one team, or halves of CTAs of two)
+// dynamic shared memory of the small-M matmul: panel slice | per team: ring | warp partials | item sums | peers' sums (cluster) | mbarriers
+size_t gemv_smem_bytes(int np, int nkp_slice, int r, int fmt, int ns, int cl_ks, int teams = 1) {
     const int stage = fmt == LG_FMT_Q4_0 ? gemv_stage_bytes<LG_FMT_Q4_0>() : fmt == LG_FMT_Q4_K ? gemv_stage_bytes<LG_FMT_Q4_K>()
                     : fmt == LG_FMT_I8 ? gemv_stage_bytes<LG_FMT_I8>() : gemv_stage_bytes<LG_FMT_I8M>();
-    return (size_t)np * nkp_slice * 2 * (256 + 32) + 128 + (size_t)ns * stage + (size_t)(LG_GEMV_CW + 1) * r * np * 64 * 4
-         + (cl_ks > 1 ? (size_t)(cl_ks - 1) * r * np * 64 * 4 : 0) + (2 * LG_GEMV_STAGES_MAX + 2) * 8 + 16;
+    return (size_t)np * nkp_slice * 2 * (256 + 32) + 128 + 16
+         + teams * ((size_t)ns * stage + (size_t)(LG_GEMV_CW + 1) * r * np * 64 * 4 + (cl_ks > 1 ? (size_t)(cl_ks - 1) * r * np * 64 * 4 : 0) + (2 * LG_GEMV_STAGES_MAX + 2) * 8);
 }
 // most dynamic shared memory a CTA may take while two CTAs still share an SM (228 KB per SM, 1 KB reserved per CTA), less
 // the kernel's few static bytes
 constexpr size_t GEMV_SMEM_2CTA = (233472 - 2 * 1024) / 2 - 256;
+constexpr size_t GEMV_SMEM_2TEAM = 232448 - 256;                 // one CTA per SM
 // One more ring stage where two CTAs per SM still fit: a short kernel (an item or two per CTA) then has its whole share of
 // the weights in flight before the activations arrive instead of refilling a stage behind a full memory latency.
-void gemv_pick_stages(GemvPlan &p, int np, int nkp_slice, int fmt) {
+// may_team: where two CTAs do not fit an SM (two panels of activations), one CTA of two teams that share the panel does.
+void gemv_pick_stages(GemvPlan &p, int np, int nkp_slice, int fmt, bool may_team = false) {
     static const int max_ns = env_int("LG_GEMV_STAGES", LG_GEMV_STAGES_MAX);
     const int cl_ks = p.cl ? p.ks : 0;
-    p.ns = LG_GEMV_STAGES;
+    p.ns = LG_GEMV_STAGES; p.teams = 1;
     p.smem = gemv_smem_bytes(np, nkp_slice, p.r, fmt, p.ns, cl_ks);
-    if (max_ns >= 4 && p.smem <= GEMV_SMEM_2CTA) {
-        const size_t s4 = gemv_smem_bytes(np, nkp_slice, p.r, fmt, 4, cl_ks);
-        if (s4 <= GEMV_SMEM_2CTA) { p.ns = 4; p.smem = s4; }
+    if (may_team && np == 2 && p.smem > GEMV_SMEM_2CTA && gemv_smem_bytes(np, nkp_slice, p.r, fmt, p.ns, cl_ks, 2) <= GEMV_SMEM_2TEAM) p.teams = 2;
+    const size_t limit = p.teams == 2 ? GEMV_SMEM_2TEAM : GEMV_SMEM_2CTA;
+    p.smem = gemv_smem_bytes(np, nkp_slice, p.r, fmt, p.ns, cl_ks, p.teams);
+    if (max_ns >= 4 && p.smem <= limit) {
+        const size_t s4 = gemv_smem_bytes(np, nkp_slice, p.r, fmt, 4, cl_ks, p.teams);
+        if (s4 <= limit) { p.ns = 4; p.smem = s4; }
     }
 }
 constexpr size_t GEMV_SMEM_MAX = 200 * 1024, ATTN_SMEM_MAX = 220 * 1024;
 constexpr int MAX_KV_HEADS = 64;
 
-template <int R, int NP, int FMT, int EPI> void gemv_attr() {
-    LG_CHECK(cudaFuncSetAttribute(lg_gemv_kernel<R, NP, FMT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMV_SMEM_MAX));
-    if constexpr (R > 1) LG_CHECK(cudaFuncSetAttribute(lg_gemv_tiled_kernel<R, NP, FMT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMV_SMEM_MAX));
+template <int R, int NP, int FMT, int EPI, int TEAMS = 1> void gemv_attr() {
+    LG_CHECK(cudaFuncSetAttribute(lg_gemv_kernel<R, NP, FMT, EPI, TEAMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMV_SMEM_2TEAM));
+    if constexpr (R > 1) LG_CHECK(cudaFuncSetAttribute(lg_gemv_tiled_kernel<R, NP, FMT, EPI, TEAMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMV_SMEM_2TEAM));
+    if constexpr (NP == 2 && TEAMS == 1) gemv_attr<R, NP, FMT, EPI, 2>();
 }
 template <int R, int FMT> void gemv_attr_rf() {
     gemv_attr<R, 1, FMT, LG_EPI_STORE>(); gemv_attr<R, 2, FMT, LG_EPI_STORE>();
@@ -303,19 +309,20 @@ GemvPlan plan_gemv(const Engine *e, const WMat &W, int np_actual, int want_ks, b
     // thread-block cluster that adds its partial sums in rank 0 -- possible with one item per CTA and a portable cluster size.
     static const int cl_on = env_int("LG_GEMV_CLUSTER", 1);
     if (complete && cl_on && p.ks > 1 && p.ks <= LG_GEMV_CL_MAX && waves == 1) p.cl = 1;
-    gemv_pick_stages(p, np_actual, (W.nkp + p.ks - 1) / p.ks + 1, W.fmt);
+    const bool crowded = p.gx * p.ks > e->sm_count;                        // more items at once than SMs
+    gemv_pick_stages(p, np_actual, (W.nkp + p.ks - 1) / p.ks + 1, W.fmt, crowded);
     if (p.cl && (gemv_smem_bytes(2, (W.nkp + p.ks - 1) / p.ks + 1, p.r, W.fmt, LG_GEMV_STAGES, p.ks) > GEMV_SMEM_MAX)) {
         p.cl = 0;
-        gemv_pick_stages(p, np_actual, (W.nkp + p.ks - 1) / p.ks + 1, W.fmt);
+        gemv_pick_stages(p, np_actual, (W.nkp + p.ks - 1) / p.ks + 1, W.fmt, crowded);
     }
 
     return p;
 }
 
-template <int R, int NP, int FMT, int EPI>
+template <int R, int NP, int FMT, int EPI, int TEAMS>
 void launch_gemv_t(Engine *e, const LgGemvArgs &a, const GemvPlan &p) {
-    if (p.smem > GEMV_SMEM_MAX) { fprintf(stderr, "lg_b200: matmul slice needs %zu bytes of shared memory\n", p.smem); exit(1); }
-    dim3 grid(p.gx, p.ks);
+    if (TEAMS == 1 && p.smem > GEMV_SMEM_MAX) { fprintf(stderr, "lg_b200: matmul slice needs %zu bytes of shared memory\n", p.smem); exit(1); }
+    const dim3 grid((p.gx + TEAMS - 1) / TEAMS, p.ks), block(TEAMS * LG_GEMV_THREADS);
     if constexpr (R > 1) {
         // Tiled copies where a CTA streams at least four stages (the deepest ring): they issue R times fewer copies, the first of
         // which waits for its descriptor.  q4_K rounds of width 8 27.9 -> 27.5 ms, 12B-class q4_0 device-resident rounds 2.97 ->
@@ -329,13 +336,18 @@ void launch_gemv_t(Engine *e, const LgGemvArgs &a, const GemvPlan &p) {
             maps.s = tile_boxes_map(a.ws, 64, a.nkp, a.n_row_tiles, P, R);
             if (FMT != LG_FMT_Q4_0) maps.d = tile_boxes_map(a.wd, 64, a.nkp, a.n_row_tiles, P, R);
             if (FMT == LG_FMT_I8M) maps.m = tile_boxes_map(a.wm, 128, a.nkp, a.n_row_tiles, P, R);
-            if (p.cl) launch_k_cluster_y(e, (lg_gemv_tiled_kernel<R, NP, FMT, EPI>), dim3(grid), dim3(LG_GEMV_THREADS), p.smem, maps, a);
-            else launch_k(e, (lg_gemv_tiled_kernel<R, NP, FMT, EPI>), dim3(grid), dim3(LG_GEMV_THREADS), p.smem, maps, a);
+            if (p.cl) launch_k_cluster_y(e, (lg_gemv_tiled_kernel<R, NP, FMT, EPI, TEAMS>), dim3(grid), dim3(block), p.smem, maps, a);
+            else launch_k(e, (lg_gemv_tiled_kernel<R, NP, FMT, EPI, TEAMS>), dim3(grid), dim3(block), p.smem, maps, a);
             return;
         }
     }
-    if (p.cl) launch_k_cluster_y(e, (lg_gemv_kernel<R, NP, FMT, EPI>), dim3(grid), dim3(LG_GEMV_THREADS), p.smem, a);
-    else launch_k(e, (lg_gemv_kernel<R, NP, FMT, EPI>), dim3(grid), dim3(LG_GEMV_THREADS), p.smem, a);
+    if (p.cl) launch_k_cluster_y(e, (lg_gemv_kernel<R, NP, FMT, EPI, TEAMS>), dim3(grid), dim3(block), p.smem, a);
+    else launch_k(e, (lg_gemv_kernel<R, NP, FMT, EPI, TEAMS>), dim3(grid), dim3(block), p.smem, a);
+}
+template <int R, int NP, int FMT, int EPI>
+void launch_gemv_t(Engine *e, const LgGemvArgs &a, const GemvPlan &p) {
+    if constexpr (NP == 2) if (p.teams == 2) { launch_gemv_t<R, NP, FMT, EPI, 2>(e, a, p); return; }
+    launch_gemv_t<R, NP, FMT, EPI, 1>(e, a, p);
 }
 // dispatch on the weight format (a template parameter of the kernel)
 template <int R, int NP, int EPI>
@@ -381,7 +393,7 @@ void launch_gemv(Engine *e, const WMat &W, const LgPanel &X, int M, float *out, 
     if (sums && p.ks > 1 && !p.cl) { fprintf(stderr, "lg_b200: the SUMS epilogue needs complete rows (see sums_ok)\n"); exit(1); }
     if (epi == LG_EPI_GATE) {                    // one panel group (32 rows) per item, the whole k range in one CTA
         p.r = 2; p.ks = 1; p.cl = 0; p.gx = std::max(1, std::min(W.n_row_tiles / 2, e->sm_count * 2));
-        gemv_pick_stages(p, np, W.nkp + 1, W.fmt);
+        gemv_pick_stages(p, np, W.nkp + 1, W.fmt, p.gx > e->sm_count);
     }
     LgGemvArgs a{};
     a.wq = W.wq; a.ws = W.ws; a.wd = W.wd; a.wm = W.wm; a.x = X; a.nkp = W.nkp; a.n_row_tiles = W.n_row_tiles; a.kslices = p.ks;
@@ -393,7 +405,7 @@ void launch_gemv(Engine *e, const WMat &W, const LgPanel &X, int M, float *out, 
     a.tag = (int)e->launches; a.ns = p.ns;
     if (X.nsb * 32 != W.k) { fprintf(stderr, "lg_b200: panel width %d does not match matrix k %d\n", X.nsb * 32, W.k); exit(1); }
     if (x.ks_out) *x.ks_out = p.cl ? 1 : p.ks;
-    if (x.gx_out) *x.gx_out = p.gx;
+    if (x.gx_out) *x.gx_out = (p.gx + p.teams - 1) / p.teams * p.teams;
     if (x.groups_out) *x.groups_out = (W.n_row_tiles + p.r - 1) / p.r;
     if (sums) {
         if (np == 1) {

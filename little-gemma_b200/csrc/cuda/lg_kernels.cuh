@@ -375,8 +375,8 @@ enum { LG_EPI_STORE = 0, LG_EPI_HEAD = 1, LG_EPI_GEGLU = 2, LG_EPI_SUMS = 3, LG_
 #define LG_GEMV_STAGE_TILES 32         // 16x64 q4 weight tiles per stage (R row tiles x 32/R positions); i8 tiles: 16
 template <int FMT> __host__ __device__ constexpr int gemv_stage_tiles() { return FMT >= LG_FMT_I8 ? 16 : LG_GEMV_STAGE_TILES; }
 
-__device__ __forceinline__ void consumer_sync() {       // the consumer warps only; the producer warp never joins
-    asm volatile("bar.sync 1, %0;" :: "n"(LG_GEMV_CW * 32) : "memory");
+__device__ __forceinline__ void consumer_sync(int team) {       // a team's consumer warps only; its producer warp never joins
+    asm volatile("bar.sync %0, %1;" :: "r"(1 + team), "n"(LG_GEMV_CW * 32) : "memory");
 }
 
 // Bytes of one ring stage: nibbles, scales (and the {d,dmin} pairs of q4_K)
@@ -408,12 +408,15 @@ struct LgStageMaps { CUtensorMap q, s, d, m; };
 // takes 12.6 us where 48 cold ones take 13.4 (12B-class gate/up, 66 MB), without the arithmetic 11.5.  Hence addresses of the shared
 // window (generic ones cost 64-bit arithmetic per load), packed f32 operations, and registers for two CTAs an SM (left to itself
 // the compiler stopped at 56 and spilled): 14.3 -> 13.0 us, down 8.9 -> 8.5, qkv 6.1 -> 5.6, o 4.25 -> 4.04.
+// Two panels (5..8 tokens) of a 3840-column matrix leave room for one CTA per SM: then a CTA has two teams of consumers, each with a
+// producer, ring and items of its own, behind ONE panel.  Gate/up 23.9 -> 17.7 us, down 15.2 -> 10.8, qkv 8.9 -> 6.9, o 7.2 -> 5.2.  For one panel
+// two CTAs are as good or better (12B-class verify step of width 4: 2.35 against 2.40 ms).
 // Every wait is bounded; a timeout raises LG_ERR_MBAR_TIMEOUT and the kernel runs to its end.
 //   * k slices (gridDim.y > 1) either leave one partial result per slice for the consumer to add, or -- cl_ks -- form
 //     a thread-block cluster whose ranks 1.. send their sums into rank 0's shared memory (st.async, counted on an
 //     mbarrier of rank 0), so that rank 0 runs the epilogue on complete rows.
 // Dynamic shared memory: panel q | panel s | ring | warp partials | item sums | peers' sums (cluster) | mbarriers
-template <int R, int NP, int FMT, int EPI, bool TILED>
+template <int R, int NP, int FMT, int EPI, int TEAMS, bool TILED>
 __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvArgs &a) {
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr int ST = gemv_stage_tiles<FMT>();
@@ -428,7 +431,10 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
     constexpr int SC_OFF = ST * TB;                          // scales after the weights, {d,dmin} / integer scales after them, offsets last
     constexpr int DD_OFF = SC_OFF + ST * 64;
     constexpr int MM_OFF = DD_OFF + ST * 64;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    // a CTA is one or two teams, each with ring, sums and items of its own; the panel is shared
+    const int team = TEAMS == 1 ? 0 : threadIdx.x / LG_GEMV_THREADS, tid = threadIdx.x - team * LG_GEMV_THREADS;
+    const int vcta = blockIdx.x + team * gridDim.x, n_vctas = TEAMS * gridDim.x;
+    const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int ks = blockIdx.y;
     const int kp0 = (int)((long long)a.nkp * ks / a.kslices), kp1 = (int)((long long)a.nkp * (ks + 1) / a.kslices);
     const int nkp_s = kp1 - kp0, nsb_s = nkp_s * 2;
@@ -440,18 +446,21 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
     float2 *ss = (float2 *)(smem + (size_t)NP * nsb_s * 256);
     unsigned char *ring = (unsigned char *)(ss + (size_t)NP * nsb_s * 4);
     ring = (unsigned char *)(((uintptr_t)ring + 127) & ~(uintptr_t)127);
+    const int cred_n = cl ? (a.kslices - 1) * RN : 0;
+    ring += (size_t)team * ((size_t)NS * STAGE + (size_t)((LG_GEMV_CW + 1) * RN + cred_n) * 4);
     float *red = (float *)(ring + (size_t)NS * STAGE);
     float *fin = red + LG_GEMV_CW * RN;                      // [RN] complete sums of the item (GeGLU, SUMS)
     float *cred = fin + RN;                                  // cluster reduce: [kslices - 1][RN] partials of ranks 1.. (rank 0's copy is used)
-    uint64_t *full = (uint64_t *)(cred + (cl ? (a.kslices - 1) * RN : 0));
-    uint64_t *empty = full + NS, *pbar = empty + NS, *cbar = pbar + 1;
+    // mbarriers behind the last team's area: the panel's, then each team's
+    uint64_t *pbar = (uint64_t *)((unsigned char *)(cred + cred_n) + (size_t)(TEAMS - 1 - team) * ((size_t)NS * STAGE + (size_t)((LG_GEMV_CW + 1) * RN + cred_n) * 4));
+    uint64_t *full = pbar + 1 + team * (2 * NS + 1), *empty = full + NS, *cbar = empty + NS;
 
     pdl_launch();
     LG_STAMP(a.tag, 0);
     LG_STAMP_KIND(a.tag, 1 + EB);
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
         for (int i = 0; i < NS; i++) { mbar_init(full + i, 1); mbar_init(empty + i, LG_GEMV_CW); }
-        mbar_init(pbar, 1);
+        if (team == 0) mbar_init(pbar, 1);
         mbar_init(cbar, 1);
         // rank 0 of a cluster expects every peer's RN partial sums (once: a cluster-reduced launch has one item per CTA)
         if (cl && ks == 0) mbar_expect_tx(cbar, (uint32_t)(a.kslices - 1) * RN * 4);
@@ -466,10 +475,10 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
         if (lane == 0) {
             int stage = 0; uint32_t phase = 0; bool panel_sent = false, ok = true;
             // stages this CTA will stream in all, and how many of them go out before the dependency wait: a full ring
-            const int my_groups = blockIdx.x < n_groups ? (n_groups - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+            const int my_groups = vcta < n_groups ? (n_groups - vcta + n_vctas - 1) / n_vctas : 0;
             const int total_stages = my_groups * n_chunks, early = min(NS, total_stages);
             int issued = 0;
-            for (int grp = blockIdx.x; grp < n_groups && ok; grp += gridDim.x) {
+            for (int grp = vcta; grp < n_groups && ok; grp += n_vctas) {
                 const size_t tile_base = (size_t)grp * R * a.nkp + kp0;
                 for (int c = 0; c < n_chunks && ok; c++) {
                     if (!mbar_wait(empty + stage, phase ^ 1)) { atomicOr(a.err, LG_ERR_MBAR_TIMEOUT); ok = false; break; }
@@ -510,6 +519,8 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
                             ok = false;
                             break;
                         }
+                        panel_sent = true;
+                        if (team != 0) continue;                 // one panel for all
                         uint32_t qb = (uint32_t)nsb_s * 256, sb = (uint32_t)nsb_s * 32;
                         mbar_expect_tx(pbar, NP * (qb + sb));
                         #pragma unroll
@@ -517,7 +528,6 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
                             bulk_g2s(sq + (size_t)p * qb, a.x.q + ((size_t)p * a.x.nsb + kp0 * 2) * 256, qb, pbar);
                             bulk_g2s(ss + (size_t)p * nsb_s * 4, a.x.s + ((size_t)p * a.x.nsb + kp0 * 2) * 4, sb, pbar);
                         }
-                        panel_sent = true;
                     }
                 }
             }
@@ -536,21 +546,21 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
     LG_STAMP(a.tag, 1);
     if (a.skip && *a.skip) return;
     bool ok = mbar_wait(pbar, 0);
-    if (!ok && threadIdx.x == 0) atomicOr(a.err, LG_ERR_MBAR_TIMEOUT);
+    if (!ok && tid == 0) atomicOr(a.err, LG_ERR_MBAR_TIMEOUT);
     LG_STAMP(a.tag, 2);
     int stage = 0; uint32_t phase = 0;
     // this lane's places in shared memory (addresses of the shared window: no 64-bit arithmetic in the loop)
     const uint32_t b_lane = smem_u32(sq) + lane * 8, x_lane = smem_u32(ss) + t * 8;
     const uint32_t w_lane = smem_u32(ring) + lane * 16, s_lane = smem_u32(ring) + SC_OFF + g * 8;
 
-    for (int grp = blockIdx.x; grp < n_groups; grp += gridDim.x) {
+    for (int grp = vcta; grp < n_groups; grp += n_vctas) {
         const int rt0 = grp * R;
         // SUMS: this thread's residual elements and norm weights, fetched now and used after the main loop
         float x_v[SLOTS], w_v[SLOTS];
         if (EB == LG_EPI_SUMS && ks == 0) {
             #pragma unroll
             for (int j = 0; j < SLOTS; j++) {
-                const int idx = threadIdx.x + j * CT;
+                const int idx = tid + j * CT;
                 const int rp = idx >> 6, r = rp / NP, p = rp % NP, tok = p * 4 + ((idx >> 4) & 3), row = (rt0 + r) * 16 + (idx & 15);
                 const bool live = idx < RN && tok < a.M && row < a.n_cols;
                 x_v[j] = live ? __ldcg(a.xres + (size_t)tok * a.ldx + row) : 0.0f;
@@ -668,11 +678,11 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
                 red[(warp * R * NP + r * NP + p) * 64 + t * 16 + g] = acc[r][p].x;
                 red[(warp * R * NP + r * NP + p) * 64 + t * 16 + g + 8] = acc[r][p].y;
             }
-        consumer_sync();
+        consumer_sync(team);
         float fs[SLOTS];
         #pragma unroll
         for (int j = 0; j < SLOTS; j++) {
-            const int idx = threadIdx.x + j * CT;
+            const int idx = tid + j * CT;
             float sum = 0.0f;
             if (idx < RN) {
                 #pragma unroll
@@ -687,10 +697,10 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
             if (ks != 0) {
                 #pragma unroll
                 for (int j = 0; j < SLOTS; j++) {
-                    const int idx = threadIdx.x + j * CT;
+                    const int idx = tid + j * CT;
                     if (idx < RN) dsmem_st_async_f32(cred + (size_t)(ks - 1) * RN + idx, cbar, 0, fs[j]);
                 }
-                consumer_sync();
+                consumer_sync(team);
                 continue;
             }
             // (waited for even after an earlier timeout: this CTA must not leave while peers still send into it)
@@ -698,7 +708,7 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
             LG_STAMP(a.tag, 4);
             #pragma unroll
             for (int j = 0; j < SLOTS; j++) {
-                const int idx = threadIdx.x + j * CT;
+                const int idx = tid + j * CT;
                 if (idx < RN)
                     for (int r2 = 1; r2 < a.kslices; r2++) fs[j] += cred[(size_t)(r2 - 1) * RN + idx];
             }
@@ -706,10 +716,10 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
         if (EB == LG_EPI_GEGLU) {
             #pragma unroll
             for (int j = 0; j < SLOTS; j++) {
-                const int idx = threadIdx.x + j * CT;
+                const int idx = tid + j * CT;
                 if (idx < RN) fin[idx] = fs[j];
             }
-            consumer_sync();
+            consumer_sync(team);
             // one warp per token: lane o = output (r, row8) of this item's 32 outputs
             for (int tok = warp; tok < NP * 4 && tok < a.M; tok += LG_GEMV_CW) {
                 const int p = tok >> 2, tl = tok & 3, row8 = lane & 7;
@@ -725,10 +735,10 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
         } else if (EB == LG_EPI_GATE) {
             #pragma unroll
             for (int j = 0; j < SLOTS; j++) {
-                const int idx = threadIdx.x + j * CT;
+                const int idx = tid + j * CT;
                 if (idx < RN) fin[idx] = fs[j];
             }
-            consumer_sync();
+            consumer_sync(team);
             // one warp per token: lane = row of the item's 32 rows (R = 2)
             for (int tok = warp; tok < NP * 4 && tok < a.M; tok += LG_GEMV_CW) {
                 const int p = tok >> 2, tl = tok & 3, r = lane >> 4, row = (rt0 + r) * 16 + (lane & 15);
@@ -740,7 +750,7 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
             float4 part[SLOTS];
             #pragma unroll
             for (int j = 0; j < SLOTS; j++) {
-                int idx = threadIdx.x + j * CT;
+                int idx = tid + j * CT;
                 part[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 if (idx < RN) {
                     int rp = idx >> 6, r = rp / NP, p = rp % NP, tok = p * 4 + ((idx >> 4) & 3);
@@ -774,12 +784,12 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
                         v.x += __shfl_xor_sync(0xffffffffu, v.x, o); v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
                         v.z += __shfl_xor_sync(0xffffffffu, v.z, o); v.w += __shfl_xor_sync(0xffffffffu, v.w, o);
                     }
-                    const int idx = threadIdx.x + j * CT;
+                    const int idx = tid + j * CT;
                     if (idx < RN && (idx & 15) == 0) hs[idx >> 4] = v;
                 }
-                consumer_sync();
-                if (threadIdx.x < a.M) {
-                    const int tok = threadIdx.x, p = tok >> 2, tl = tok & 3;
+                consumer_sync(team);
+                if (tid < a.M) {
+                    const int tok = tid, p = tok >> 2, tl = tok & 3;
                     float4 tot = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     #pragma unroll
                     for (int r = 0; r < R; r++) {
@@ -790,7 +800,7 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
                 }
             }
         }
-        consumer_sync();
+        consumer_sync(team);
         LG_STAMP(a.tag, 6);
     }
 
@@ -799,12 +809,12 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
         float *cv = red; int *ci = (int *)(red + RN); float *c2 = red + 2 * RN;
         #pragma unroll
         for (int j = 0; j < SLOTS; j++) {
-            int idx = threadIdx.x + j * CT;
+            int idx = tid + j * CT;
             if (idx < RN) { cv[idx] = best_v[j]; ci[idx] = best_i[j]; c2[idx] = sec_v[j]; }
         }
-        consumer_sync();
-        if (threadIdx.x < a.M) {
-            int tok = threadIdx.x, p = tok >> 2, tl = tok & 3;
+        consumer_sync(team);
+        if (tid < a.M) {
+            int tok = tid, p = tok >> 2, tl = tok & 3;
             float bv = -INFINITY, s2 = -INFINITY; int bi = 0x7fffffff;
             for (int r = 0; r < R; r++)
                 for (int row = 0; row < 16; row++) {
@@ -814,18 +824,18 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
                     else s2 = fmaxf(s2, v);
                     s2 = fmaxf(s2, c2[idx]);
                 }
-            a.amax_val[(size_t)blockIdx.x * LG_MAXM + tok] = bv;
-            a.amax_idx[(size_t)blockIdx.x * LG_MAXM + tok] = bi;
-            if (a.amax_val2) a.amax_val2[(size_t)blockIdx.x * LG_MAXM + tok] = s2;
+            a.amax_val[(size_t)vcta * LG_MAXM + tok] = bv;
+            a.amax_idx[(size_t)vcta * LG_MAXM + tok] = bi;
+            if (a.amax_val2) a.amax_val2[(size_t)vcta * LG_MAXM + tok] = s2;
         }
     }
 }
-template <int R, int NP, int FMT, int EPI>
-__global__ void __launch_bounds__(LG_GEMV_THREADS, 2) lg_gemv_kernel(LgGemvArgs a) { gemv_body<R, NP, FMT, EPI, false>(nullptr, a); }
+template <int R, int NP, int FMT, int EPI, int TEAMS>
+__global__ void __launch_bounds__(TEAMS * LG_GEMV_THREADS, 2 / TEAMS) lg_gemv_kernel(LgGemvArgs a) { gemv_body<R, NP, FMT, EPI, TEAMS, false>(nullptr, a); }
 // the same with stages of several row tiles brought by tiled copies
-template <int R, int NP, int FMT, int EPI>
-__global__ void __launch_bounds__(LG_GEMV_THREADS, 2) lg_gemv_tiled_kernel(const __grid_constant__ LgStageMaps maps, const __grid_constant__ LgGemvArgs a) {
-    gemv_body<R, NP, FMT, EPI, true>(&maps, a);
+template <int R, int NP, int FMT, int EPI, int TEAMS>
+__global__ void __launch_bounds__(TEAMS * LG_GEMV_THREADS, 2 / TEAMS) lg_gemv_tiled_kernel(const __grid_constant__ LgStageMaps maps, const __grid_constant__ LgGemvArgs a) {
+    gemv_body<R, NP, FMT, EPI, TEAMS, true>(&maps, a);
 }
 
 // Merge the per-CTA argmax candidates: out[tok] = index of the largest logit, lowest index on ties.
