@@ -14,22 +14,27 @@
 // speculative stream byte-identical to plain decoding.
 #pragma once
 #include "lg_kernels.cuh"
+#include "lg_attn_cluster.cuh"         // kv_at
 
 #define LG_DEEP_S 64
 
-// dynamic smem: Qhi | Qlo [NQ16][HD+8] f16 | K [64][HD+8] | V [64][HD+8] | scores 2 x [NQ16][64] f32 | Phi | Plo [NQ16][72] f16 | m, l, alpha [NQ16][3]
-template <int HD, int MTM>      // MTM = 16-row query blocks the CTA carries accumulators for (>= nq16 / 16)
-__global__ void __launch_bounds__(LG_ATTN_THREADS) lg_attn_deep_kernel(LgAttnArgs a) {
-    extern __shared__ __align__(128) unsigned char smem[];
+// dynamic smem (1024-byte aligned): K | V tile [HD/64][64][64] f16 swizzled | Qhi | Qlo [NQ16][HD+8] f16 | scores 2 x [NQ16][64] f32
+//               | Phi | Plo [NQ16][72] f16 | m, l, alpha [NQ16][3] | new K / V rows [2 LG_MAXM][HD] f16
+template <int HD>
+__global__ void __launch_bounds__(LG_ATTN_THREADS)
+lg_attn_deep_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constant__ CUtensorMap tmv, LgAttnArgs a) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ float s_qn[HD], s_kn[HD];
+    __shared__ __align__(8) uint64_t kbar, vbar;
     pdl_launch();
     LG_STAMP_KIND(a.tag, 5);
+    if (threadIdx.x == 0) { mbar_init(&kbar, 1); mbar_init(&vbar, 1); }
     if (!a.q_ready)
         for (int i = threadIdx.x; i < HD; i += LG_ATTN_THREADS) { s_qn[i] = a.q_norm[i]; s_kn[i] = a.k_norm ? a.k_norm[i] : 1.0f; }
     if (!a.early_kv) pdl_wait();
     constexpr int S = LG_DEEP_S, LDH = HD + 8, LDP = S + 8, PER = HD / 64, HALF = HD / 2, NW = LG_ATTN_THREADS / 32;
     const int G = a.G;
-    const int kvh = blockIdx.x, gqa = a.H / a.Hkv, nq = gqa * a.M, nq16 = (nq + 15) & ~15, nmt = nq16 / 16;
+    const int kvh = blockIdx.x, gqa = a.H / a.Hkv, nq = gqa * a.M, nq16 = (nq + 15) & ~15;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int pos0 = *a.pos;
     const int p_first = pos0 + a.qpos_off, p_last = pos0 + a.M - 1 + a.qpos_off;
@@ -43,46 +48,28 @@ __global__ void __launch_bounds__(LG_ATTN_THREADS) lg_attn_deep_kernel(LgAttnArg
     const int T0 = max(SP * G, t_lo), T1 = min(SP * G + G - 1, t_hi);
     const bool writes_kv = a.owns_kv && !a.q_ready;
 
-    __half *qhi = (__half *)smem, *qlo = qhi + (size_t)nq16 * LDH;
-    __half *sk = qlo + (size_t)nq16 * LDH, *sv = sk + (size_t)S * LDH;
-    float *sc = (float *)(sv + (size_t)S * LDH), *sc2 = sc + (size_t)nq16 * S;    // scores: lower / upper half of the head dims
+    unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    __half *sk = (__half *)smem, *sv = sk + (size_t)S * HD;
+    __half *qhi = sv + (size_t)S * HD, *qlo = qhi + (size_t)nq16 * LDH;
+    float *sc = (float *)(qlo + (size_t)nq16 * LDH), *sc2 = sc + (size_t)nq16 * S;    // scores: lower / upper half of the head dims
     __half *phi = (__half *)(sc2 + (size_t)nq16 * S), *plo = phi + (size_t)nq16 * LDP;
     float *row_m = (float *)(plo + (size_t)nq16 * LDP), *row_l = row_m + nq16, *row_a = row_l + nq16;
+    __half *kvnew = (__half *)(row_a + nq16);                   // the block's own K / V rows (row 2 tok + isv)
 
-    constexpr int CH = HD / 8;
-    auto load_tile = [&](int T) {
-        for (int i = threadIdx.x; i < S * CH; i += LG_ATTN_THREADS) {
-            const int key = i / CH, c = i % CH, p = T * S + key;
-            __half *dk = sk + (size_t)key * LDH + c * 8, *dv = sv + (size_t)key * LDH + c * 8;
-            if (p <= p_last && !(writes_kv && p >= pos0)) {
-                const size_t off = (size_t)(p % a.seq) * a.kv_dim + (size_t)kvh * HD + c * 8;
-                cp_async16(dk, a.kc + off);
-                cp_async16(dv, a.vc + off);
-            } else if (p > p_last) {
-                *(uint4 *)dk = make_uint4(0, 0, 0, 0);
-                *(uint4 *)dv = make_uint4(0, 0, 0, 0);
-            }
-        }
+    // one thread sends a tile's boxes; rows past the last position arrive as the cache holds them and meet zero weights
+    auto load_rows = [&](int T, const CUtensorMap *map, __half *dst, uint64_t *bar) {
+        mbar_expect_tx(bar, (uint32_t)S * HD * 2);
+        const int y = (int)(((long long)T * S) % a.seq);
+        #pragma unroll
+        for (int c = 0; c < HD / 64; c++) tma_load_2d(dst + (size_t)c * S * 64, map, kvh * HD + c * 64, y, bar);
     };
-    load_tile(T0);
+    if (threadIdx.x == 0) { load_rows(T0, &tmk, sk, &kbar); load_rows(T0, &tmv, sv, &vbar); }
     if (a.early_kv) pdl_wait();
+    __syncthreads();                                            // the norm weights and the barriers are in place
 
-    // queries: per-head RMSNorm + RoPE, split into f16 hi + lo
-    for (int qi = warp; qi < nq16; qi += NW) {
-        float v0[PER], v1[PER];
-        if (qi < nq) {
-            const int tok = qi / gqa, hq = kvh * gqa + qi % gqa;
-            if (a.q_ready) {
-                const float *src = a.qkv + ((size_t)tok * a.H + hq) * HD;
-                #pragma unroll
-                for (int e = 0; e < PER; e++) { v0[e] = src[lane * PER + e]; v1[e] = src[lane * PER + e + HALF]; }
-            } else {
-                head_norm_rope<HD>(a.qkv + (size_t)tok * a.ld + (size_t)hq * HD, s_qn, a.rope + (size_t)tok * HALF, a.eps, lane, v0, v1);
-            }
-        } else {
-            #pragma unroll
-            for (int e = 0; e < PER; e++) v0[e] = v1[e] = 0.0f;
-        }
+    // the block's own K / V rows that fall into this span (norm + rope, f16 RNE): to the cache, and set aside for the tile.  Their
+    // loads go out with those of the warp's first query row.
+    auto store_q = [&](int qi, const float (&v0)[PER], const float (&v1)[PER]) {
         #pragma unroll
         for (int e = 0; e < PER; e++) {
             int i = lane * PER + e;
@@ -90,6 +77,66 @@ __global__ void __launch_bounds__(LG_ATTN_THREADS) lg_attn_deep_kernel(LgAttnArg
             qhi[(size_t)qi * LDH + i] = h0; qhi[(size_t)qi * LDH + i + HALF] = h1;
             qlo[(size_t)qi * LDH + i] = __float2half_rn(v0[e] - __half2float(h0));
             qlo[(size_t)qi * LDH + i + HALF] = __float2half_rn(v1[e] - __half2float(h1));
+        }
+    };
+    {
+        auto q_src = [&](int qi) {
+            const int tok = qi / gqa, hq = kvh * gqa + qi % gqa;
+            return a.q_ready ? a.qkv + ((size_t)tok * a.H + hq) * HD : a.qkv + (size_t)tok * a.ld + (size_t)hq * HD;
+        };
+        float qv0[2][PER], qv1[2][PER]; float2 qcs[2][PER];
+        float kv0[2][PER], kv1[2][PER]; float2 kcs[2][PER];
+        bool hask[2];
+        #pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int qi = warp + u * NW;
+            if (qi < nq) head_load<HD>(q_src(qi), a.q_ready ? nullptr : a.rope + (size_t)(qi / gqa) * HALF, lane, qv0[u], qv1[u], qcs[u]);
+        }
+        #pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int j = warp + u * NW, tok = j >> 1, isv = j & 1, TT = (pos0 + tok) / S;
+            hask[u] = writes_kv && j < 2 * a.M && TT >= T0 && TT <= T1;
+            if (hask[u])
+                head_load<HD>(a.qkv + (size_t)tok * a.ld + (size_t)(a.H + ((isv && a.has_v) ? a.Hkv : 0) + kvh) * HD,
+                              isv ? nullptr : a.rope + (size_t)tok * HALF, lane, kv0[u], kv1[u], kcs[u]);
+        }
+        #pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int qi = warp + u * NW;
+            if (qi < nq) {
+                if (!a.q_ready) head_finish<HD>(s_qn, true, a.eps, lane, qv0[u], qv1[u], qcs[u]);
+                store_q(qi, qv0[u], qv1[u]);
+            }
+        }
+        #pragma unroll
+        for (int u = 0; u < 2; u++) {
+            if (!hask[u]) continue;
+            const int j = warp + u * NW, tok = j >> 1, isv = j & 1, p = pos0 + tok;
+            head_finish<HD>(isv ? nullptr : s_kn, !isv, a.eps, lane, kv0[u], kv1[u], kcs[u]);
+            __half *dst = (isv ? a.vc : a.kc) + (size_t)(p % a.seq) * a.kv_dim + (size_t)kvh * HD;
+            #pragma unroll
+            for (int e = 0; e < PER; e++) {
+                const __half h0 = __float2half_rn(kv0[u][e]), h1 = __float2half_rn(kv1[u][e]);
+                dst[lane * PER + e] = h0; dst[lane * PER + e + HALF] = h1;
+                kvnew[(size_t)j * HD + lane * PER + e] = h0; kvnew[(size_t)j * HD + lane * PER + e + HALF] = h1;
+            }
+        }
+        for (int qi = warp + 2 * NW; qi < nq; qi += NW) {
+            float v0[PER], v1[PER];
+            if (a.q_ready) {
+                const float *src = q_src(qi);
+                #pragma unroll
+                for (int e = 0; e < PER; e++) { v0[e] = src[lane * PER + e]; v1[e] = src[lane * PER + e + HALF]; }
+            } else {
+                head_norm_rope<HD>(q_src(qi), s_qn, a.rope + (size_t)(qi / gqa) * HALF, a.eps, lane, v0, v1);
+            }
+            store_q(qi, v0, v1);
+        }
+        for (int qi = nq + warp; qi < nq16; qi += NW) {
+            float z[PER];
+            #pragma unroll
+            for (int e = 0; e < PER; e++) z[e] = 0.0f;
+            store_q(qi, z, z);
         }
     }
     for (int r = threadIdx.x; r < nq16; r += LG_ATTN_THREADS) { row_m[r] = -INFINITY; row_l[r] = 0.0f; row_a[r] = 1.0f; }
@@ -110,32 +157,24 @@ __global__ void __launch_bounds__(LG_ATTN_THREADS) lg_attn_deep_kernel(LgAttnArg
         #pragma unroll
         for (int n = 0; n < 4; n++) o[mt][n][0] = o[mt][n][1] = o[mt][n][2] = o[mt][n][3] = 0.0f;
 
-    for (int T = T0; T <= T1; T++) {
-        if (T > T0) {
-            __syncthreads();                                     // the previous tile's K, V and P are no longer read
-            if (T == T0 + 2) LG_STAMP(a.tag, 0);
-            load_tile(T);
-        }
-        if (writes_kv) {
-            // rows of the new positions that fall into this tile: K (norm + rope) and V (plain norm), f16 RNE
-            for (int j = warp; j < 2 * a.M; j += NW) {
-                const int tok = j >> 1, isv = j & 1, p = pos0 + tok;
-                if (p / S != T) continue;
-                float v0[PER], v1[PER];
-                const float *src = a.qkv + (size_t)tok * a.ld + (size_t)(a.H + ((isv && a.has_v) ? a.Hkv : 0) + kvh) * HD;
-                head_norm_rope<HD>(src, isv ? nullptr : s_kn, isv ? nullptr : a.rope + (size_t)tok * HALF, a.eps, lane, v0, v1);
-                __half *dst = (isv ? a.vc : a.kc) + (size_t)(p % a.seq) * a.kv_dim + (size_t)kvh * HD;
-                __half *dsm = (isv ? sv : sk) + (size_t)(p - T * S) * LDH;
-                #pragma unroll
-                for (int e = 0; e < PER; e++) {
-                    const __half h0 = __float2half_rn(v0[e]), h1 = __float2half_rn(v1[e]);
-                    dst[lane * PER + e] = h0; dst[lane * PER + e + HALF] = h1;
-                    dsm[lane * PER + e] = h0; dsm[lane * PER + e + HALF] = h1;
-                }
+    // a tile's rows of the block's own positions go over whatever the copy brought for them
+    auto patch = [&](int T, __half *tile, int isv) {
+        for (int tok = warp; tok < a.M; tok += NW) {
+            const int p = pos0 + tok;
+            if (p / S != T) continue;
+            #pragma unroll
+            for (int e = 0; e < PER; e++) {
+                *kv_at<S>(tile, p - T * S, lane * PER + e) = kvnew[(size_t)(2 * tok + isv) * HD + lane * PER + e];
+                *kv_at<S>(tile, p - T * S, lane * PER + e + HALF) = kvnew[(size_t)(2 * tok + isv) * HD + lane * PER + e + HALF];
             }
         }
-        cp_async_wait_all();
-        __syncthreads();
+    };
+    uint32_t parity = 0;
+    for (int T = T0; T <= T1; T++, parity ^= 1) {
+        __syncthreads();                                         // Q and the new rows are in place; the previous tile's V and P are no longer read
+        if (T > T0 && threadIdx.x == 0) { fence_async_shared(); load_rows(T, &tmv, sv, &vbar); }
+        if (!mbar_wait(&kbar, parity) && a.err && lane == 0) atomicOr(a.err, LG_ERR_MBAR_TIMEOUT);
+        if (writes_kv && pos0 + a.M > T * S && pos0 < (T + 1) * S) { patch(T, sk, 0); __syncthreads(); }
         if (T == T0 + 2) LG_STAMP(a.tag, 1);
 
         // scores S^T = K Q^T: warp w holds keys [16 (w & 3), +16) as the tile's rows and half (w >> 2) of the head dims,
@@ -147,11 +186,11 @@ __global__ void __launch_bounds__(LG_ATTN_THREADS) lg_attn_deep_kernel(LgAttnArg
                 #pragma unroll
                 for (int f = 0; f < 4; f++) c0[n][f] = c1[n][f] = 0.0f;
             const int kt = warp & 3, dh = warp >> 2;
-            const __half *ka_p = sk + (size_t)(kt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDH + dh * (HD / 2) + (lane >> 4) * 8;
+            const int krow = kt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, kcol = dh * (HD / 2) + (lane >> 4) * 8;
             #pragma unroll 2
             for (int k0 = 0; k0 < HD / 2; k0 += 16) {
                 uint32_t ka[4];                                  // A operand: 16 keys x 16 dims
-                ldsm_x4(ka, ka_p + k0);
+                ldsm_x4(ka, kv_at<S>(sk, krow, kcol + k0));
                 #pragma unroll
                 for (int n = 0; n < 4; n++) {
                     if (n >= nq8) break;
@@ -180,6 +219,7 @@ __global__ void __launch_bounds__(LG_ATTN_THREADS) lg_attn_deep_kernel(LgAttnArg
             }
         }
         __syncthreads();
+        if (T < T1 && threadIdx.x == 0) { fence_async_shared(); load_rows(T + 1, &tmk, sk, &kbar); }     // K is free: the next tile's under softmax and value product
         if (T == T0 + 2) LG_STAMP(a.tag, 2);
 
         // online softmax, one warp per query row: new running max, the tile's weights against it, the rescale
@@ -201,6 +241,8 @@ __global__ void __launch_bounds__(LG_ATTN_THREADS) lg_attn_deep_kernel(LgAttnArg
                 row_m[qi] = m_new;
             }
         }
+        if (!mbar_wait(&vbar, parity) && a.err && lane == 0) atomicOr(a.err, LG_ERR_MBAR_TIMEOUT);
+        if (writes_kv && pos0 + a.M > T * S && pos0 < (T + 1) * S) patch(T, sv, 1);
         __syncthreads();
         if (T == T0 + 2) LG_STAMP(a.tag, 3);
 
@@ -226,8 +268,8 @@ __global__ void __launch_bounds__(LG_ATTN_THREADS) lg_attn_deep_kernel(LgAttnArg
                 for (int mt = 0; mt < MTW; mt++) {
                     const int d0 = (warp * MTW + mt) * 16;
                     uint32_t va[4], vb[4];                      // A operands (transposed loads): 16 dims x keys k0..k0+15, k0+16..k0+31
-                    ldsm_x4_t(va, sv + (size_t)(k0 + (lane & 7) + (lane >> 4) * 8) * LDH + d0 + ((lane >> 3) & 1) * 8);
-                    ldsm_x4_t(vb, sv + (size_t)(k0 + 16 + (lane & 7) + (lane >> 4) * 8) * LDH + d0 + ((lane >> 3) & 1) * 8);
+                    ldsm_x4_t(va, kv_at<S>(sv, k0 + (lane & 7) + (lane >> 4) * 8, d0 + ((lane >> 3) & 1) * 8));
+                    ldsm_x4_t(vb, kv_at<S>(sv, k0 + 16 + (lane & 7) + (lane >> 4) * 8, d0 + ((lane >> 3) & 1) * 8));
                     #pragma unroll
                     for (int n = 0; n < 4; n++) {
                         if (n >= nq8) break;
@@ -259,84 +301,78 @@ __global__ void __launch_bounds__(LG_ATTN_THREADS) lg_attn_deep_kernel(LgAttnArg
             if (warp == 0 && g == 0) a.part_ml[((size_t)slot * a.M + tok) * a.H + hq] = make_float2(row_m[qi], row_l[qi]);
         }
     }
+}
 
-    // the last CTA of this KV head merges the spans
-    __shared__ int s_last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        s_last = atomicAdd(a.tickets + kvh, 1) == s_hi - s_lo;
+// Merge of the spans.  One CTA per (query row, 128 output dims): a warp owns every eighth span, a lane 4 dims.  Bound by one
+// round of loads: the partials (1 MB per KV head at 64 spans x 16 queries) are read by M H hd / 128 CTAs at once, where the last
+// CTA of the span kernel used to read them alone.  E4B-class, 8192 positions: attention of a verify step of width 1 / 4 / 8 356 / 742 /
+// 1295 us before, 291 / 457 / 724 with this merge and the tiled copies.  Which sums a span enters, and in which order, follows
+// from its absolute index alone; spans outside a query's window add exact zeros.
+#define LG_MERGE_DIMS 128
+#define LG_MERGE_UNROLL 8
+__global__ void __launch_bounds__(256) lg_attn_merge_kernel(LgAttnArgs a) {
+    __shared__ float s_red[8], s_sum[8];
+    __shared__ float4 s_acc[8][LG_MERGE_DIMS / 4];
+    pdl_launch();
+    const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;          // a warp per eighth of the spans
+    const int tok = blockIdx.y, hq = blockIdx.x, d4 = blockIdx.z * LG_MERGE_DIMS + lane * 4;
+    pdl_wait();
+    const int S = LG_DEEP_S, G = a.G, pos0 = *a.pos;
+    const int p_first = pos0 + a.qpos_off, p_last = pos0 + a.M - 1 + a.qpos_off, pj = p_first + tok;
+    if (p_last < 0) return;
+    const int s_lo = (a.window > 0 ? max(0, p_first + a.win_shrink - a.window + 1) : 0) / S / G, s_hi = p_last / S / G;
+    const int i0 = (a.window > 0 ? max(0, pj + a.win_shrink - a.window + 1) : 0) / S / G, i1 = pj >= 0 ? pj / S / G : -1;
+    const size_t row = (size_t)tok * a.H + hq, slot = (size_t)a.M * a.H;
+    // spans part, part + 8, ... (absolute indices) belong to this warp
+    const int first = s_lo + ((part - s_lo) & 7);
+    // largest score maximum over all spans of the query
+    float mx = -INFINITY;
+    for (int s = s_lo + threadIdx.x; s <= s_hi; s += 256) {
+        const float2 v = __ldcg(a.part_ml + (s % a.n_slots) * slot + row);
+        if (s >= i0 && s <= i1 && v.y > 0.0f) mx = fmaxf(mx, v.x);
     }
+    mx = warp_max(mx);
+    if (lane == 0) s_red[part] = mx;
     __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    const int ns_all = s_hi - s_lo + 1;
-    float2 *mls = (float2 *)sk;                               // [nq][ns_all]: (max, sum) then (weight, -); the K/V area is free now
-    float *invl = row_l;                                      // [nq]
-    for (int i = threadIdx.x; i < nq * ns_all; i += LG_ATTN_THREADS) {
-        const int qi = i / ns_all, S2 = s_lo + i % ns_all;
-        const int tok = qi / gqa, hq = kvh * gqa + qi % gqa;
-        mls[i] = __ldcg(a.part_ml + ((size_t)(S2 % a.n_slots) * a.M + tok) * a.H + hq);
+    #pragma unroll
+    for (int w = 0; w < 8; w++) mx = fmaxf(mx, s_red[w]);
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float lsum = 0.0f;
+    for (int s = first; s <= s_hi; s += 8 * LG_MERGE_UNROLL) {
+        float4 v[LG_MERGE_UNROLL]; float2 m[LG_MERGE_UNROLL];
+        #pragma unroll
+        for (int j = 0; j < LG_MERGE_UNROLL; j++)
+            if (s + 8 * j <= s_hi) {
+                const size_t at = ((s + 8 * j) % a.n_slots) * slot + row;
+                m[j] = __ldcg(a.part_ml + at);
+                v[j] = __ldcg((const float4 *)(a.part + at * a.hd + d4));
+            }
+        #pragma unroll
+        for (int j = 0; j < LG_MERGE_UNROLL; j++)
+            if (s + 8 * j <= s_hi) {
+                const int sp = s + 8 * j;
+                const float w = (sp >= i0 && sp <= i1 && m[j].y > 0.0f) ? expf(m[j].x - mx) : 0.0f;
+                lsum = fmaf(w, m[j].y, lsum);
+                acc.x = fmaf(w, v[j].x, acc.x); acc.y = fmaf(w, v[j].y, acc.y);
+                acc.z = fmaf(w, v[j].z, acc.z); acc.w = fmaf(w, v[j].w, acc.w);
+            }
     }
+    s_acc[part][lane] = acc;
+    if (lane == 0) s_sum[part] = lsum;
     __syncthreads();
-    for (int qi = warp; qi < nq; qi += NW) {
-        const int pj = pos0 + qi / gqa + a.qpos_off;
-        const int lo = a.window > 0 ? max(0, pj + a.win_shrink - a.window + 1) : 0;
-        const int i0 = pj >= 0 ? (lo / S) / G - s_lo : 0, i1 = pj >= 0 ? (pj / S) / G - s_lo : -1;
-        float mx = -INFINITY;
-        for (int i = i0 + lane; i <= i1; i += 32) { float2 v = mls[qi * ns_all + i]; if (v.y > 0.0f) mx = fmaxf(mx, v.x); }
-        mx = warp_max(mx);
-        // a span always lands in lane (absolute span index % 32): the order of this sum is the same wherever the block's
-        // first span lies (spans outside the query's window add exact zeros)
-        float lsum = 0.0f;
-        for (int S2 = (s_lo & ~31) + lane; S2 <= s_hi; S2 += 32) {
-            if (S2 < s_lo) continue;
-            const int i = S2 - s_lo;
-            float2 v = mls[qi * ns_all + i];
-            float w = (i >= i0 && i <= i1 && v.y > 0.0f) ? expf(v.x - mx) : 0.0f;
-            mls[qi * ns_all + i].x = w;
-            lsum += w * v.y;
-        }
-        lsum = warp_sum(lsum);
-        if (lane == 0) invl[qi] = lsum > 0.0f ? 1.0f / lsum : 0.0f;
-    }
-    __syncthreads();
-    float *ybuf = (float *)qhi;                                // [nq][HD] f32 (the query area is free now)
-    const size_t slot_stride = (size_t)a.M * a.H * HD;
-    for (int u = threadIdx.x; u < nq * (HD / 4); u += LG_ATTN_THREADS) {
-        const int qi = u / (HD / 4), d4 = (u % (HD / 4)) * 4;
-        const float *base = a.part + ((size_t)(qi / gqa) * a.H + kvh * gqa + qi % gqa) * HD + d4;
-        const float2 *wq = mls + (size_t)qi * ns_all;
-        float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        for (int i = 0; i < ns_all; i += 8) {                  // ascending span order, 8 loads in flight
-            float4 v[8];
-            #pragma unroll
-            for (int j = 0; j < 8; j++)
-                if (i + j < ns_all) v[j] = __ldcg((const float4 *)(base + (size_t)((s_lo + i + j) % a.n_slots) * slot_stride));
-            #pragma unroll
-            for (int j = 0; j < 8; j++)
-                if (i + j < ns_all) {
-                    const float w = wq[i + j].x;
-                    acc.x = fmaf(w, v[j].x, acc.x); acc.y = fmaf(w, v[j].y, acc.y);
-                    acc.z = fmaf(w, v[j].z, acc.z); acc.w = fmaf(w, v[j].w, acc.w);
-                }
-        }
-        const float il = invl[qi];
-        *(float4 *)(ybuf + (size_t)qi * HD + d4) = make_float4(acc.x * il, acc.y * il, acc.z * il, acc.w * il);
-    }
-    __syncthreads();
-    for (int u = warp; u < nq * (HD / 32); u += NW) {
-        const int qi = u / (HD / 32), d = (u % (HD / 32)) * 32 + lane;
-        const int tok = qi / gqa, hq = kvh * gqa + qi % gqa;
-        const float y = ybuf[(size_t)qi * HD + d];
-        if (a.out_f32) a.out_f32[((size_t)tok * a.H + hq) * HD + d] = y;
-        if (a.out_h) a.out_h[(size_t)tok * a.ld_h + hq * HD + d] = __float2half_rn(y);
-        if (a.out.q) quant_group_store(y, lane, tok, (hq * HD + d) >> 5, a.out);
-    }
-    if (threadIdx.x == 0) a.tickets[kvh] = 0;
+    if (part >= LG_MERGE_DIMS / 32) return;
+    // warp `part` finishes 32 dims: the eight partial sums in order
+    float y = 0.0f, l = 0.0f;
+    #pragma unroll
+    for (int w = 0; w < 8; w++) { y += ((const float *)s_acc[w])[part * 32 + lane]; l += s_sum[w]; }
+    y = l > 0.0f ? y * (1.0f / l) : 0.0f;
+    const int d = blockIdx.z * LG_MERGE_DIMS + part * 32 + lane;
+    if (a.out_f32) a.out_f32[row * a.hd + d] = y;
+    if (a.out_h) a.out_h[(size_t)tok * a.ld_h + hq * a.hd + d] = __float2half_rn(y);
+    if (a.out.q) quant_group_store(y, lane, tok, (hq * a.hd + d) >> 5, a.out);
 }
 
 inline size_t attn_deep_smem(int nq, int hd) {
     size_t nq16 = (size_t)((nq + 15) & ~15), ldh = hd + 8, S = LG_DEEP_S;
-    return 2 * nq16 * ldh * 2 + 2 * S * ldh * 2 + 2 * nq16 * S * 4 + 2 * nq16 * (S + 8) * 2 + nq16 * 12 + 64;
+    return 1024 + 2 * S * hd * 2 + 2 * nq16 * ldh * 2 + 2 * nq16 * S * 4 + 2 * nq16 * (S + 8) * 2 + nq16 * 12 + (size_t)2 * LG_MAXM * hd * 2;
 }

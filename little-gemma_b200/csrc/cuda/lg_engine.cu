@@ -242,10 +242,8 @@ void set_kernel_attributes() {
     LG_CHECK(cudaFuncSetAttribute(lg_attn_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATTN_SMEM_MAX));
     attn_cluster_attr<64>(); attn_cluster_attr<128>(); attn_cluster_attr<256>(); attn_cluster_attr<512>();
     pf_attr<LG_FMT_Q4_0, LG_PF_STORE>(); pf_attr<LG_FMT_Q4_0, LG_PF_GEGLU>(); pf_attr<LG_FMT_Q4_K, LG_PF_STORE>(); pf_attr<LG_FMT_Q4_K, LG_PF_GEGLU>();
-    LG_CHECK(cudaFuncSetAttribute(lg_attn_deep_kernel<128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATTN_SMEM_MAX));
-    LG_CHECK(cudaFuncSetAttribute(lg_attn_deep_kernel<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATTN_SMEM_MAX));
-    LG_CHECK(cudaFuncSetAttribute(lg_attn_deep_kernel<256, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATTN_SMEM_MAX));
-    LG_CHECK(cudaFuncSetAttribute(lg_attn_deep_kernel<256, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATTN_SMEM_MAX));
+    LG_CHECK(cudaFuncSetAttribute(lg_attn_deep_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATTN_SMEM_MAX));
+    LG_CHECK(cudaFuncSetAttribute(lg_attn_deep_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATTN_SMEM_MAX));
     LG_CHECK(cudaFuncSetAttribute(lg_pf_attn_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pf_attn_smem<64>()));
     LG_CHECK(cudaFuncSetAttribute(lg_pf_attn_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pf_attn_smem<128>()));
     LG_CHECK(cudaFuncSetAttribute(lg_pf_attn_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pf_attn_smem<256>()));
@@ -579,16 +577,18 @@ int deep_span_tiles(const Engine *e, int max_seq, int n_kv_heads, int hd, int nq
 }
 
 void launch_attn_deep(Engine *e, LgAttnArgs a, int max_seq, int G) {
-    const int nq = (a.H / a.Hkv) * a.M, nmt = ((nq + 15) & ~15) / 16;
+    const int nq = (a.H / a.Hkv) * a.M;
     const size_t sm = attn_deep_smem(nq, a.hd);
     const int n_spans = ((max_seq + LG_DEEP_S - 1) / LG_DEEP_S + G - 1) / G + 1;
-    if (n_spans > a.n_slots || (size_t)nq * n_spans * 8 > 2 * (size_t)LG_DEEP_S * (a.hd + 8) * 2 || sm > ATTN_SMEM_MAX || a.Hkv > MAX_KV_HEADS) {
+    if (n_spans > a.n_slots || sm > ATTN_SMEM_MAX || a.Hkv > MAX_KV_HEADS) {
         fprintf(stderr, "lg_b200: %d key spans x %d queries do not fit the span attention kernel\n", n_spans, nq); exit(1);
     }
-    a.tickets = e->tickets; a.G = G; a.tag = (int)e->launches;
+    a.G = G; a.tag = (int)e->launches;
+    const CUtensorMap tmk = kv_tensor_map(a.kc, a.kv_dim, a.seq, LG_DEEP_S), tmv = kv_tensor_map(a.vc, a.kv_dim, a.seq, LG_DEEP_S);
     dim3 grid(a.Hkv, n_spans), block(LG_ATTN_THREADS);
-    if (a.hd == 256) { if (nmt <= 1) launch_k(e, lg_attn_deep_kernel<256, 1>, grid, block, sm, a); else launch_k(e, lg_attn_deep_kernel<256, 2>, grid, block, sm, a); }
-    else             { if (nmt <= 1) launch_k(e, lg_attn_deep_kernel<128, 1>, grid, block, sm, a); else launch_k(e, lg_attn_deep_kernel<128, 2>, grid, block, sm, a); }
+    if (a.hd == 256) launch_k(e, lg_attn_deep_kernel<256>, grid, block, sm, tmk, tmv, a);
+    else launch_k(e, lg_attn_deep_kernel<128>, grid, block, sm, tmk, tmv, a);
+    launch_k(e, lg_attn_merge_kernel, dim3(a.H, a.M, a.hd / LG_MERGE_DIMS), dim3(256), 0, a);
 }
 
 int tiles_for(int window, int max_seq, int M, int hd);

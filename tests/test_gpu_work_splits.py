@@ -1,8 +1,9 @@
-"""GPU tests of how matmuls and attention are cut into work: two teams of a CTA behind one panel."""
+"""GPU tests of how matmuls and attention are cut into work: two teams of a CTA behind one panel, spans merged by a launch of their
+own."""
 import numpy as np
 import pytest
 
-from tests.conftest import synth_module
+from tests.conftest import model_files, synth_module
 from tests.test_gpu_prefill import _weights
 
 pytestmark = pytest.mark.gpu
@@ -21,3 +22,22 @@ def test_two_teams_of_a_cta(lg, port_built, wtype, m, k, M):
     # activations: 16-bit integers of their 32-group (2^-16 of its largest); f32 sums
     assert np.abs(got - want).max() / np.abs(want).max() < 2e-4
     assert np.array_equal(got[:4], lg.gemv(t, raw, m, k, x[:4]))
+
+
+@pytest.mark.parametrize("depth", [100, 128 * 8 - 2, 128 * 8 + 5, 128 * 65 + 1])
+def test_span_merge(lg, depth):
+    """Spans of two tiles of 64 keys: a single one, eight (one per warp of the merge), nine, and more than eight per warp.  The two
+    decompositions add the same f32 terms in another order: 1e-4 of the logits' range is some 50 times what that makes."""
+    s = synth_module()
+    tp, _ = model_files("mid")
+    out = []
+    for spans in (False, True):
+        lg.set_attn_deep(64 if spans else 1 << 30, 2 if spans else 0)
+        try:
+            with lg.Session(tp, None, 8704) as g:
+                toks = s.prompt_ids(depth + 4, g.n_vocab, seed=61)
+                g.prefill(toks[:depth], 0)
+                out.append(np.stack([g.forward(int(toks[depth + i]), depth + i) for i in range(4)]))
+        finally:
+            lg.set_attn_deep(4096, 0)
+    assert np.abs(out[0] - out[1]).max() / (out[0].max() - out[0].min()) < 1e-4
