@@ -32,11 +32,13 @@ lg_attn_deep_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
     if (!a.q_ready)
         for (int i = threadIdx.x; i < HD; i += LG_ATTN_THREADS) { s_qn[i] = a.q_norm[i]; s_kn[i] = a.k_norm ? a.k_norm[i] : 1.0f; }
     if (!a.early_kv) pdl_wait();
+    const int called_off = !a.early_kv && a.skip ? __ldcg(a.skip) : 0;      // read beside the position
     constexpr int S = LG_DEEP_S, LDH = HD + 8, LDP = S + 8, PER = HD / 64, HALF = HD / 2, NW = LG_ATTN_THREADS / 32;
     const int G = a.G;
     const int kvh = blockIdx.x, gqa = a.H / a.Hkv, nq = gqa * a.M, nq16 = (nq + 15) & ~15;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int pos0 = *a.pos;
+    const int pos0 = __ldcg(a.pos);
+    if (called_off) return;
     const int p_first = pos0 + a.qpos_off, p_last = pos0 + a.M - 1 + a.qpos_off;
     if (p_last < 0) return;
     const int lo_first = a.window > 0 ? max(0, p_first + a.win_shrink - a.window + 1) : 0;
@@ -317,7 +319,9 @@ __global__ void __launch_bounds__(256) lg_attn_merge_kernel(LgAttnArgs a) {
     const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;          // a warp per eighth of the spans
     const int tok = blockIdx.y, hq = blockIdx.x, d4 = blockIdx.z * LG_MERGE_DIMS + lane * 4;
     pdl_wait();
-    const int S = LG_DEEP_S, G = a.G, pos0 = *a.pos;
+    const int called_off = a.skip ? __ldcg(a.skip) : 0;
+    const int S = LG_DEEP_S, G = a.G, pos0 = __ldcg(a.pos);
+    if (called_off) return;
     const int p_first = pos0 + a.qpos_off, p_last = pos0 + a.M - 1 + a.qpos_off, pj = p_first + tok;
     if (p_last < 0) return;
     const int s_lo = (a.window > 0 ? max(0, p_first + a.win_shrink - a.window + 1) : 0) / S / G, s_hi = p_last / S / G;

@@ -512,21 +512,24 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
                     if (!panel_sent && ++issued == early) {
                         // a ring of weights is in flight; now the activations, which the previous kernel produced
                         pdl_wait();
-                        if (a.skip && *a.skip) {
-                            // called off: let the copies already in flight land (shared memory must not be released under
-                            // them), then leave; the consumers have left on the same word
+                        const int called_off = a.skip ? __ldcg(a.skip) : 0;      // arrives while the panel is on its way
+                        panel_sent = true;
+                        if (team == 0) {                         // one panel for all
+                            uint32_t qb = (uint32_t)nsb_s * 256, sb = (uint32_t)nsb_s * 32;
+                            mbar_expect_tx(pbar, NP * (qb + sb));
+                            #pragma unroll
+                            for (int p = 0; p < NP; p++) {
+                                bulk_g2s(sq + (size_t)p * qb, a.x.q + ((size_t)p * a.x.nsb + kp0 * 2) * 256, qb, pbar);
+                                bulk_g2s(ss + (size_t)p * nsb_s * 4, a.x.s + ((size_t)p * a.x.nsb + kp0 * 2) * 4, sb, pbar);
+                            }
+                        }
+                        if (called_off) {
+                            // let the copies already in flight land (shared memory must not be released under them), then
+                            // leave; the consumers leave on the same word
                             for (int i = 0; i < issued; i++) mbar_wait(full + (i % NS), 0);
+                            mbar_wait(pbar, 0);
                             ok = false;
                             break;
-                        }
-                        panel_sent = true;
-                        if (team != 0) continue;                 // one panel for all
-                        uint32_t qb = (uint32_t)nsb_s * 256, sb = (uint32_t)nsb_s * 32;
-                        mbar_expect_tx(pbar, NP * (qb + sb));
-                        #pragma unroll
-                        for (int p = 0; p < NP; p++) {
-                            bulk_g2s(sq + (size_t)p * qb, a.x.q + ((size_t)p * a.x.nsb + kp0 * 2) * 256, qb, pbar);
-                            bulk_g2s(ss + (size_t)p * nsb_s * 4, a.x.s + ((size_t)p * a.x.nsb + kp0 * 2) * 4, sb, pbar);
                         }
                     }
                 }
@@ -544,8 +547,9 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
 
     pdl_wait();
     LG_STAMP(a.tag, 1);
-    if (a.skip && *a.skip) return;
+    const int called_off = a.skip ? __ldcg(a.skip) : 0;
     bool ok = mbar_wait(pbar, 0);
+    if (called_off) return;
     if (!ok && tid == 0) atomicOr(a.err, LG_ERR_MBAR_TIMEOUT);
     LG_STAMP(a.tag, 2);
     int stage = 0; uint32_t phase = 0;
@@ -1010,7 +1014,8 @@ __global__ void __launch_bounds__(LG_NORM_CL_THREADS) lg_norm_cluster_kernel(LgN
     LG_STAMP_KIND(a.tag, 7);
     pdl_wait();
     LG_STAMP(a.tag, 1);
-    if (a.skip && *a.skip) return;                       // the whole cluster leaves on the same word: nobody waits at a cluster barrier
+    // read beside the rows, looked at before the first cluster barrier: the whole cluster leaves on the same word
+    const int called_off = a.skip ? __ldcg(a.skip) : 0;
     float *x = a.x + (size_t)tok * a.ldx;
     float ss2 = 0.0f;
     if (a.add_src && cnt <= LG_NORM_CL_EPT * LG_NORM_CL_THREADS && a.n_parts <= 4) {
@@ -1025,6 +1030,7 @@ __global__ void __launch_bounds__(LG_NORM_CL_THREADS) lg_norm_cluster_kernel(LgN
                 pv[u][p] = (j < cnt && p < a.n_parts) ? __ldcg(a.add_src + (size_t)p * a.part_stride + (size_t)tok * a.ld_add + i0 + j) : 0.0f;
             xv[u] = j < cnt ? __ldcg(x + i0 + j) : 0.0f;
         }
+        if (called_off) return;
         float ss = 0.0f, sv[LG_NORM_CL_EPT];
         #pragma unroll
         for (int u = 0; u < LG_NORM_CL_EPT; u++) {
@@ -1053,6 +1059,7 @@ __global__ void __launch_bounds__(LG_NORM_CL_THREADS) lg_norm_cluster_kernel(LgN
             }
         }
     } else if (a.add_src) {
+        if (called_off) return;
         float ss = 0.0f;
         for (int j = threadIdx.x; j < cnt; j += LG_NORM_CL_THREADS) {
             const int i = i0 + j;
@@ -1078,6 +1085,7 @@ __global__ void __launch_bounds__(LG_NORM_CL_THREADS) lg_norm_cluster_kernel(LgN
         }
     } else {
         for (int j = threadIdx.x; j < cnt; j += LG_NORM_CL_THREADS) { float v = x[i0 + j]; row[j] = v; ss2 += v * v; }
+        if (called_off) return;
     }
     if (!a.norm_w && !a.want_panel && !a.y) return;
     float s = 1.0f;
@@ -1131,8 +1139,8 @@ __global__ void __launch_bounds__(LG_ELT_WARPS * 32) lg_elt_kernel(LgEltArgs a) 
     LG_STAMP_KIND(a.tag, 7);
     pdl_wait();
     LG_STAMP(a.tag, 1);
-    if (a.skip && *a.skip) return;
     if (gq * 32 >= a.n) return;
+    const int called_off = a.skip ? __ldcg(a.skip) : 0;      // read beside the rows
     float4 pv[LG_SS_PER_LANE];
     #pragma unroll
     for (int j = 0; j < LG_SS_PER_LANE; j++) {
@@ -1141,6 +1149,7 @@ __global__ void __launch_bounds__(LG_ELT_WARPS * 32) lg_elt_kernel(LgEltArgs a) 
     }
     const float xv = live ? __ldcg(a.x + (size_t)tok * a.ldx + i) : 0.0f;
     const float ov = live ? __ldcg(a.o + (size_t)tok * a.ldo + i) : 0.0f;
+    if (called_off) return;
     float4 tot = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     #pragma unroll
     for (int j = 0; j < LG_SS_PER_LANE; j++) { tot.x += pv[j].x; tot.y += pv[j].y; tot.z += pv[j].z; tot.w += pv[j].w; }
@@ -1306,11 +1315,13 @@ __global__ void __launch_bounds__(LG_ATTN_THREADS) lg_attn_kernel(LgAttnArgs a) 
         for (int i = threadIdx.x; i < HD; i += LG_ATTN_THREADS) { s_qn[i] = a.q_norm[i]; s_kn[i] = a.k_norm ? a.k_norm[i] : 1.0f; }
     // early_kv: the position and the cached rows below the block were written by earlier graph launches (this layer
     // writes its own rows, and only here), so the tile may start streaming before the previous kernel has finished
-    if (!a.early_kv) { pdl_wait(); if (a.skip && *a.skip) return; }
+    if (!a.early_kv) pdl_wait();
+    const int called_off = !a.early_kv && a.skip ? __ldcg(a.skip) : 0;      // read beside the position
     constexpr int S = lg_attn_tile(HD), LDH = HD + 8, LDP = S + 8, PER = HD / 64, HALF = HD / 2, NW = LG_ATTN_THREADS / 32;
     const int kvh = blockIdx.x, gqa = a.H / a.Hkv, nq = gqa * a.M, nq16 = (nq + 15) & ~15;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int pos0 = *a.pos;
+    const int pos0 = __ldcg(a.pos);
+    if (called_off) return;
     const int p_first = pos0 + a.qpos_off, p_last = pos0 + a.M - 1 + a.qpos_off;
     if (p_last < 0) return;
     const int lo_first = a.window > 0 ? max(0, p_first + a.win_shrink - a.window + 1) : 0;
