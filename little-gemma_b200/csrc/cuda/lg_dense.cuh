@@ -253,11 +253,15 @@ __global__ void __launch_bounds__(DN_GEMV_THREADS, 2) lg_dn_gemv_kernel(LgDnGemv
 // ---------------------------------------------------------------------------------------------
 // wide matmul on tcgen05: out[tok][row] = W x[tok], bf16 operands, f32 accumulation in tensor memory
 // ---------------------------------------------------------------------------------------------
-// One CTA owns 128 tokens (the TMEM lanes) x NT weight rows (TMEM columns) and walks k in blocks of 64:
-//   warp 4 (one thread)  loads the activation and the weight tile of a block with tiled TMA copies (128-byte swizzle); the
-//                        weight tiles of the first stages are requested before the dependency wait;
+// A tile is 128 tokens (the TMEM lanes) x NT weight rows (TMEM columns); a CTA walks tiles blockIdx.x, + gridDim.x, ..., the
+// token tiles of one weight tile first, and k in blocks of 64:
+//   warp 4 (one thread)  loads the activation and the weight tile of a block with tiled TMA copies (128-byte swizzle), on from
+//                        tile to tile; the weight tiles of the first stages are requested before the dependency wait;
 //   warp 5 (one thread)  issues four tcgen05.mma (M = 128, N = NT, K = 16) per block and commits the stage back;
-//   warps 0-3            read the accumulator (lane = token) and store 32 columns at a time with 16-byte stores.
+//   warps 0-3            read the accumulator (lane = token) and store 32 columns at a time with 16-byte stores, while the
+//                        next tile is multiplied into the other of two accumulators.
+// Bound by the tensor pipe.  The order matters as much as the overlap: the CTAs at work at one time share few weight tiles, so
+// a matrix larger than L2 crosses HBM once; weight tiles first, every token tile would read it again.
 enum { DN_G_F32 = 0, DN_G_BF16 = 1, DN_G_GLU = 2, DN_G_RELU2 = 3 };
 #define DN_GEMM_BM 128
 #define DN_GEMM_BK 64
@@ -268,6 +272,7 @@ template <int NT> __host__ __device__ constexpr size_t dn_gemm_smem() {
 }
 struct LgDnGemmArgs {
     int nkb, n_tok, cols;            // blocks of k; valid tokens; stored columns (a multiple of 32)
+    int n_ty, tiles;                 // token tiles; tiles in all
     int w_early;                     // the second operand does not depend on earlier kernels
     void *out; int ldo;              // f32 / bf16 rows; GLU: bf16 rows of cols / 2
     int *err;
@@ -282,17 +287,20 @@ __global__ void __launch_bounds__(DN_GEMM_THREADS) lg_dn_gemm_kernel(const __gri
     constexpr int ST = dn_gemm_stages<NT>(), A_BYTES = DN_GEMM_BM * 128, B_BYTES = NT * 128;
     unsigned char *base = (unsigned char *)(((uintptr_t)dn_smem + 1023) & ~(uintptr_t)1023);
     unsigned char *sA = base, *sB = base + ST * A_BYTES;
-    uint64_t *full = (uint64_t *)(sB + ST * B_BYTES), *empty = full + ST, *acc_full = empty + ST;
-    uint32_t *tmem_slot = (uint32_t *)(acc_full + 1);
+    uint64_t *full = (uint64_t *)(sB + ST * B_BYTES), *empty = full + ST, *acc_full = empty + ST, *acc_empty = acc_full + 2;
+    uint32_t *tmem_slot = (uint32_t *)(acc_empty + 2);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row0 = blockIdx.x * NT, tok0 = blockIdx.y * DN_GEMM_BM, nkb = a.nkb;
+    const int nkb = a.nkb, my_tiles = (a.tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
+    // tile i of this CTA
+    auto row_of = [&](int i) { return (int)(blockIdx.x + i * gridDim.x) / a.n_ty * NT; };
+    auto tok_of = [&](int i) { return (int)(blockIdx.x + i * gridDim.x) % a.n_ty * DN_GEMM_BM; };
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < ST; i++) { mbar_init(full + i, 1); mbar_init(empty + i, 1); }
-        mbar_init(acc_full, 1);
+        for (int i = 0; i < 2; i++) { mbar_init(acc_full + i, 1); mbar_init(acc_empty + i, 4); }
     }
     if (warp == 5) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(tmem_slot)), "r"(NT) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(tmem_slot)), "r"(2 * NT) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -303,57 +311,64 @@ __global__ void __launch_bounds__(DN_GEMM_THREADS) lg_dn_gemm_kernel(const __gri
 
     if (warp == 4) {
         if (lane == 0) {
-            const int pre = min(ST, nkb);
+            const int total = my_tiles * nkb, pre = min(ST, nkb);
             if (!a.w_early) pdl_wait();
             for (int kb = 0; kb < pre; kb++) {
                 mbar_expect_tx(full + kb, A_BYTES + B_BYTES);
-                tma_load_2d(sB + kb * B_BYTES, &tmw, kb * DN_GEMM_BK, row0, full + kb);
+                tma_load_2d(sB + kb * B_BYTES, &tmw, kb * DN_GEMM_BK, row_of(0), full + kb);
             }
             if (a.w_early) pdl_wait();
-            for (int kb = 0; kb < pre; kb++) tma_load_2d(sA + kb * A_BYTES, &tmx, kb * DN_GEMM_BK, tok0, full + kb);
-            bool ok = true;
-            int issued = pre;
-            for (int kb = pre; kb < nkb && ok; kb++) {
-                const int s = kb % ST;
-                if (!mbar_wait(empty + s, ((kb / ST) & 1) ^ 1)) { atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 4); ok = false; break; }
+            for (int kb = 0; kb < pre; kb++) tma_load_2d(sA + kb * A_BYTES, &tmx, kb * DN_GEMM_BK, tok_of(0), full + kb);
+            int it = pre, tile = pre / nkb, kb = pre % nkb;          // blocks issued; where the next one lies
+            for (; it < total; it++) {
+                const int s = it % ST;
+                if (!mbar_wait(empty + s, ((it / ST) & 1) ^ 1)) { atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 4); break; }
                 mbar_expect_tx(full + s, A_BYTES + B_BYTES);
-                tma_load_2d(sB + s * B_BYTES, &tmw, kb * DN_GEMM_BK, row0, full + s);
-                tma_load_2d(sA + s * A_BYTES, &tmx, kb * DN_GEMM_BK, tok0, full + s);
-                issued = kb + 1;
+                tma_load_2d(sB + s * B_BYTES, &tmw, kb * DN_GEMM_BK, row_of(tile), full + s);
+                tma_load_2d(sA + s * A_BYTES, &tmx, kb * DN_GEMM_BK, tok_of(tile), full + s);
+                if (++kb == nkb) { kb = 0; tile++; }
             }
-            if (!ok)      // drain: the copies already issued must land before the CTA's shared memory is released
-                for (int kb = max(0, issued - ST); kb < issued; kb++) mbar_wait(full + kb % ST, (kb / ST) & 1);
+            if (it < total)      // drain: the copies already issued must land before the CTA's shared memory is released
+                for (int i = max(0, it - ST); i < it; i++) mbar_wait(full + i % ST, (i / ST) & 1);
         }
     } else if (warp == 5) {
         if (lane == 0) {
             // f32 accumulator, bf16 x bf16, both operands K-major
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(DN_GEMM_BM >> 4) << 24);
             bool ok = true;
-            uint32_t acc = 0;
-            for (int kb = 0; kb < nkb && ok; kb++) {
-                const int s = kb % ST;
-                if (!mbar_wait(full + s, (kb / ST) & 1)) { atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 8); ok = false; break; }
+            int it = 0;
+            for (int i = 0; i < my_tiles && ok; i++) {
+                const uint32_t d = tmem + (uint32_t)(i & 1) * NT;
+                if (!mbar_wait(acc_empty + (i & 1), ((i >> 1) & 1) ^ 1)) { atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 8); break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t ad = umma_desc_k128(smem_u32(sA + s * A_BYTES)), bd = umma_desc_k128(smem_u32(sB + s * B_BYTES));
-                #pragma unroll
-                for (int j = 0; j < DN_GEMM_BK / 16; j++) { umma_f16(tmem, ad + 2 * j, bd + 2 * j, idesc, acc); acc = 1u; }
-                umma_commit(empty + s);
+                uint32_t acc = 0;
+                for (int kb = 0; kb < nkb; kb++, it++) {
+                    const int s = it % ST;
+                    if (!mbar_wait(full + s, (it / ST) & 1)) { atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 8); ok = false; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t ad = umma_desc_k128(smem_u32(sA + s * A_BYTES)), bd = umma_desc_k128(smem_u32(sB + s * B_BYTES));
+                    #pragma unroll
+                    for (int j = 0; j < DN_GEMM_BK / 16; j++) { umma_f16(d, ad + 2 * j, bd + 2 * j, idesc, acc); acc = 1u; }
+                    umma_commit(empty + s);
+                }
+                umma_commit(acc_full + (i & 1));
             }
-            umma_commit(acc_full);
         }
     } else {
         pdl_wait();                                // the outputs' earlier readers have finished
-        const bool ok = mbar_wait(acc_full, 0);
-        if (!ok && lane == 0) atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 128);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int tok = tok0 + warp * 32 + lane;
-        if (ok)
+        bool ok = true;
+        for (int i = 0; i < my_tiles && ok; i++) {
+            ok = mbar_wait(acc_full + (i & 1), (i >> 1) & 1);
+            if (!ok) { if (lane == 0) atomicOr(a.err, LG_ERR_MBAR_TIMEOUT | 128); break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int tok = tok_of(i) + warp * 32 + lane, row0 = row_of(i);
+            const uint32_t d = tmem + (uint32_t)(i & 1) * NT + ((uint32_t)(warp * 32) << 16);
             for (int c0 = 0; c0 < NT; c0 += 32) {
                 const int col = row0 + c0;
                 if (col >= a.cols) break;           // uniform per CTA
                 uint32_t v[32];
                 __syncwarp();
-                tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + c0, v);
+                tmem_ld32(d + c0, v);
                 if (tok >= a.n_tok) continue;
                 if (EPI == DN_G_F32) {
                     float4 *o = (float4 *)((float *)a.out + (size_t)tok * a.ldo + col);
@@ -394,12 +409,16 @@ __global__ void __launch_bounds__(DN_GEMM_THREADS) lg_dn_gemm_kernel(const __gri
                     }
                 }
             }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            // this accumulator may be written again
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty + (i & 1));
+        }
     }
     __syncthreads();
     if (warp == 5) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(NT) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(2 * NT) : "memory");
     }
 }
 

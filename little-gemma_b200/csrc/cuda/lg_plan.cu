@@ -465,11 +465,15 @@ const CUtensorMap &buf_map(PlanModel *pm, const void *x, int k, int ld, int rows
 template <int EPI>
 void launch_gemm_maps(Engine *e, const CUtensorMap &x, int n, const CUtensorMap &w128, const CUtensorMap &w256, int w_rows, int nkb, void *out, int ldo, bool w_early, LgDnGemmArgs a = LgDnGemmArgs{}) {
     a.nkb = nkb; a.n_tok = n; a.cols = w_rows; a.out = out; a.ldo = ldo; a.err = e->err; a.w_early = w_early;
-    const int ty = (n + DN_GEMM_BM - 1) / DN_GEMM_BM;
-    if ((w_rows + 255) / 256 * ty >= e->sm_count)
-        launch_k(e, lg_dn_gemm_kernel<256, EPI>, dim3((w_rows + 255) / 256, ty), dim3(DN_GEMM_THREADS), dn_gemm_smem<256>(), x, w256, a);
-    else
-        launch_k(e, lg_dn_gemm_kernel<128, EPI>, dim3((w_rows + 127) / 128, ty), dim3(DN_GEMM_THREADS), dn_gemm_smem<128>(), x, w128, a);
+    a.n_ty = (n + DN_GEMM_BM - 1) / DN_GEMM_BM;
+    const int t256 = (w_rows + 255) / 256 * a.n_ty, t128 = (w_rows + 127) / 128 * a.n_ty;
+    if (t256 >= e->sm_count) {
+        a.tiles = t256;                            // one CTA per SM
+        launch_k(e, lg_dn_gemm_kernel<256, EPI>, dim3(e->sm_count), dim3(DN_GEMM_THREADS), dn_gemm_smem<256>(), x, w256, a);
+    } else {
+        a.tiles = t128;                            // two
+        launch_k(e, lg_dn_gemm_kernel<128, EPI>, dim3(std::min(t128, 2 * e->sm_count)), dim3(DN_GEMM_THREADS), dn_gemm_smem<128>(), x, w128, a);
+    }
 }
 // x: [x_rows][ldx] bf16, of which n rows count
 template <int EPI>

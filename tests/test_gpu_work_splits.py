@@ -1,5 +1,5 @@
 """GPU tests of how matmuls and attention are cut into work: two teams of a CTA behind one panel, spans merged by a launch of their
-own."""
+own, several tiles per CTA of the dense prompt matmul."""
 import numpy as np
 import pytest
 
@@ -41,3 +41,14 @@ def test_span_merge(lg, depth):
         finally:
             lg.set_attn_deep(4096, 0)
     assert np.abs(out[0] - out[1]).max() / (out[0].max() - out[0].min()) < 1e-4
+
+
+@pytest.mark.parametrize("m,k,n", [(2400, 150, 2000), (4128, 320, 2048), (2080, 64, 2300), (1312, 640, 4100)])
+def test_dense_prompt_matmul_of_several_tiles_per_cta(lg, m, k, n):
+    """More tiles than CTAs, ragged in tokens and rows, fewer and more blocks of k than ring stages."""
+    rng = np.random.default_rng(m + k)
+    bf = lambda a: (np.ascontiguousarray(a, np.float32).view(np.uint32) & 0xffff0000).view(np.float32)
+    w, x = bf(rng.standard_normal((m, k)) * k ** -0.5), bf(rng.standard_normal((n, k)))
+    want = x.astype(np.float64) @ w.T.astype(np.float64)
+    # exact products, f32 sums of up to 640 terms
+    assert np.abs(lg.dense_matmul(w, x) - want).max() / np.abs(want).max() < 2e-5
