@@ -442,9 +442,11 @@ __device__ __forceinline__ void gemv_body(const LgStageMaps *maps, const LgGemvA
     const int n_groups = (a.n_row_tiles + R - 1) / R;
     const bool cl = a.cl_ks != 0;                            // cluster (1, kslices, 1): cluster rank == blockIdx.y
 
+    // laid out for the longest slice: the ranks of a cluster address each other's sums and barrier by their own offsets
+    const int nsb_l = (a.nkp + a.kslices - 1) / a.kslices * 2;
     int8_t *sq = (int8_t *)smem;
-    float2 *ss = (float2 *)(smem + (size_t)NP * nsb_s * 256);
-    unsigned char *ring = (unsigned char *)(ss + (size_t)NP * nsb_s * 4);
+    float2 *ss = (float2 *)(smem + (size_t)NP * nsb_l * 256);
+    unsigned char *ring = (unsigned char *)(ss + (size_t)NP * nsb_l * 4);
     ring = (unsigned char *)(((uintptr_t)ring + 127) & ~(uintptr_t)127);
     const int cred_n = cl ? (a.kslices - 1) * RN : 0;
     ring += (size_t)team * ((size_t)NS * STAGE + (size_t)((LG_GEMV_CW + 1) * RN + cred_n) * 4);

@@ -1,5 +1,5 @@
 """GPU tests of how matmuls and attention are cut into work: two teams of a CTA behind one panel, spans merged by a launch of their
-own, several tiles per CTA of the dense prompt matmul."""
+own, several tiles per CTA of the dense prompt matmul, k slices of a cluster."""
 import numpy as np
 import pytest
 
@@ -52,3 +52,24 @@ def test_dense_prompt_matmul_of_several_tiles_per_cta(lg, m, k, n):
     want = x.astype(np.float64) @ w.T.astype(np.float64)
     # exact products, f32 sums of up to 640 terms
     assert np.abs(lg.dense_matmul(w, x) - want).max() / np.abs(want).max() < 2e-5
+
+
+@pytest.mark.parametrize("m,k", [(1024, 4800), (1152, 11840)])
+@pytest.mark.parametrize("M", [1, 6])
+def test_cluster_slices_of_unequal_length(lg, port_built, m, k, M):
+    """75 and 185 positions in four k slices: the ranks of a cluster hold panels of different lengths, yet send their sums to the
+    same places of rank 0's shared memory."""
+    from tests.test_gpu_kernels import _oracle, _resid_ref
+    s = synth_module()
+    rng = np.random.default_rng(m + k + M)
+    o = _oracle()
+    raw = s.quantize_q4_0(rng.standard_normal(m * k).astype(np.float32) * 0.02)
+    w = o.dequant(s.Q4_0, raw, m * k).reshape(m, k)
+    o.close()
+    act, x = rng.standard_normal((M, k)).astype(np.float32), rng.standard_normal((M, m)).astype(np.float32)
+    add_w, norm_w = ((1.0 + 0.3 * rng.standard_normal(m)).astype(np.float32) for _ in range(2))
+    xn, y, cluster = lg.matmul_resid(s.Q4_0, raw, m, k, act, x, add_w, 1.0, norm_w, 1e-6)
+    want_x, want_y = _resid_ref(w, act, x, add_w, 1.0, norm_w, 1e-6)
+    assert cluster
+    # 16-bit integers of the 32-group (2^-16 of its largest), f32 sums
+    assert np.abs(xn - want_x).max() / np.abs(want_x).max() < 2e-4 and np.abs(y - want_y).max() / np.abs(want_y).max() < 2e-4
