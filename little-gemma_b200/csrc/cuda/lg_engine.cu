@@ -708,8 +708,8 @@ bool g_compute_f32 = false;                   // lg_set_compute_f32: the next mo
 
 void session_state(Engine *e) {
     e->st = dalloc<LgRoundState>(1);
-    LG_CHECK(cudaMallocHost(&e->st_host, sizeof(LgRoundState)));
-    memset(e->st_host, 0, sizeof(LgRoundState));
+    LG_CHECK(cudaMallocHost(&e->st_host, sizeof(LgRoundState) + sizeof(int)));
+    memset(e->st_host, 0, sizeof(LgRoundState) + sizeof(int));
     e->log = dalloc<int>(LOG_CAP);
 }
 
@@ -883,10 +883,12 @@ void engine_free(Engine *e) {
     free_wmat(e->head); free_wmat(e->pmp);
     cudaFree(e->rope_local); cudaFree(e->rope_global); cudaFree(e->part_ml);
     cudaFree(e->ple_table); cudaFree(e->out_norm); cudaFree(e->ple_proj_norm); cudaFree(e->rope_div);
+    cudaFree(e->sums);
     cudaFree(e->x); cudaFree(e->qkv); cudaFree(e->qrot); cudaFree(e->oout); cudaFree(e->gu); cudaFree(e->dout);
     cudaFree(e->hidden); cudaFree(e->h_prev); cudaFree(e->part); cudaFree(e->tokrow); cudaFree(e->pproj); cudaFree(e->ipl);
     cudaFree(e->pg); cudaFree(e->logits); cudaFree(e->amax_val); cudaFree(e->amax_idx);
     panel_free(e->p_ne); panel_free(e->p_attn); panel_free(e->p_ff); panel_free(e->p_ple);
+    cudaFreeHost(e->host_out);
     cudaFree(e->st); cudaFreeHost(e->st_host); cudaFree(e->log); cudaFree(e->replay); cudaFree(e->d_n_replay); cudaFree(e->err); cudaFree(e->tickets); cudaFree(e->d_margin_thr);
     free(e->pick_rows);
     cudaStreamDestroy(e->stream);
@@ -1219,17 +1221,20 @@ bool prefill_wide_ok(const Engine *e) {
 }
 
 // Run (capturing on first use) the forward graph for (M, flags).
-void run_forward(Engine *e, const struct kvcache *kv, int M, int flags) {
+// host_io: pos and toks of st_host enter and the state returns there with the status word, as parts of the graph
+void run_forward(Engine *e, const struct kvcache *kv, int M, int flags, bool host_io = false) {
     bind_kv(e, kv);
     char key[48];
-    snprintf(key, sizeof key, "f%d_%d", M, flags);
+    snprintf(key, sizeof key, "%c%d_%d", host_io ? 'i' : 'f', M, flags);
     auto it = e->graphs.find(key);
     if (it == e->graphs.end()) {
         e->launches = 0;
         cudaGraph_t graph;
         if ((flags & F_LOGITS) && !e->logits) e->logits = dalloc<float>((size_t)LG_MAXM * e->head.ldo);   // not inside capture
         LG_CHECK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed));
+        if (host_io) launch_k(e, lg_import_kernel, dim3(1), dim3(32), 0, e->st, (const volatile LgRoundState *)e->st_host, M);
         enqueue_forward(e, kv, M, flags);
+        if (host_io) launch_k(e, lg_export_state_kernel, dim3(1), dim3(32), 0, (int *)e->st_host, (const LgRoundState *)e->st, (const int *)e->err);
         LG_CHECK(cudaStreamEndCapture(e->stream, &graph));
         cudaGraphExec_t exec;
         LG_CHECK(cudaGraphInstantiate(&exec, graph, 0));
@@ -1237,6 +1242,40 @@ void run_forward(Engine *e, const struct kvcache *kv, int M, int flags) {
         it = e->graphs.emplace(key, exec).first;
     }
     LG_CHECK(cudaGraphLaunch(it->second, e->stream));
+}
+
+void report_err(int err);
+int host_status(const Engine *e) { return *(const int *)(e->st_host + 1); }       // behind the returned state
+
+// One token with its logits on the host (and the hidden row, where `hidden` is not null): one graph, one wait.
+void forward_host(Engine *e, const struct kvcache *kv, int token, int pos, int flags, float *logits, float *hidden) {
+    bind_kv(e, kv);
+    const int V = e->m->cfg.n_vocab, ne = e->m->cfg.n_embd, up = (V + 3) & ~3;
+    char key[48];
+    snprintf(key, sizeof key, "h%d", flags);
+    auto it = e->graphs.find(key);
+    if (it == e->graphs.end()) {
+        if (!e->logits) e->logits = dalloc<float>((size_t)LG_MAXM * e->head.ldo);          // not inside capture
+        if (!e->host_out) LG_CHECK(cudaMallocHost(&e->host_out, ((size_t)up + ne + 1) * sizeof(float)));
+        e->launches = 0;
+        cudaGraph_t graph;
+        LG_CHECK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed));
+        launch_k(e, lg_import_kernel, dim3(1), dim3(32), 0, e->st, (const volatile LgRoundState *)e->st_host, 1);
+        enqueue_forward(e, kv, 1, flags);
+        launch_k(e, lg_export_kernel, dim3(64), dim3(256), 0, e->host_out, (const float *)e->logits, V, (const float *)e->hidden, ne, (const int *)e->err);
+        LG_CHECK(cudaStreamEndCapture(e->stream, &graph));
+        cudaGraphExec_t exec;
+        LG_CHECK(cudaGraphInstantiate(&exec, graph, 0));
+        LG_CHECK(cudaGraphDestroy(graph));
+        it = e->graphs.emplace(key, exec).first;
+    }
+    e->st_host->pos = pos;
+    e->st_host->toks[0] = token;
+    LG_CHECK(cudaGraphLaunch(it->second, e->stream));
+    LG_CHECK(cudaStreamSynchronize(e->stream));
+    report_err(((const int *)e->host_out)[up + ne]);
+    memcpy(logits, e->host_out, (size_t)V * sizeof(float));
+    if (hidden) memcpy(hidden, e->host_out + up, (size_t)ne * sizeof(float));
 }
 
 // LG_MTP_PROFILE (any value, as in the reference: src/cuda/mtp-kernel.cuh:44-61,99-101): the verify forward runs
@@ -1276,10 +1315,13 @@ void lg::check_err(Engine *e) {
     int err = 0;
     LG_CHECK(cudaMemcpyAsync(&err, e->err, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
     LG_CHECK(cudaStreamSynchronize(e->stream));
+    report_err(err);
+}
+namespace {
+void report_err(int err) {
     if (err == LG_ERR_SEQ_POS) { fprintf(stderr, "lg_b200: a block started at a position whose sequence state is gone\n"); exit(1); }
     if (err) { fprintf(stderr, "lg_b200: device status %d (a bounded wait inside a kernel gave up)\n", err); exit(1); }
 }
-namespace {
 
 // ------------------------------------------------------------------------------------------
 // draft head
@@ -1476,9 +1518,19 @@ int spec_n(struct model *m, struct kvcache *kv, int n, const int *toks, int pos,
         }
         // other tokens than predicted (or a sampling hook): run the verify now; it overwrites the same cache rows
     }
-    upload_round(e, toks, n, pos);
     int flags = F_HEAD | F_ACCEPT | (model_pick ? F_LOGITS : 0);
     static const int profile = getenv("LG_MTP_PROFILE") != nullptr;
+    if (!model_pick && !(profile && n > 1)) {
+        e->st_host->pos = pos;
+        for (int j = 0; j < n; j++) e->st_host->toks[j] = toks[j];
+        run_forward(e, kv, n, flags, true);
+        LG_CHECK(cudaStreamSynchronize(e->stream));
+        report_err(host_status(e));
+        e->host_syncs++;
+        for (int j = 0; j < n; j++) out[j] = e->st_host->out[j];
+        return e->st_host->adv;
+    }
+    upload_round(e, toks, n, pos);
     if (profile && n > 1) run_forward_profiled(e, kv, n, flags);
     else run_forward(e, kv, n, flags);
     const struct config *c = &m->cfg;
@@ -1517,6 +1569,8 @@ cudaGraphExec_t round_graph(Engine *e, const struct kvcache *kv, DraftW *d, int 
         cudaGraph_t graph;
         e->launches = 0;
         LG_CHECK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed));
+        // a round that the host waits for takes its state from the pinned mirror and leaves the outcome there
+        if (!advance) launch_k(e, lg_import_state_kernel, dim3(1), dim3(32), 0, e->st, (const volatile int *)e->st_host);
         if (d) {
             for (int j = 1; j < n; j++) {
                 if (j >= 2 && !d->has_post) {           // no chaining: pad like the reference caller does
@@ -1528,6 +1582,7 @@ cudaGraphExec_t round_graph(Engine *e, const struct kvcache *kv, DraftW *d, int 
         }
         if (replay && n > 1) launch_k(e, lg_replay_drafts_kernel, dim3(1), dim3(32), 0, e->st, n, (const int *)e->replay, (const int *)e->d_n_replay);
         enqueue_forward(e, kv, n, F_HEAD | F_ACCEPT | (advance ? F_ADVANCE : 0));
+        if (!advance) launch_k(e, lg_export_state_kernel, dim3(1), dim3(32), 0, (int *)e->st_host, (const LgRoundState *)e->st, (const int *)e->err);
         LG_CHECK(cudaStreamEndCapture(e->stream, &graph));
         cudaGraphExec_t exec;
         LG_CHECK(cudaGraphInstantiate(&exec, graph, 0));
@@ -1637,11 +1692,9 @@ void model_forward(struct model *m, struct kvcache *kv, int token, int pos, floa
     Engine *e = engine_for(m);
     e->lazy.valid = false;
     if (!pos_in_cache(kv, pos, 1, "model_forward") || !can_start(e, kv, pos, 1, false, "model_forward")) exit(1);
+    if (logits) { forward_host(e, kv, token, pos, F_HEAD | F_LOGITS | F_ACCEPT, logits, m->last_hidden); return; }
     upload_round(e, &token, 1, pos);
-    run_forward(e, kv, 1, logits ? (F_HEAD | F_LOGITS | F_ACCEPT) : 0);
-    if (logits) LG_CHECK(cudaMemcpyAsync(logits, e->logits, (size_t)m->cfg.n_vocab * 4, cudaMemcpyDeviceToHost, e->stream));
-    if (logits && m->last_hidden)
-        LG_CHECK(cudaMemcpyAsync(m->last_hidden, e->hidden, (size_t)m->cfg.n_embd * 4, cudaMemcpyDeviceToHost, e->stream));
+    run_forward(e, kv, 1, 0);
     check_err(e);
 }
 
@@ -1676,6 +1729,9 @@ static void prefill_impl(struct model *m, struct kvcache *kv, const float *rows,
     }
     // the wide pass leaves no logits: with places asked for, it ends before the first of them
     const int n_all = n, n_wide = n_want > 0 ? std::min(n, want[0]) : n;
+    std::vector<std::vector<int>> gpos_all, toks_all, ridx_all;       // host staging of the wide blocks, alive until the last wait
+    std::vector<std::vector<float>> stage_all;
+    bool unchecked = n_want > 0;                                      // the status word is still to be looked at
     if (!e->fam && prefill_wide_ok(e) && n_wide >= 4 * LG_MAXM) {
         n = n_wide;
         // Blocks of up to LG_PF_MAXN tokens on the wide pass.  A ragged tail of more than one attention group is padded to
@@ -1684,8 +1740,6 @@ static void prefill_impl(struct model *m, struct kvcache *kv, const float *rows,
         // query can see them.  Host staging of every block stays alive until the single synchronisation at the end.
         bind_kv(e, kv);
         prefill_alloc(e);
-        std::vector<std::vector<int>> gpos_all, toks_all, ridx_all;
-        std::vector<std::vector<float>> stage_all;
         while (n - i > LG_MAXM) {                                    // a last group of <= 8 tokens is cheaper on the verify path
             int real = std::min(LG_PF_MAXN, n - i);
             int b = (real + LG_MAXM - 1) / LG_MAXM * LG_MAXM;
@@ -1720,8 +1774,8 @@ static void prefill_impl(struct model *m, struct kvcache *kv, const float *rows,
             enqueue_prefill_block(e, kv, b, C_ALL, blk_media);
             i += real;
         }
-        check_err(e);                                               // the one wait: every copy above has read its host buffer by now
         n = n_all;
+        unchecked = true;                                           // no wait here: a narrow step that follows has one
     }
     int w = 0;
     while (w < n_want && want[w] < i) w++;
@@ -1742,13 +1796,18 @@ static void prefill_impl(struct model *m, struct kvcache *kv, const float *rows,
                                              cudaMemcpyHostToDevice, e->stream));
         }
         const bool head = w < n_want && want[w] < i + b;
+        if (head && b == 1 && !blk_media) {
+            forward_host(e, kv, toks[i], pos0 + i, F_HEAD | F_LOGITS, logits + (size_t)w++ * n_vocab, nullptr);
+            unchecked = false;                                   // it has looked at the status word
+            continue;
+        }
         run_forward(e, kv, b, (blk_media ? F_NOEMBED : 0) | (head ? F_HEAD | F_LOGITS : 0));
         for (; w < n_want && want[w] < i + b; w++)
             LG_CHECK(cudaMemcpyAsync(logits + (size_t)w * n_vocab, e->logits + (size_t)(want[w] - i) * e->head.ldo, n_vocab * 4,
                                      cudaMemcpyDeviceToHost, e->stream));
         LG_CHECK(cudaStreamSynchronize(e->stream));      // st_host is reused by the next upload
     }
-    if (n_want > 0) check_err(e);
+    if (unchecked) check_err(e);
 }
 
 void model_prefill(struct model *m, struct kvcache *kv, const int *tokens, int n, int pos0) {
@@ -1801,11 +1860,10 @@ int mtp_draft_device(struct mtp *t, const struct model *m, const struct kvcache 
         // find their answers in it.
         memset(h, 0, sizeof *h);
         h->pos = pos; h->toks[0] = token; h->n_emitted = pos + e->replay_off;
-        LG_CHECK(cudaMemcpyAsync(e->st, h, sizeof *h, cudaMemcpyHostToDevice, e->stream));
         const bool replay = e->lazy_replay && e->replay != nullptr && e->n_replay > 0;
         LG_CHECK(cudaGraphLaunch(round_graph(e, kv, d, n, replay, false), e->stream));
-        LG_CHECK(cudaMemcpyAsync(h, e->st, sizeof *h, cudaMemcpyDeviceToHost, e->stream));
-        check_err(e);                                    // the one wait of this round
+        LG_CHECK(cudaStreamSynchronize(e->stream));      // the one wait of this round
+        report_err(host_status(e));
         e->host_syncs++;
         e->lazy.valid = true; e->lazy.n = n; e->lazy.pos = pos; e->lazy.adv = h->adv; e->lazy.chained = d->has_post != 0;
         for (int j = 0; j < n; j++) { e->lazy.toks[j] = h->toks[j]; e->lazy.out[j] = h->out[j]; }

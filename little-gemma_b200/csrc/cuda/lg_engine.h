@@ -137,7 +137,8 @@ struct Engine {
     int part_slots = 0;
     // session
     LgRoundState *st = nullptr;               // device
-    LgRoundState *st_host = nullptr;          // pinned mirror for uploads / downloads
+    LgRoundState *st_host = nullptr;          // pinned mirror for uploads / downloads; the status word behind it
+    float *host_out = nullptr;                // pinned: logits row, hidden row and status word of a forward for the host
     int *log = nullptr, *replay = nullptr, *d_n_replay = nullptr; int n_replay = 0, replay_cap = 0;   // replay table (capacity grows; its length lives on the device)
     int *err = nullptr, *tickets = nullptr;
     std::map<std::string, cudaGraphExec_t> graphs;

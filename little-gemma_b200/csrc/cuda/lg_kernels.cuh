@@ -1663,6 +1663,37 @@ __global__ void lg_accept_kernel(LgRoundState *st, int M, const float *__restric
     for (int i = threadIdx.x; i < ne; i += blockDim.x) h_prev[i] = src[i];
 }
 
+// The ends of a forward or round that the host waits for, as parts of its graph: position and tokens (or the whole state) come straight
+// out of the pinned mirror; state and status word, or logits, hidden row and status word, go straight into pinned memory.  Copies
+// through the copy engine, the last of them into pageable memory, cost 25 to 30 us a round and 65 to 80 us a token with logits.
+__global__ void lg_import_kernel(LgRoundState *st, const volatile LgRoundState *from, int n) {
+    pdl_launch(); pdl_wait();
+    if (threadIdx.x == 0) st->pos = from->pos;
+    if ((int)threadIdx.x < n) st->toks[threadIdx.x] = from->toks[threadIdx.x];
+}
+__global__ void lg_import_state_kernel(LgRoundState *st, const volatile int *from) {
+    pdl_launch(); pdl_wait();
+    if (threadIdx.x < sizeof(LgRoundState) / 4) ((int *)st)[threadIdx.x] = from[threadIdx.x];
+}
+// to: the state, then the status word
+__global__ void lg_export_state_kernel(int *to, const LgRoundState *st, const int *err) {
+    pdl_launch(); pdl_wait();
+    constexpr unsigned n = sizeof(LgRoundState) / 4;
+    static_assert(n < 32, "a warp copies the state");
+    if (threadIdx.x < n) to[threadIdx.x] = ((const int *)st)[threadIdx.x];
+    else if (threadIdx.x == n) to[n] = *err;
+}
+// to: [n_logits, rounded up to a multiple of 4] logits | [n_hidden] | status (16-byte aligned; the logits row too)
+__global__ void lg_export_kernel(float *__restrict__ to, const float *__restrict__ logits, int n_logits, const float *__restrict__ hidden, int n_hidden,
+                                 const int *__restrict__ err) {
+    pdl_launch(); pdl_wait();
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x, up = (n_logits + 3) & ~3;
+    for (int i = i0; i < n_logits / 4; i += step) ((float4 *)to)[i] = ((const float4 *)logits)[i];
+    for (int i = n_logits / 4 * 4 + i0; i < n_logits; i += step) to[i] = logits[i];
+    for (int i = i0; i < n_hidden; i += step) to[up + i] = hidden[i];
+    if (i0 == 0) ((int *)to)[up + n_hidden] = *err;
+}
+
 // drafts for the coming round: slot j <- replay[n_emitted + j - 1] (oracle-replayed drafts)
 __global__ void lg_replay_drafts_kernel(LgRoundState *st, int M, const int *__restrict__ replay, const int *__restrict__ n_replay) {
     pdl_launch(); pdl_wait();
