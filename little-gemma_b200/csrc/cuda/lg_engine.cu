@@ -1054,7 +1054,9 @@ void enqueue_forward(Engine *e, const struct kvcache *kv, int M, int flags, int 
 // ------------------------------------------------------------------------------------------
 // the wide prompt pass: blocks of up to LG_PF_MAXN tokens, matmuls on tcgen05
 // ------------------------------------------------------------------------------------------
-constexpr int PF_MAX_KS = 4;
+// Most k slices: every one gives a block of few tokens, which leaves SMs without an item, more of them, and costs its readers a plane (for
+// q/k/v every head's row).  E4B-class block of 45 tokens, at most 4 (q/k/v 2) slices 3182 us, 8 (4) 2986 us; of 90 tokens 3369 and 3211.
+constexpr int PF_MAX_KS = 8, PF_MAX_KS_QKV = 4;
 void prefill_alloc(Engine *e) {
     PrefillBuf &b = e->pf;
     if (b.ready) return;
@@ -1145,7 +1147,7 @@ void enqueue_prefill_block(Engine *e, const struct kvcache *kv, int n, int only 
         const int gqa = H / w.nkv;
         static const int block_attn = env_int("LG_PREFILL_BLOCK_ATTN", 1);
         const bool whole = block_attn && (hd == 64 || hd == 128 || hd == 256) && 32 % gqa == 0;
-        const int ks_q = whole ? pf_kslices(e, w.qkv, n, 2) : 1, ks_o = pf_kslices(e, w.o, n, PF_MAX_KS), ks_d = pf_kslices(e, w.down, n, PF_MAX_KS);
+        const int ks_q = whole ? pf_kslices(e, w.qkv, n, PF_MAX_KS_QKV) : 1, ks_o = pf_kslices(e, w.o, n, PF_MAX_KS), ks_d = pf_kslices(e, w.down, n, PF_MAX_KS);
         if (only & C_QKV) launch_pf_gemm(e, w.qkv, b.a_ne, LG_PF_MAXN, n, b.qkv, nullptr, 0, LG_PF_STORE, ks_q);
         if ((only & C_ATTN) && whole) {
             // the whole block at once: rows to the cache + f16 queries, then the tiled online-softmax kernel
