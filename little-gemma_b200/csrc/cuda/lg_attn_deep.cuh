@@ -21,7 +21,7 @@
 // dynamic smem (1024-byte aligned): K | V tile [HD/64][64][64] f16 swizzled | Qhi | Qlo [NQ16][HD+8] f16 | scores 2 x [NQ16][64] f32
 //               | Phi | Plo [NQ16][72] f16 | m, l, alpha [NQ16][3] | new K / V rows [2 LG_MAXM][HD] f16
 template <int HD>
-__global__ void __launch_bounds__(LG_ATTN_THREADS)
+__global__ void __launch_bounds__(LG_ATTN_THREADS, 2)
 lg_attn_deep_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constant__ CUtensorMap tmv, LgAttnArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ float s_qn[HD], s_kn[HD];
