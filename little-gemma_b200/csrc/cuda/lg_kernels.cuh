@@ -1666,13 +1666,17 @@ __global__ void lg_accept_kernel(LgRoundState *st, int M, const float *__restric
 // The ends of a forward or round that the host waits for, as parts of its graph: position and tokens (or the whole state) come straight
 // out of the pinned mirror; state and status word, or logits, hidden row and status word, go straight into pinned memory.  Copies
 // through the copy engine, the last of them into pageable memory, cost 25 to 30 us a round and 65 to 80 us a token with logits.
+// The two imports give no early trigger: the first attention reads the position before its own dependency wait (early_kv), and a
+// chain of kernels that all trigger at their start could bring it there before the position is in.  Without the trigger the next kernel
+// starts, and so every later one, when the import has finished.
 __global__ void lg_import_kernel(LgRoundState *st, const volatile LgRoundState *from, int n) {
-    pdl_launch(); pdl_wait();
+    pdl_wait();
     if (threadIdx.x == 0) st->pos = from->pos;
     if ((int)threadIdx.x < n) st->toks[threadIdx.x] = from->toks[threadIdx.x];
 }
 __global__ void lg_import_state_kernel(LgRoundState *st, const volatile int *from) {
-    pdl_launch(); pdl_wait();
+    static_assert(sizeof(LgRoundState) / 4 <= 32, "a warp copies the state");
+    pdl_wait();
     if (threadIdx.x < sizeof(LgRoundState) / 4) ((int *)st)[threadIdx.x] = from[threadIdx.x];
 }
 // to: the state, then the status word
