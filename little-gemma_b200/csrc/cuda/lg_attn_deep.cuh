@@ -159,7 +159,8 @@ lg_attn_deep_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
         #pragma unroll
         for (int n = 0; n < 4; n++) o[mt][n][0] = o[mt][n][1] = o[mt][n][2] = o[mt][n][3] = 0.0f;
 
-    // a tile's rows of the block's own positions go over whatever the copy brought for them
+    // a tile's rows of the block's own positions go over whatever the copy brought for them; rows of V behind the block become zeros
+    // (a cache that was used before may hold infinities there, and the product takes every row of the tile)
     auto patch = [&](int T, __half *tile, int isv) {
         for (int tok = warp; tok < a.M; tok += NW) {
             const int p = pos0 + tok;
@@ -245,6 +246,9 @@ lg_attn_deep_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
         }
         if (!mbar_wait(&vbar, parity) && a.err && lane == 0) atomicOr(a.err, LG_ERR_MBAR_TIMEOUT);
         if (writes_kv && pos0 + a.M > T * S && pos0 < (T + 1) * S) patch(T, sv, 1);
+        if (p_last + 1 < (T + 1) * S)
+            for (int i = threadIdx.x; i < (T * S + S - 1 - p_last) * (HD / 8); i += LG_ATTN_THREADS)
+                *(uint4 *)kv_at<S>(sv, p_last + 1 - T * S + i / (HD / 8), i % (HD / 8) * 8) = make_uint4(0, 0, 0, 0);
         __syncthreads();
         if (T == T0 + 2) LG_STAMP(a.tag, 3);
 
