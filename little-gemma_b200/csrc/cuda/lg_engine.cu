@@ -1804,6 +1804,7 @@ static void prefill_impl(struct model *m, struct kvcache *kv, const float *rows,
             unchecked = false;                                   // it has looked at the status word
             continue;
         }
+        unchecked |= n_want > 0;
         run_forward(e, kv, b, (blk_media ? F_NOEMBED : 0) | (head ? F_HEAD | F_LOGITS : 0));
         for (; w < n_want && want[w] < i + b; w++)
             LG_CHECK(cudaMemcpyAsync(logits + (size_t)w * n_vocab, e->logits + (size_t)(want[w] - i) * e->head.ldo, n_vocab * 4,

@@ -39,7 +39,7 @@ def test_span_merge(lg, depth):
                 g.prefill(toks[:depth], 0)
                 out.append(np.stack([g.forward(int(toks[depth + i]), depth + i) for i in range(4)]))
         finally:
-            lg.set_attn_deep(4096, 0)
+            lg.set_attn_deep(4097, 0)
     assert np.abs(out[0] - out[1]).max() / (out[0].max() - out[0].min()) < 1e-4
 
 
