@@ -566,8 +566,11 @@ void launch_attn(Engine *e, LgAttnArgs a, int n_tiles_max) {
 // in speculative decoding.  0 = the one-tile-per-CTA kernel.
 // Caches of up to 4096 rows keep the clusters (up to four tiles of 128 keys per CTA): a verify step of width 4 of the 12B-class
 // model takes 2.297 / 2.390 / 2.402 ms at 300 / 1024 / 2999 positions with them and 2.314 / 2.426 / 2.420 with spans.
+// Caches above that whose spans of two tiles would leave SMs idle take a cluster where one fits, spans of two where none does (`least`):
+// E4B-class (two KV heads) at 8192 positions, verify width 1 / 4 / 8 1.577 / 2.010 / 2.904 ms with one tile per CTA, 1.524 / 1.718 / 2.312 with
+// spans of two; at 4200 positions 1.523 / 1.734 / 2.358 with clusters, 1.544 / 1.737 / 2.298 with spans.
 int g_deep_min = -1, g_deep_force = 0;
-int deep_span_tiles(const Engine *e, int max_seq, int n_kv_heads, int hd, int nq) {
+int deep_span_tiles(const Engine *e, int max_seq, int n_kv_heads, int hd, int nq, int least = 0) {
     if (g_deep_min < 0) { g_deep_min = env_int("LG_ATTN_DEEP_MIN", 4097); g_deep_force = env_int("LG_ATTN_DEEP_G", 0); }
     static const int on = env_int("LG_ATTN_DEEP", 1);
     if (!on || max_seq < g_deep_min || (hd != 128 && hd != 256) || ((nq + 15) & ~15) > 32) return 0;
@@ -575,7 +578,7 @@ int deep_span_tiles(const Engine *e, int max_seq, int n_kv_heads, int hd, int nq
     const int tiles = (max_seq + LG_DEEP_S - 1) / LG_DEEP_S;
     const int want = std::max(1, 2 * e->sm_count / std::max(1, n_kv_heads));     // spans per KV head that fill the GPU once
     int G = (tiles + want - 1) / want;
-    return G < 2 ? 0 : std::min(G, 64);
+    return G < 2 ? least : std::min(G, 64);
 }
 
 void launch_attn_deep(Engine *e, LgAttnArgs a, int max_seq, int G) {
@@ -980,10 +983,11 @@ void enqueue_forward(Engine *e, const struct kvcache *kv, int M, int flags, int 
         static const int early_kv = env_int("LG_ATTN_EARLY_KV", 1);
         aa.early_kv = early_kv && w.owns_kv;     // the target's position and this layer's older rows come from earlier graph launches
         static const int deep_local = env_int("LG_ATTN_DEEP_LOCAL", 0);
-        const int deepG = w.local && (!deep_local || (aa.seq < kv->max_seq && aa.seq % LG_DEEP_S)) ? 0 :   // a tile must not straddle the ring's wrap
-                          deep_span_tiles(e, kv->max_seq, w.nkv, hd, (H / w.nkv) * LG_MAXM);
+        int deepG = w.local && (!deep_local || (aa.seq < kv->max_seq && aa.seq % LG_DEEP_S)) ? 0 :   // a tile must not straddle the ring's wrap
+                    deep_span_tiles(e, kv->max_seq, w.nkv, hd, (H / w.nkv) * LG_MAXM);
         if (only & C_ATTN) {
             const int cl = deepG ? 0 : attn_cluster_size(e, aa.window, kv->max_seq, aa.seq, hd, H, w.nkv);
+            if (!deepG && !cl && !w.local) deepG = deep_span_tiles(e, kv->max_seq, w.nkv, hd, (H / w.nkv) * LG_MAXM, 2);
             if (deepG) launch_attn_deep(e, aa, kv->max_seq, deepG);
             else if (cl) launch_attn_cluster(e, aa, cl);
             else launch_attn(e, aa, tiles_for(aa.window, kv->max_seq, M, hd));
@@ -1443,7 +1447,7 @@ void enqueue_draft(Engine *e, DraftW *d, const struct kvcache *kv, int slot, boo
         aa.out = pa; aa.out_f32 = nullptr;
         const int cl = attn_cluster_size(e, aa.window, kv->max_seq, aa.seq, hd, d->n_head, Hkv);
         // caches too long for one cluster per KV head: spans
-        const int deepG = cl || aa.window > 0 ? 0 : deep_span_tiles(e, kv->max_seq, Hkv, hd, d->n_head / Hkv);
+        const int deepG = cl || aa.window > 0 ? 0 : deep_span_tiles(e, kv->max_seq, Hkv, hd, d->n_head / Hkv, 2);
         if (cl) launch_attn_cluster(e, aa, cl);
         else if (deepG) launch_attn_deep(e, aa, kv->max_seq, deepG);
         else launch_attn(e, aa, tiles_for(aa.window, kv->max_seq, 1, hd));

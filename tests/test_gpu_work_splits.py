@@ -43,6 +43,30 @@ def test_span_merge(lg, depth):
     assert np.abs(out[0] - out[1]).max() / (out[0].max() - out[0].min()) < 1e-4
 
 
+@pytest.mark.parametrize("n", [4, 8])
+def test_spans_where_no_cluster_fits(lg, n):
+    """A cache too long for a cluster and too short for spans that fill the GPU: spans of two tiles against one tile per CTA, and a
+    speculative stream that equals the plain one."""
+    s = synth_module()
+    tp, _ = model_files("mid")
+    out = []
+    for min_seq in (4097, 1 << 30):
+        lg.set_attn_deep(min_seq, 0)
+        try:
+            with lg.Session(tp, None, 8300, mtp_n=n) as g:
+                prompt = s.prompt_ids(700, g.n_vocab, seed=63)
+                g.prefill(prompt[:-1], 0)
+                out.append(g.forward(int(prompt[-1]), len(prompt) - 1))
+        finally:
+            lg.set_attn_deep(4097, 0)
+    assert np.abs(out[0] - out[1]).max() / (out[0].max() - out[0].min()) < 1e-4        # as above
+    with lg.Session(tp, None, 8300, mtp_n=n) as g:
+        plain, _ = g.generate_device(prompt, 200, 0)
+    with lg.Session(tp, None, 8300, mtp_n=n) as g:
+        mtp, _ = g.generate_device(prompt, 200, 2, s.replay_drafts(plain, g.n_vocab, 0.7))
+    assert np.array_equal(plain[:200], mtp[:200])
+
+
 @pytest.mark.parametrize("m,k,n", [(2400, 150, 2000), (4128, 320, 2048), (2080, 64, 2300), (1312, 640, 4100)])
 def test_dense_prompt_matmul_of_several_tiles_per_cta(lg, m, k, n):
     """More tiles than CTAs, ragged in tokens and rows, fewer and more blocks of k than ring stages."""
