@@ -130,6 +130,9 @@ void  lg_engine_release(void);                       /* free all device state of
  * bit a production kernel's bounded wait would raise; returns the status word read back (1 = the wait ran out, as it must)
  * and clears it.  The device context stays usable: no trap, no fault, no endless loop. */
 int   lg_debug_bounded_wait(struct model *m, int polls);
+/* Edges from the kernels that bring a host-waited step's inputs in to the kernels behind them, over the graphs captured so far;
+ * *early: those over which a kernel may start before its inputs are in (always 0). */
+int   lg_debug_import_edges(struct model *m, int *early);
 /* Profiling builds only (-DLG_STAMPS): phase time stamps of the latest launches / clear them; -1 in the product build. */
 int   lg_debug_stamps(long long *out);
 int   lg_debug_clear_stamps(void);

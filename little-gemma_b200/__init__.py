@@ -30,7 +30,7 @@ ABI_SYMBOLS = [
     "lg_forward_spec_n", "lg_prefill_logits", "lg_set_compute_f32", "lg_set_replay", "lg_rounds_begin", "lg_rounds_enqueue", "lg_rounds_collect",
     "lg_set_round_width", "lg_set_replay_origin", "lg_host_syncs", "lg_set_draft_margin", "lg_drafts_skipped", "lg_weight_bytes", "lg_round_launches", "lg_last_hidden", "lg_kv_row", "lg_stream", "lg_engine_release",
     "lg_bench_matmul_pass", "lg_bench_prefill_pass", "lg_set_attn_deep", "lg_flash_decode_noalloc",
-    "lg_debug_bounded_wait", "lg_debug_stamps", "lg_debug_clear_stamps", "lg_matmul_resid_host",
+    "lg_debug_bounded_wait", "lg_debug_import_edges", "lg_debug_stamps", "lg_debug_clear_stamps", "lg_matmul_resid_host",
     "lg_dequant_host", "lg_gemv_host", "lg_flash_decode_host", "lg_flash_decode_cluster_host", "lg_prefill_matmul_host",
     "lg_dense_matmul_host", "lg_row_norm_host", "lg_latent_attn_host", "lg_latent_prompt_attn_host",
     "lg_dense_pair_host", "lg_row_norm_pair_host", "lg_mixer_blocks_host",
@@ -115,6 +115,7 @@ def load() -> C.CDLL:
     L.lg_set_draft_margin.argtypes = [C.c_void_p, C.c_float]; L.lg_set_draft_margin.restype = None
     L.lg_drafts_skipped.argtypes = [C.c_void_p]; L.lg_drafts_skipped.restype = C.c_longlong
     L.lg_debug_bounded_wait.argtypes = [C.c_void_p, C.c_int]; L.lg_debug_bounded_wait.restype = C.c_int
+    L.lg_debug_import_edges.argtypes = [C.c_void_p, _i32p]; L.lg_debug_import_edges.restype = C.c_int
     L.lgs_host_syncs.argtypes = [C.c_void_p]; L.lgs_host_syncs.restype = C.c_longlong
     L.lg_set_round_width.argtypes = [C.c_int]; L.lg_set_round_width.restype = None
     L.lg_set_replay_origin.argtypes = [C.c_void_p, C.c_int, C.c_int]; L.lg_set_replay_origin.restype = None

@@ -83,8 +83,9 @@ lg_attn_cluster_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_con
     if (!a.q_ready)
         for (int i = threadIdx.x; i < HD; i += LG_ATTN_THREADS) { s_qn[i] = a.q_norm[i]; s_kn[i] = a.k_norm ? a.k_norm[i] : 1.0f; }
     for (int qi = threadIdx.x; qi < nq16; qi += LG_ATTN_THREADS) ml[qi] = make_float2(-INFINITY, 0.0f);
-    // early_kv: the position and the cached rows below the block were written by earlier graph launches (this layer
-    // writes its own rows, and only here), so the first tile may start streaming before the previous kernel has finished
+    // early_kv: the cached rows below the block were written by earlier launches (this layer writes its own rows, and only
+    // here), the position by an earlier launch or by an import that ended before any other kernel of this graph began, so the
+    // first tile may start streaming before the previous kernel has finished
     if (!a.early_kv) pdl_wait();
     const int called_off = !a.early_kv && a.skip ? __ldcg(a.skip) : 0;      // read beside the position
     const int pos0 = __ldcg(a.pos);

@@ -56,7 +56,8 @@ __device__ __forceinline__ float gelu_tanh(float x) {
 // Programmatic dependent launch: every kernel of a forward may be started before its predecessor
 // has finished.  pdl_launch() lets the successor begin its own prologue; pdl_wait() blocks until the
 // predecessor grid has completed and its writes are visible.  Nothing produced by an earlier kernel
-// may be read, and nothing may be written, before pdl_wait().  (No-ops for a plain launch.)
+// may be read, and nothing may be written, before pdl_wait() -- an earlier kernel with a launch in between that was not allowed to
+// start early is none of these (launch_import).  (No-ops for a plain launch.)
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

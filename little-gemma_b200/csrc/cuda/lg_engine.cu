@@ -457,7 +457,7 @@ void launch_norm(Engine *e, int M, float *x, int ldx, int n, float eps,
         at[0].val.clusterDim.x = LG_NORM_CL; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = at; cfg.numAttrs = e->pdl ? 2 : 1;
+        cfg.attrs = at; cfg.numAttrs = early_start(e) ? 2 : 1;
         LG_CHECK(cudaLaunchKernelEx(&cfg, lg_norm_cluster_kernel, a));
         e->launches++;
         return;
@@ -687,7 +687,7 @@ void launch_attn_cluster(Engine *e, LgAttnArgs a, int C) {
     const int S = lg_attn_tile(a.hd);
     const CUtensorMap tmk = kv_tensor_map(a.kc, a.kv_dim, a.seq, S), tmv = kv_tensor_map(a.vc, a.kv_dim, a.seq, S);
     cudaLaunchConfig_t cfg; cudaLaunchAttribute at[2];
-    attn_cluster_config(cfg, at, a.Hkv, C, attn_cluster_smem(nq, a.hd), e->stream, e->pdl != 0);
+    attn_cluster_config(cfg, at, a.Hkv, C, attn_cluster_smem(nq, a.hd), e->stream, early_start(e));
     switch (a.hd) {
     case 64:  LG_CHECK(cudaLaunchKernelEx(&cfg, lg_attn_cluster_kernel<64>, tmk, tmv, a)); break;
     case 128: LG_CHECK(cudaLaunchKernelEx(&cfg, lg_attn_cluster_kernel<128>, tmk, tmv, a)); break;
@@ -981,7 +981,7 @@ void enqueue_forward(Engine *e, const struct kvcache *kv, int M, int flags, int 
         LgPanel pa = e->p_attn; pa.nsb = H * hd / 32;
         aa.out = pa;
         static const int early_kv = env_int("LG_ATTN_EARLY_KV", 1);
-        aa.early_kv = early_kv && w.owns_kv;     // the target's position and this layer's older rows come from earlier graph launches
+        aa.early_kv = early_kv && w.owns_kv;     // this layer's older rows come from earlier launches, the position too or from an import that has ended
         static const int deep_local = env_int("LG_ATTN_DEEP_LOCAL", 0);
         int deepG = w.local && (!deep_local || (aa.seq < kv->max_seq && aa.seq % LG_DEEP_S)) ? 0 :   // a tile must not straddle the ring's wrap
                     deep_span_tiles(e, kv->max_seq, w.nkv, hd, (H / w.nkv) * LG_MAXM);
@@ -1227,6 +1227,26 @@ bool prefill_wide_ok(const Engine *e) {
     return true;
 }
 
+// The first kernel of a graph that the host waits for: position and tokens, or the whole state, from the pinned mirror.  The kernel behind it
+// does not start before it has ended: an attention kernel further on reads the position before its own dependency wait (early_kv), and
+// only the end of a launch makes its stores visible to a kernel that has not waited for it.
+template <typename... KArgs, typename... Args>
+void launch_import(Engine *e, void (*kernel)(KArgs...), Args... args) {
+    launch_k(e, kernel, dim3(1), dim3(32), 0, args...);
+    e->hold_next = true;
+}
+// Edges out of the import of a captured graph (its only root), counted for lg_debug_import_edges.
+void count_import_edges(Engine *e, cudaGraph_t graph) {
+    cudaGraphNode_t root;
+    size_t n = 1;
+    LG_CHECK(cudaGraphGetRootNodes(graph, &root, &n));
+    LG_CHECK(cudaGraphNodeGetDependentNodes_v2(root, nullptr, nullptr, &n));
+    std::vector<cudaGraphNode_t> to(n);
+    std::vector<cudaGraphEdgeData> edge(n);
+    LG_CHECK(cudaGraphNodeGetDependentNodes_v2(root, to.data(), edge.data(), &n));
+    for (const auto &d : edge) { e->import_edges++; e->import_edges_early += d.type == cudaGraphDependencyTypeProgrammatic; }
+}
+
 // Run (capturing on first use) the forward graph for (M, flags).
 // host_io: pos and toks of st_host enter and the state returns there with the status word, as parts of the graph
 void run_forward(Engine *e, const struct kvcache *kv, int M, int flags, bool host_io = false) {
@@ -1239,10 +1259,11 @@ void run_forward(Engine *e, const struct kvcache *kv, int M, int flags, bool hos
         cudaGraph_t graph;
         if ((flags & F_LOGITS) && !e->logits) e->logits = dalloc<float>((size_t)LG_MAXM * e->head.ldo);   // not inside capture
         LG_CHECK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed));
-        if (host_io) launch_k(e, lg_import_kernel, dim3(1), dim3(32), 0, e->st, (const volatile LgRoundState *)e->st_host, M);
+        if (host_io) launch_import(e, lg_import_kernel, e->st, (const volatile LgRoundState *)e->st_host, M);
         enqueue_forward(e, kv, M, flags);
         if (host_io) launch_k(e, lg_export_state_kernel, dim3(1), dim3(32), 0, (int *)e->st_host, (const LgRoundState *)e->st, (const int *)e->err);
         LG_CHECK(cudaStreamEndCapture(e->stream, &graph));
+        if (host_io) count_import_edges(e, graph);
         cudaGraphExec_t exec;
         LG_CHECK(cudaGraphInstantiate(&exec, graph, 0));
         LG_CHECK(cudaGraphDestroy(graph));
@@ -1267,10 +1288,11 @@ void forward_host(Engine *e, const struct kvcache *kv, int token, int pos, int f
         e->launches = 0;
         cudaGraph_t graph;
         LG_CHECK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed));
-        launch_k(e, lg_import_kernel, dim3(1), dim3(32), 0, e->st, (const volatile LgRoundState *)e->st_host, 1);
+        launch_import(e, lg_import_kernel, e->st, (const volatile LgRoundState *)e->st_host, 1);
         enqueue_forward(e, kv, 1, flags);
         launch_k(e, lg_export_kernel, dim3(64), dim3(256), 0, e->host_out, (const float *)e->logits, V, (const float *)e->hidden, ne, (const int *)e->err);
         LG_CHECK(cudaStreamEndCapture(e->stream, &graph));
+        count_import_edges(e, graph);
         cudaGraphExec_t exec;
         LG_CHECK(cudaGraphInstantiate(&exec, graph, 0));
         LG_CHECK(cudaGraphDestroy(graph));
@@ -1577,7 +1599,7 @@ cudaGraphExec_t round_graph(Engine *e, const struct kvcache *kv, DraftW *d, int 
         e->launches = 0;
         LG_CHECK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed));
         // a round that the host waits for takes its state from the pinned mirror and leaves the outcome there
-        if (!advance) launch_k(e, lg_import_state_kernel, dim3(1), dim3(32), 0, e->st, (const volatile int *)e->st_host);
+        if (!advance) launch_import(e, lg_import_state_kernel, e->st, (const volatile int *)e->st_host);
         if (d) {
             for (int j = 1; j < n; j++) {
                 if (j >= 2 && !d->has_post) {           // no chaining: pad like the reference caller does
@@ -1591,6 +1613,7 @@ cudaGraphExec_t round_graph(Engine *e, const struct kvcache *kv, DraftW *d, int 
         enqueue_forward(e, kv, n, F_HEAD | F_ACCEPT | (advance ? F_ADVANCE : 0));
         if (!advance) launch_k(e, lg_export_state_kernel, dim3(1), dim3(32), 0, (int *)e->st_host, (const LgRoundState *)e->st, (const int *)e->err);
         LG_CHECK(cudaStreamEndCapture(e->stream, &graph));
+        if (!advance) count_import_edges(e, graph);
         cudaGraphExec_t exec;
         LG_CHECK(cudaGraphInstantiate(&exec, graph, 0));
         LG_CHECK(cudaGraphDestroy(graph));
@@ -2140,6 +2163,14 @@ int lg_debug_bounded_wait(struct model *m, int polls) {
     LG_CHECK(cudaMemsetAsync(e->err, 0, sizeof(int), e->stream));
     LG_CHECK(cudaStreamSynchronize(e->stream));
     return err;
+}
+
+// Edges from the imports of the graphs captured so far to the kernels behind them; *early: those over which a kernel may start before
+// its import has ended (none may).
+int lg_debug_import_edges(struct model *m, int *early) {
+    const Engine *e = engine_for(m);
+    *early = e->import_edges_early;
+    return e->import_edges;
 }
 
 void *lg_stream(struct model *m) { return (void *)engine_for(m)->stream; }

@@ -147,6 +147,8 @@ struct Engine {
     float *pick_rows = nullptr;               // host logits rows for model_pick
     long long launches = 0;                   // kernels enqueued by the most recent graph build
     int pdl = 1;                              // programmatic dependent launch (LG_PDL=0 turns it off)
+    bool hold_next = false;                   // the next launch starts only when its predecessor has ended (behind an import)
+    int import_edges = 0, import_edges_early = 0;   // edges out of captured imports; those that let the next kernel start early
     long long round_launches = 0;
     PrefillBuf pf;
     float4 *sums = nullptr;                   // SUMS epilogue: per work item and token the partial sums the next kernel builds the norms from
@@ -161,6 +163,12 @@ struct Engine {
     int mm_launches = 0;                      // kernels in the captured matmul-only pass             // kernels in one captured round (lg_rounds_enqueue)
 };
 
+// Whether the next launch may start before its predecessor has ended.
+inline bool early_start(Engine *e) {
+    const bool early = e->pdl && !e->hold_next;
+    e->hold_next = false;
+    return early;
+}
 // Kernel launch on the engine's stream, marked for programmatic dependent launch so the kernel may
 // start while its predecessor drains (every forward kernel begins with pdl_wait()).
 template <typename... KArgs, typename... Args>
@@ -170,7 +178,7 @@ void launch_k(Engine *e, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at; cfg.numAttrs = e->pdl ? 1 : 0;
+    cfg.attrs = at; cfg.numAttrs = early_start(e) ? 1 : 0;
     LG_CHECK(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
     e->launches++;
 }
@@ -184,7 +192,7 @@ void launch_k_cluster_y(Engine *e, void (*kernel)(KArgs...), dim3 grid, dim3 blo
     at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = grid.y; at[0].val.clusterDim.z = 1;
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at; cfg.numAttrs = e->pdl ? 2 : 1;
+    cfg.attrs = at; cfg.numAttrs = early_start(e) ? 2 : 1;
     LG_CHECK(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
     e->launches++;
 }

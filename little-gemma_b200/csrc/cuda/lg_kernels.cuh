@@ -1315,8 +1315,9 @@ __global__ void __launch_bounds__(LG_ATTN_THREADS) lg_attn_kernel(LgAttnArgs a) 
     LG_STAMP_KIND(a.tag, 5);
     if (!a.q_ready)
         for (int i = threadIdx.x; i < HD; i += LG_ATTN_THREADS) { s_qn[i] = a.q_norm[i]; s_kn[i] = a.k_norm ? a.k_norm[i] : 1.0f; }
-    // early_kv: the position and the cached rows below the block were written by earlier graph launches (this layer
-    // writes its own rows, and only here), so the tile may start streaming before the previous kernel has finished
+    // early_kv: the cached rows below the block were written by earlier launches (this layer writes its own rows, and only
+    // here), the position by an earlier launch or by an import that ended before any other kernel of this graph began, so the
+    // tile may start streaming before the previous kernel has finished
     if (!a.early_kv) pdl_wait();
     const int called_off = !a.early_kv && a.skip ? __ldcg(a.skip) : 0;      // read beside the position
     constexpr int S = lg_attn_tile(HD), LDH = HD + 8, LDP = S + 8, PER = HD / 64, HALF = HD / 2, NW = LG_ATTN_THREADS / 32;
@@ -1666,9 +1667,9 @@ __global__ void lg_accept_kernel(LgRoundState *st, int M, const float *__restric
 // The ends of a forward or round that the host waits for, as parts of its graph: position and tokens (or the whole state) come straight
 // out of the pinned mirror; state and status word, or logits, hidden row and status word, go straight into pinned memory.  Copies
 // through the copy engine, the last of them into pageable memory, cost 25 to 30 us a round and 65 to 80 us a token with logits.
-// The two imports give no early trigger: the first attention reads the position before its own dependency wait (early_kv), and a
-// chain of kernels that all trigger at their start could bring it there before the position is in.  Without the trigger the next kernel
-// starts, and so every later one, when the import has finished.
+// The two imports give no early trigger, and the kernel behind one is launched without leave to start early (launch_import): the first
+// attention reads the position before its own dependency wait (early_kv), and a launch's stores are visible to a kernel that has not
+// waited for it only where an edge without that leave lies in between.
 __global__ void lg_import_kernel(LgRoundState *st, const volatile LgRoundState *from, int n) {
     pdl_wait();
     if (threadIdx.x == 0) st->pos = from->pos;
