@@ -184,7 +184,8 @@ lg_attn_deep_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
         if (T == T0 + 2) LG_STAMP(a.tag, 1);
 
         // scores S^T = K Q^T: warp w holds keys [16 (w & 3), +16) as the tile's rows and half (w >> 2) of the head dims,
-        // 8 queries per column tile; the two halves land in two buffers the softmax adds
+        // 8 queries per column tile; the two halves land in two buffers the softmax adds.  A key that a query does not see is -inf in
+        // both: rows behind the block arrive as the cache holds them, and -inf plus what a NaN or an infinity of an earlier use makes is NaN
         {
             float c0[4][4], c1[4][4];
             #pragma unroll
@@ -219,7 +220,7 @@ lg_attn_deep_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
                     for (int h2 = 0; h2 < 2; h2++) {
                         const int key = kt * 16 + g + h2 * 8, p = T * S + key;
                         const float v = c0[n][h2 * 2 + e] + c1[n][h2 * 2 + e];
-                        dst[(size_t)qi * S + key] = (dh || (qi < nq && p >= lo && p <= pj)) ? v : -INFINITY;
+                        dst[(size_t)qi * S + key] = qi < nq && p >= lo && p <= pj ? v : -INFINITY;
                     }
                 }
             }

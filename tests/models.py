@@ -21,6 +21,9 @@ def shapes():
         "mid": (s.TargetShape(n_layer=6, n_embd=512, n_head=8, n_head_kv=2, head_dim=256, n_ff=2048, n_vocab=8192,
                               window=64, local_per_global=2, ple=0, q_norm_scale=256 ** -0.5),
                 s.HeadShape(n_layer=2, n_inner=256, n_head=8, n_ff=512), 5, 6),
+        # the same without sliding-window layers
+        "full": (s.TargetShape(n_layer=2, n_embd=512, n_head=8, n_head_kv=2, head_dim=256, n_ff=2048, n_vocab=8192,
+                               window=64, local_per_global=0, ple=0, q_norm_scale=256 ** -0.5), None, 32, 33),
         # q4_K weights (super-blocks of 256)
         "mid_k": (s.TargetShape(n_layer=3, n_embd=512, n_head=8, n_head_kv=2, head_dim=256, n_ff=2048, n_vocab=8192,
                                 window=64, local_per_global=2, ple=0, q_norm_scale=256 ** -0.5, wtype=s.Q4_K),
