@@ -222,6 +222,11 @@ lg_attn_cluster_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_con
                 }
                 __syncthreads();
             }
+            // rows of V behind the block hold what the cache holds there; their weights are zero, but zero times an infinity or a NaN of an
+            // earlier use is not.  The value product ends with the 32 keys that hold the last position, so only their rows become zeros.
+            if (p_last + 1 < (T + 1) * S)
+                for (int i = threadIdx.x; i < ((T * S - 1 - p_last) & 31) * (HD / 8); i += LG_ATTN_THREADS)
+                    *(uint4 *)kv_at<S>(sv, p_last + 1 - T * S + i / (HD / 8), i % (HD / 8) * 8) = make_uint4(0, 0, 0, 0);
             if (T == T_first) LG_STAMP(a.tag, 3);
 
             // ---- scores S^T = K Q^T: warp w < KW holds keys [16w, 16w + 16) as the tile's rows, 8 queries per column tile;
@@ -315,6 +320,7 @@ lg_attn_cluster_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_con
                 }
                 #pragma unroll
                 for (int k0 = 0; k0 < S; k0 += 32) {
+                    if (T * S + k0 > p_last) break;             // exact zeros from here on
                     uint32_t ph[4][4], pl[4][4];                // B operands: 8 queries x keys k0, +8, +16, +24 (hi and lo halves of P)
                     #pragma unroll
                     for (int n = 0; n < 4; n++) {

@@ -23,8 +23,8 @@ def _steps(g, prompt, spoil):
     return out
 
 
-# spans of two tiles of 64 keys
-@pytest.mark.parametrize("name,rows", [("full", 8300)])
+# spans of two tiles of 64 keys, a cluster's tiles of 128; sliding-window layers
+@pytest.mark.parametrize("name,rows", [("full", 8300), ("full", 4096), ("mid", 512)])
 @pytest.mark.parametrize("n", [40, 57])
 def test_rows_behind_a_block_are_not_seen(lg, name, rows, n):
     s = synth_module()
