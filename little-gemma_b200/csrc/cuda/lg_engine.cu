@@ -898,12 +898,22 @@ void engine_free(Engine *e) {
     delete e;
 }
 
+// Scratch for the partials of a draft head's attention; it grows with the longest cache the head has met.
+void draft_scratch(DraftW *d, const struct kvcache *kv) {
+    const int slots = tiles_for(0, kv->max_seq, 1, 512);        // the smallest tiles, so the most
+    if (slots <= d->n_slots_global) return;
+    cudaFree(d->part); cudaFree(d->part_ml);
+    d->n_slots_global = slots;
+    d->part = dalloc<float>((size_t)slots * d->n_head * d->hd_max);
+    d->part_ml = dalloc<float2>((size_t)slots * d->n_head);
+}
+
 // Scratch for the flash-decode partials depends on the cache geometry; (re)bind when the cache changes.
 void bind_kv(Engine *e, const struct kvcache *kv) {
     if (e->kv_bound == kv && (e->part || e->fam)) return;
     LG_CHECK(cudaStreamSynchronize(e->stream));
     free_graphs(e->graphs);
-    if (e->draft) free_graphs(e->draft->graphs);
+    if (e->draft) { free_graphs(e->draft->graphs); draft_scratch(e->draft, kv); }
     if (e->fam) { e->fam->bind(e, kv); e->kv_bound = kv; return; }
     const struct config *c = &e->m->cfg;
     int slots = 0, maxhd = 0;
@@ -1370,7 +1380,7 @@ DraftW *draft_build(Engine *e, struct mtp *t, const struct kvcache *kv) {
     d->has_post = t->post && t->post->n_dims == 2 && (int)t->post->dims[0] == t->n_inner && (int)t->post->dims[1] == t->n_bb;
     if (d->has_post) d->post = build_wmat(e, {t->post});
     d->out_norm = upload_f32(t->out_norm, d->ni);
-    int qmax = 0, maxhd = 0;
+    int qmax = 0;
     for (int L = 0; L < t->n_layer; L++) {
         const struct mtp_layer *s = &t->l[L];
         DraftBlockW b{};
@@ -1382,7 +1392,7 @@ DraftW *draft_build(Engine *e, struct mtp *t, const struct kvcache *kv) {
         b.out_scale = s->out_scale ? s->out_scale[0] : 1.0f;
         b.hd = s->hd; b.local = s->local; b.src = s->src;
         if (d->n_head * s->hd > qmax) qmax = d->n_head * s->hd;
-        if (s->hd > maxhd) maxhd = s->hd;
+        if (s->hd > d->hd_max) d->hd_max = s->hd;
         if (s->local) d->hd_local = s->hd; else d->hd_global = s->hd;
         d->blk.push_back(b);
         if (d->n_head % m->n_head_kv[s->src]) {
@@ -1400,10 +1410,7 @@ DraftW *draft_build(Engine *e, struct mtp *t, const struct kvcache *kv) {
     d->qbuf = dalloc<float>((size_t)LG_MAXM * (qmax + 64)); d->qrot = dalloc<float>(qmax);
     d->obuf = dalloc<float>((size_t)e->max_ks * LG_MAXM * (std::max(d->ni, d->nb) + 64));
     d->gu = dalloc<float>(32);
-    int slots = tiles_for(0, kv->max_seq, 1, 512);
-    d->n_slots_global = slots;
-    d->part = dalloc<float>((size_t)slots * d->n_head * maxhd);
-    d->part_ml = dalloc<float2>((size_t)slots * d->n_head);
+    draft_scratch(d, kv);
     d->amax_val = dalloc<float>((size_t)e->head_ctas * LG_MAXM); d->amax_idx = dalloc<int>((size_t)e->head_ctas * LG_MAXM);
     d->best = dalloc<int>(LG_MAXM);
     d->amax_val2 = dalloc<float>((size_t)e->head_ctas * LG_MAXM); d->margin = dalloc<float>(LG_MAXM);

@@ -92,8 +92,8 @@ struct DraftW {
     float *amax_val2 = nullptr, *margin = nullptr;      // runner-up logits per CTA; best - second best of the latest draft
     float2 *part_ml = nullptr;
     LgPanel p_cat{}, p_ni{}, p_attn{}, p_ff{};
-    float2 *rope_local = nullptr, *rope_global = nullptr; int hd_local = 0, hd_global = 0;
-    int n_slots_local = 0, n_slots_global = 0;
+    float2 *rope_local = nullptr, *rope_global = nullptr; int hd_local = 0, hd_global = 0, hd_max = 0;
+    int n_slots_global = 0;
     std::map<std::string, cudaGraphExec_t> graphs;
 };
 
