@@ -120,10 +120,10 @@ int   lg_bench_matmul_pass(struct model *m, int n, int classes);
 /* Enqueue the kernels of one wide prompt block of n <= 1024 tokens restricted to kernel classes
  * (<= 0: the four layer matmuls); returns the number of launches or -1.  Timing utility. */
 int   lg_bench_prefill_pass(struct model *m, int n, int classes);
-/* Long-context attention: caches of at least min_seq rows run full-attention layers through the
- * span kernel (G tiles of 64 keys per CTA, online softmax); force_g > 0 fixes G (tests), 0 derives it
- * from the cache length.  Default: min_seq 4097 (LG_ATTN_DEEP_MIN), G derived.  Set before the
- * session's first forward. */
+/* Long-context attention: full-attention layers of caches of at least min_seq rows run through the span kernel (G tiles of 64
+ * keys per CTA, online softmax) where spans of two tiles fill the GPU or no cluster holds the cache; force_g > 0 fixes G and
+ * takes spans in any case (tests), 0 derives it from the cache length.  min_seq < 0: back to the defaults (LG_ATTN_DEEP_MIN or
+ * 4097 rows, LG_ATTN_DEEP_G or derived).  Set before the session's first forward. */
 void  lg_set_attn_deep(int min_seq, int force_g);
 void  lg_engine_release(void);                       /* free all device state of the loaded model */
 /* Test entry: one CTA waits on a barrier nothing completes, gives up after `polls` polls (1 .. 2^20) and raises the status

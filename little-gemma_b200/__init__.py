@@ -276,9 +276,9 @@ def mixer_blocks(layer: PlanLayer, weights, rows, blocks, eps: float, max_seq: i
     return out
 
 
-def set_attn_deep(min_seq: int = 4096, force_g: int = 0) -> None:
-    """Caches of at least min_seq rows use the span attention kernel on full-attention layers (force_g > 0 fixes the
-    tiles per span).  Call before opening the Session it should apply to."""
+def set_attn_deep(min_seq: int = -1, force_g: int = 0) -> None:
+    """Caches of at least min_seq rows may use the span attention kernel on full-attention layers (force_g > 0 fixes the
+    tiles per span); without arguments, back to the default.  Call before opening the Session it should apply to."""
     load().lg_set_attn_deep(min_seq, force_g)
 
 

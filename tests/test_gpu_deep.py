@@ -16,7 +16,7 @@ TOL = 1e-2
 def deep(lg):
     lg.set_attn_deep(128, 3)            # spans of 3 x 64 keys on every full-attention layer
     yield lg
-    lg.set_attn_deep(4096, 0)
+    lg.set_attn_deep()
 
 
 @pytest.mark.parametrize("name", ["mid", "var"])
@@ -66,8 +66,29 @@ def test_span_attention_equals_tile_attention_stream(lg):
         with lg.Session(tp, None, 1024) as g:
             b, _ = g.generate_device(prompt, 300, 0)
     finally:
-        lg.set_attn_deep(4096, 0)
+        lg.set_attn_deep()
     same = int((a[:300] == b[:300]).sum())
     print(f"span vs tile kernel: {same}/300 tokens equal")
     first_diff = int(np.argmax(a[:300] != b[:300])) if same < 300 else 300
     assert first_diff >= 50                      # free-running streams may part ways late; early divergence would be a bug
+
+
+def test_default_threshold_comes_back(lg):
+    """Without arguments set_attn_deep restores the default.  A cache of 4096 rows of the 12B-class shape keeps its clusters there; spans
+    take one launch more on its one full-attention layer."""
+    tp, _ = model_files("b12_cut_cond")
+
+    def launches():
+        with lg.Session(tp, None, 4096) as g:
+            g.rounds_begin(5, 0, 1)
+            assert g.rounds_enqueue(1, 0, 1, use_head=False) == 0
+            g.rounds_collect(1, 0)
+            return g.round_launches()
+
+    want = launches()
+    lg.set_attn_deep(64)
+    try:
+        assert launches() == want + 1
+    finally:
+        lg.set_attn_deep()
+    assert launches() == want

@@ -59,13 +59,13 @@ def test_drafts_of_spans_equal_those_of_single_tiles(lg):
     s = synth_module()
     tp, hp = model_files("mid")
     out = []
-    for min_seq in (4097, 1 << 30):
+    for min_seq in (-1, 1 << 30):
         lg.set_attn_deep(min_seq, 0)
         try:
             with lg.Session(tp, hp, LONG, mtp_n=4) as g:
                 out.append(_drafts(g, s.prompt_ids(400, g.n_vocab, seed=92), PLACES))
         finally:
-            lg.set_attn_deep(4097, 0)
+            lg.set_attn_deep()
     assert out[0] == out[1]
     assert len({tuple(d) for d in out[0]}) > len(PLACES) // 2      # and they tell the places apart
 

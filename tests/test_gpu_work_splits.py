@@ -39,7 +39,7 @@ def test_span_merge(lg, depth):
                 g.prefill(toks[:depth], 0)
                 out.append(np.stack([g.forward(int(toks[depth + i]), depth + i) for i in range(4)]))
         finally:
-            lg.set_attn_deep(4097, 0)
+            lg.set_attn_deep()
     assert np.abs(out[0] - out[1]).max() / (out[0].max() - out[0].min()) < 1e-4
 
 
@@ -50,7 +50,7 @@ def test_spans_where_no_cluster_fits(lg, n):
     s = synth_module()
     tp, _ = model_files("mid")
     out = []
-    for min_seq in (4097, 1 << 30):
+    for min_seq in (-1, 1 << 30):
         lg.set_attn_deep(min_seq, 0)
         try:
             with lg.Session(tp, None, 8300, mtp_n=n) as g:
@@ -58,7 +58,7 @@ def test_spans_where_no_cluster_fits(lg, n):
                 g.prefill(prompt[:-1], 0)
                 out.append(g.forward(int(prompt[-1]), len(prompt) - 1))
         finally:
-            lg.set_attn_deep(4097, 0)
+            lg.set_attn_deep()
     assert np.abs(out[0] - out[1]).max() / (out[0].max() - out[0].min()) < 1e-4        # as above
     with lg.Session(tp, None, 8300, mtp_n=n) as g:
         plain, _ = g.generate_device(prompt, 200, 0)
