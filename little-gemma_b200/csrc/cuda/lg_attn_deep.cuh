@@ -8,8 +8,8 @@
 // CTA's tile load overlaps the other's math, and the merge runs over spans, G times fewer partials.
 //
 // Spans, like tiles, lie on ABSOLUTE position boundaries (span s = keys [s*G*64, (s+1)*G*64)), G is a
-// property of the session (the cache length), and a tile that is wholly outside a query's window is an
-// exact no-op for that query (weights 0, rescale 1).  So a query row's result depends on its own
+// property of the session (the cache length), and a tile that lies wholly behind a query is an exact
+// no-op for that query (weights 0, rescale 1).  So a query row's result depends on its own
 // position only -- not on the verify width or on which other rows share the launch -- which keeps the
 // speculative stream byte-identical to plain decoding.
 #pragma once
@@ -42,15 +42,11 @@ lg_attn_deep_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int pos0 = __ldcg(a.pos);
     if (called_off) return;
-    const int p_first = pos0 + a.qpos_off, p_last = pos0 + a.M - 1 + a.qpos_off;
+    const int p_last = pos0 + a.M - 1 + a.qpos_off;
     if (p_last < 0) return;
-    const int lo_first = a.window > 0 ? max(0, p_first + a.win_shrink - a.window + 1) : 0;
-    const int t_lo = lo_first / S, t_hi = p_last / S;
-    const int s_lo = t_lo / G, s_hi = t_hi / G;                 // spans the block touches
-    const int SP = s_lo + blockIdx.y;
-    if (SP > s_hi) return;
-    const int slot = SP % a.n_slots;
-    const int T0 = max(SP * G, t_lo), T1 = min(SP * G + G - 1, t_hi);
+    const int t_hi = p_last / S, SP = blockIdx.y, slot = SP % a.n_slots;      // last tile; this CTA's span
+    const int T0 = SP * G, T1 = min(T0 + G - 1, t_hi);
+    if (T0 > t_hi) return;
     const bool writes_kv = a.owns_kv && !a.q_ready;
 
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -215,12 +211,11 @@ lg_attn_deep_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
                 for (int e = 0; e < 2; e++) {
                     const int qi = n * 8 + t * 2 + e;
                     const int pj = pos0 + qi / gqa + a.qpos_off;
-                    const int lo = a.window > 0 ? max(0, pj + a.win_shrink - a.window + 1) : 0;
                     #pragma unroll
                     for (int h2 = 0; h2 < 2; h2++) {
                         const int key = kt * 16 + g + h2 * 8, p = T * S + key;
                         const float v = c0[n][h2 * 2 + e] + c1[n][h2 * 2 + e];
-                        dst[(size_t)qi * S + key] = qi < nq && p >= lo && p <= pj ? v : -INFINITY;
+                        dst[(size_t)qi * S + key] = qi < nq && p <= pj ? v : -INFINITY;
                     }
                 }
             }
@@ -317,7 +312,7 @@ lg_attn_deep_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_consta
 // round of loads: the partials (1 MB per KV head at 64 spans x 16 queries) are read by M H hd / 128 CTAs at once, where the last
 // CTA of the span kernel used to read them alone.  E4B-class, 8192 positions: attention of a verify step of width 1 / 4 / 8 356 / 742 /
 // 1295 us before, 291 / 457 / 724 with this merge and the tiled copies.  Which sums a span enters, and in which order, follows
-// from its absolute index alone; spans outside a query's window add exact zeros.
+// from its absolute index alone; spans behind a query add exact zeros.
 #define LG_MERGE_DIMS 128
 #define LG_MERGE_UNROLL 8
 __global__ void __launch_bounds__(256) lg_attn_merge_kernel(LgAttnArgs a) {
@@ -330,18 +325,15 @@ __global__ void __launch_bounds__(256) lg_attn_merge_kernel(LgAttnArgs a) {
     const int called_off = a.skip ? __ldcg(a.skip) : 0;
     const int S = LG_DEEP_S, G = a.G, pos0 = __ldcg(a.pos);
     if (called_off) return;
-    const int p_first = pos0 + a.qpos_off, p_last = pos0 + a.M - 1 + a.qpos_off, pj = p_first + tok;
+    const int pj = pos0 + tok + a.qpos_off, p_last = pos0 + a.M - 1 + a.qpos_off;
     if (p_last < 0) return;
-    const int s_lo = (a.window > 0 ? max(0, p_first + a.win_shrink - a.window + 1) : 0) / S / G, s_hi = p_last / S / G;
-    const int i0 = (a.window > 0 ? max(0, pj + a.win_shrink - a.window + 1) : 0) / S / G, i1 = pj >= 0 ? pj / S / G : -1;
+    const int s_hi = p_last / S / G, i1 = pj >= 0 ? pj / S / G : -1;      // last span of the block, of the query
     const size_t row = (size_t)tok * a.H + hq, slot = (size_t)a.M * a.H;
-    // spans part, part + 8, ... (absolute indices) belong to this warp
-    const int first = s_lo + ((part - s_lo) & 7);
     // largest score maximum over all spans of the query
     float mx = -INFINITY;
-    for (int s = s_lo + threadIdx.x; s <= s_hi; s += 256) {
+    for (int s = threadIdx.x; s <= s_hi; s += 256) {
         const float2 v = __ldcg(a.part_ml + (s % a.n_slots) * slot + row);
-        if (s >= i0 && s <= i1 && v.y > 0.0f) mx = fmaxf(mx, v.x);
+        if (s <= i1 && v.y > 0.0f) mx = fmaxf(mx, v.x);
     }
     mx = warp_max(mx);
     if (lane == 0) s_red[part] = mx;
@@ -350,7 +342,7 @@ __global__ void __launch_bounds__(256) lg_attn_merge_kernel(LgAttnArgs a) {
     for (int w = 0; w < 8; w++) mx = fmaxf(mx, s_red[w]);
     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float lsum = 0.0f;
-    for (int s = first; s <= s_hi; s += 8 * LG_MERGE_UNROLL) {
+    for (int s = part; s <= s_hi; s += 8 * LG_MERGE_UNROLL) {
         float4 v[LG_MERGE_UNROLL]; float2 m[LG_MERGE_UNROLL];
         #pragma unroll
         for (int j = 0; j < LG_MERGE_UNROLL; j++)
@@ -363,7 +355,7 @@ __global__ void __launch_bounds__(256) lg_attn_merge_kernel(LgAttnArgs a) {
         for (int j = 0; j < LG_MERGE_UNROLL; j++)
             if (s + 8 * j <= s_hi) {
                 const int sp = s + 8 * j;
-                const float w = (sp >= i0 && sp <= i1 && m[j].y > 0.0f) ? expf(m[j].x - mx) : 0.0f;
+                const float w = (sp <= i1 && m[j].y > 0.0f) ? expf(m[j].x - mx) : 0.0f;
                 lsum = fmaf(w, m[j].y, lsum);
                 acc.x = fmaf(w, v[j].x, acc.x); acc.y = fmaf(w, v[j].y, acc.y);
                 acc.z = fmaf(w, v[j].z, acc.z); acc.w = fmaf(w, v[j].w, acc.w);

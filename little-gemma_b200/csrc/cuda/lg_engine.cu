@@ -992,9 +992,7 @@ void enqueue_forward(Engine *e, const struct kvcache *kv, int M, int flags, int 
         aa.out = pa;
         static const int early_kv = env_int("LG_ATTN_EARLY_KV", 1);
         aa.early_kv = early_kv && w.owns_kv;     // this layer's older rows come from earlier launches, the position too or from an import that has ended
-        static const int deep_local = env_int("LG_ATTN_DEEP_LOCAL", 0);
-        int deepG = w.local && (!deep_local || (aa.seq < kv->max_seq && aa.seq % LG_DEEP_S)) ? 0 :   // a tile must not straddle the ring's wrap
-                    deep_span_tiles(e, kv->max_seq, w.nkv, hd, (H / w.nkv) * LG_MAXM);
+        int deepG = w.local ? 0 : deep_span_tiles(e, kv->max_seq, w.nkv, hd, (H / w.nkv) * LG_MAXM);
         if (only & C_ATTN) {
             const int cl = deepG ? 0 : attn_cluster_size(e, aa.window, kv->max_seq, aa.seq, hd, H, w.nkv);
             if (!deepG && !cl && !w.local) deepG = deep_span_tiles(e, kv->max_seq, w.nkv, hd, (H / w.nkv) * LG_MAXM, 2);
