@@ -145,6 +145,8 @@ int  lg_dequant_host(int type, const void *blocks, int n_rows, int k, float *out
 /* y[tok][row] = W x[tok] for tok < M <= 8 through the tile-major repack, the 16-bit activation
  * panel and the tensor-core kernel; W is m rows of file-format blocks (q4_0, q4_K, q8_0, q6_K, q5_K, q3_K). */
 int  lg_gemv_host(int type, const void *blocks, int m, int k, const float *x, int M, int kslices, float *y);
+/* Teams of consumers a CTA of that kernel has for an m x k matrix (q4_0, q4_K) and M rows of x, kslices 0: 1 or 2; -1: bad arguments. */
+int  lg_debug_matmul_teams(int type, int m, int k, int M);
 /* The decode step's "matmul + residual update + next norm" chain on caller data: o = W act (complete rows with the partial
  * sums of the norms, k slices reduced inside a thread-block cluster where the plan has them), then
  * xres = (xres + rmsnorm(o) add_w) * out_scale and y = rmsnorm(xres) norm_w (norm_w NULL: y = xres) by the residual kernel.

@@ -30,7 +30,7 @@ ABI_SYMBOLS = [
     "lg_forward_spec_n", "lg_prefill_logits", "lg_set_compute_f32", "lg_set_replay", "lg_rounds_begin", "lg_rounds_enqueue", "lg_rounds_collect",
     "lg_set_round_width", "lg_set_replay_origin", "lg_host_syncs", "lg_set_draft_margin", "lg_drafts_skipped", "lg_weight_bytes", "lg_round_launches", "lg_last_hidden", "lg_kv_row", "lg_stream", "lg_engine_release",
     "lg_bench_matmul_pass", "lg_bench_prefill_pass", "lg_set_attn_deep", "lg_flash_decode_noalloc",
-    "lg_debug_bounded_wait", "lg_debug_import_edges", "lg_debug_stamps", "lg_debug_clear_stamps", "lg_matmul_resid_host",
+    "lg_debug_bounded_wait", "lg_debug_import_edges", "lg_debug_matmul_teams", "lg_debug_stamps", "lg_debug_clear_stamps", "lg_matmul_resid_host",
     "lg_dequant_host", "lg_gemv_host", "lg_flash_decode_host", "lg_flash_decode_cluster_host", "lg_prefill_matmul_host",
     "lg_dense_matmul_host", "lg_row_norm_host", "lg_latent_attn_host", "lg_latent_prompt_attn_host",
     "lg_dense_pair_host", "lg_row_norm_pair_host", "lg_mixer_blocks_host",
@@ -86,6 +86,7 @@ def load() -> C.CDLL:
     L.lg_dequant_host.argtypes = [C.c_int, C.c_void_p, C.c_int, C.c_int, _f32p]; L.lg_dequant_host.restype = C.c_int
     L.lg_gemv_host.argtypes = [C.c_int, C.c_void_p, C.c_int, C.c_int, _f32p, C.c_int, C.c_int, _f32p]
     L.lg_gemv_host.restype = C.c_int
+    L.lg_debug_matmul_teams.argtypes = [C.c_int] * 4; L.lg_debug_matmul_teams.restype = C.c_int
     L.lg_matmul_resid_host.argtypes = [C.c_int, C.c_void_p, C.c_int, C.c_int, _f32p, C.c_int, _f32p, _f32p, C.c_float, C.c_void_p, C.c_float, _f32p]
     L.lg_matmul_resid_host.restype = C.c_int
     L.lg_prefill_matmul_host.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int, _f32p, C.c_int, _f32p]

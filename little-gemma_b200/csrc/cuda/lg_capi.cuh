@@ -69,6 +69,15 @@ extern "C" int lg_gemv_host(int type, const void *blocks, int m, int k, const fl
     return 0;
 }
 
+// How lg_gemv_host (kslices 0) cuts the product: teams of consumers per CTA.
+extern "C" int lg_debug_matmul_teams(int type, int m, int k, int M) {
+    if (M < 1 || M > LG_MAXM || m < 1 || k < 64 || k % 64 || (type != GGML_TYPE_Q4_0 && type != GGML_TYPE_Q4_K)) return -1;
+    WMat W;
+    W.fmt = type == GGML_TYPE_Q4_0 ? LG_FMT_Q4_0 : LG_FMT_Q4_K;
+    W.m = m; W.k = k; W.nkp = k / 64; W.n_row_tiles = ((m + 15) / 16 + 3) / 4 * 4; W.ldo = W.n_row_tiles * 16;
+    return plan_gemv(scratch_engine(), W, M > 4 ? 2 : 1, 0, false).teams;
+}
+
 // The matmul with complete rows + norm sums followed by the residual kernel, as the decode step chains them:
 //   o = W act;  xres' = (xres + rmsnorm(o) add_w) * out_scale;  y = rmsnorm(xres') norm_w   (norm_w may be NULL: y = xres')
 // act [M][k], xres [M][m] (updated in place), y [M][m].  Returns 1 when the k slices were reduced inside a cluster, 0 when one

@@ -9,13 +9,15 @@ from tests.test_gpu_prefill import _weights
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("wtype,m,k", [("q4_0", 9664, 2624), ("q4_K", 9664, 2816), ("q4_0", 2400, 4160), ("q4_0", 9664, 5120)])
+@pytest.mark.parametrize("wtype,m,k,teams", [("q4_0", 9664, 2624, 2), ("q4_K", 9664, 2816, 2), ("q4_0", 2400, 4160, 2), ("q4_0", 9664, 5120, 1)])
 @pytest.mark.parametrize("M", [5, 8])
-def test_two_teams_of_a_cta(lg, port_built, wtype, m, k, M):
-    """More items than SMs and two panels; 151 items leave the last team idle, 150 do not.  Rows equal the one-panel launch's."""
+def test_two_teams_of_a_cta(lg, port_built, wtype, m, k, teams, M):
+    """More items than SMs and two panels; 151 items leave the last team idle, 150 do not.  The panels of 5120 columns leave no room for a
+    second team.  Rows equal the one-panel launch's."""
     s = synth_module()
     rng = np.random.default_rng(m + k)
     raw, t, w = _weights(s, rng, wtype, m, k)
+    assert lg.load().lg_debug_matmul_teams(t, m, k, M) == teams and lg.load().lg_debug_matmul_teams(t, m, k, 4) == 1
     x = rng.standard_normal((M, k)).astype(np.float32)
     got = lg.gemv(t, raw, m, k, x)
     want = x.astype(np.float64) @ w.astype(np.float64).T
