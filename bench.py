@@ -291,7 +291,7 @@ def sweep(a, lg, synth, torch):
                      (f"; the tcgen05 layer matmuls of its {pf['matmul_block']['tokens']}-token block: {pf['matmul_block']['ms']:.2f} ms = "
                       f"{pf['matmul_block']['achieved']:.0f} TFLOP/s = {pf['matmul_block']['frac']:.3f} of the measured sustained "
                       f"bf16 peak." if "matmul_block" in pf else "."))
-    out = a.sweep_out or os.path.join(ROOT, "gpurun_out", f"sweep_{cfg}.md")
+    out = a.sweep_out or os.path.join(ROOT, "out", f"sweep_{cfg}.md")
     os.makedirs(os.path.dirname(out), exist_ok=True)
     with open(out, "w") as f:
         f.write("\n".join(lines) + "\n")

@@ -4,8 +4,8 @@
 // lets the last CTA of a KV head merge all tiles: right at a few thousand keys, but at 32K keys that
 // is 257 one-tile CTAs per head, one per SM at a time with its load and its math back to back, and a
 // 2 MB merge by a single CTA.  Here a CTA walks a SPAN of G consecutive tiles of 64 keys with an
-// online softmax (running max / sum per query, accumulators in registers), two CTAs fit an SM so one
-// CTA's tile load overlaps the other's math, and the merge runs over spans, G times fewer partials.
+// online softmax (running max / sum per query, accumulators in registers), the next tile's copies run
+// under the math, and the merge runs over spans, G times fewer partials.
 //
 // Spans, like tiles, lie on ABSOLUTE position boundaries (span s = keys [s*G*64, (s+1)*G*64)), G is a
 // property of the session (the cache length), and a tile that lies wholly behind a query is an exact
@@ -21,7 +21,8 @@
 // dynamic smem (1024-byte aligned): K | V tile [HD/64][64][64] f16 swizzled | Qhi | Qlo [NQ16][HD+8] f16 | scores 2 x [NQ16][64] f32
 //               | Phi | Plo [NQ16][72] f16 | m, l, alpha [NQ16][3] | new K / V rows [2 LG_MAXM][HD] f16
 // Bound by the instruction chain of a tile between its four block barriers; the copies run under it.  128 registers, so that two CTAs
-// share an SM (left alone, head size 256 takes 221 and one fits).  12B-class layer, 32768 positions, 4 x 16 query rows (268 MB of
+// share an SM (left alone, head size 256 takes 221 and one fits) -- up to 16 query rows: at head size 256 the shared memory of 17 to 32
+// (E4B-class, widths 5 to 8: 134 KB) leaves room for one.  12B-class layer, 32768 positions, 4 x 16 query rows (268 MB of
 // cache): 105 us with the merge by a last CTA and plain copies, 65 + 8 us now, 0.64 of the copy rate.
 template <int HD>
 __global__ void __launch_bounds__(LG_ATTN_THREADS, 2)

@@ -564,11 +564,16 @@ void launch_attn(Engine *e, LgAttnArgs a, int n_tiles_max) {
 // Long-context sessions: full-attention layers walk spans of G tiles of 64 keys per CTA (lg_attn_deep_kernel).
 // G is a property of the cache length alone, so every query position sees the same decomposition in plain and
 // in speculative decoding.  0 = the one-tile-per-CTA kernel.
-// Caches of up to 4096 rows keep the clusters (up to four tiles of 128 keys per CTA): a verify step of width 4 of the 12B-class
-// model takes 2.297 / 2.390 / 2.402 ms at 300 / 1024 / 2999 positions with them and 2.314 / 2.426 / 2.420 with spans.
-// Caches above that whose spans of two tiles would leave SMs idle take a cluster where one fits, spans of two where none does (`least`):
-// E4B-class (two KV heads) at 8192 positions, verify width 1 / 4 / 8 1.577 / 2.010 / 2.904 ms with one tile per CTA, 1.524 / 1.718 / 2.312 with
-// spans of two; at 4200 positions 1.523 / 1.734 / 2.358 with clusters, 1.544 / 1.737 / 2.298 with spans.
+// Clusters take up to four tiles of 128 keys per CTA (12B-class: 10 CTAs, 5120 rows; E4B-class: 16, 8192); one tile or two a CTA they are
+// the faster ones, three or four the slower.  Verify steps of width 1 / 4 / 8 in ms, clusters against spans:
+//   12B-class, 4096 rows, position 1000   2.303 2.354 3.129   2.351 2.400 3.171      position 3816   2.388 2.438 3.234   2.370 2.418 3.190
+//              4600 rows                  2.302 2.355 3.121   2.356 2.399 3.179               4320   2.419 2.471 3.277   2.378 2.422 3.216
+//              5100 rows                  2.332 2.410 3.232   2.360 2.417 3.206               4820   2.484 2.622 3.552   2.380 2.434 3.223
+//   E4B-class, 5000 rows                  1.510 1.703 2.262   1.549 1.740 2.278               4720   1.557 1.767 2.351   1.556 1.756 2.278
+//              8000 rows                  1.506 1.702 2.268   1.527 1.729 2.290               7720   1.573 1.797 2.398   1.535 1.744 2.287
+// So spans begin where clusters lose more behind a full cache than they gain before: above 4096 rows, if spans of two tiles fill the GPU.
+// Longer caches that would leave SMs idle (few KV heads) take a cluster where one fits (at 8000 rows spans of two would gain more behind a
+// full cache than clusters do before), and spans of two where none does (`least`): E4B-class at 8192 positions 1.577 / 2.010 / 2.904 ms with one tile per CTA, 1.524 / 1.718 / 2.312 with spans of two.
 int g_deep_min = -1, g_deep_force = 0;
 int deep_span_tiles(const Engine *e, int max_seq, int n_kv_heads, int hd, int nq, int least = 0) {
     if (g_deep_min < 0) { g_deep_min = env_int("LG_ATTN_DEEP_MIN", 4097); g_deep_force = env_int("LG_ATTN_DEEP_G", 0); }
@@ -576,7 +581,7 @@ int deep_span_tiles(const Engine *e, int max_seq, int n_kv_heads, int hd, int nq
     if (!on || max_seq < g_deep_min || (hd != 128 && hd != 256) || ((nq + 15) & ~15) > 32) return 0;
     if (g_deep_force > 0) return g_deep_force;
     const int tiles = (max_seq + LG_DEEP_S - 1) / LG_DEEP_S;
-    const int want = std::max(1, 2 * e->sm_count / std::max(1, n_kv_heads));     // spans per KV head that fill the GPU once
+    const int want = std::max(1, 2 * e->sm_count / std::max(1, n_kv_heads));     // spans per KV head that fill the GPU once, two CTAs an SM
     int G = (tiles + want - 1) / want;
     return G < 2 ? least : std::min(G, 64);
 }

@@ -407,7 +407,7 @@ struct LgStageMaps { CUtensorMap q, s, d, m; };
 // Bound by the issue slots of its consumer warps and the hand-over between launches, not by HBM: the same matrix 48 times (in L2)
 // takes 12.6 us where 48 cold ones take 13.4 (12B-class gate/up, 66 MB), without the arithmetic 11.5.  Hence addresses of the shared
 // window (generic ones cost 64-bit arithmetic per load), packed f32 operations, and registers for two CTAs an SM (left to itself
-// the compiler stopped at 56 and spilled): 14.3 -> 13.0 us, down 8.9 -> 8.5, qkv 6.1 -> 5.6, o 4.25 -> 4.04.
+// the compiler stopped at 56 and spilled): 14.35 -> 13.4 us cold, down 8.9 -> 8.6, qkv 6.1 -> 5.4, o 4.25 -> 4.0.
 // Two panels (5..8 tokens) of a 3840-column matrix leave room for one CTA per SM: then a CTA has two teams of consumers, each with a
 // producer, ring and items of its own, behind ONE panel.  Gate/up 23.9 -> 17.7 us, down 15.2 -> 10.8, qkv 8.9 -> 6.9, o 7.2 -> 5.2.  For one panel
 // two CTAs are as good or better (12B-class verify step of width 4: 2.35 against 2.40 ms).

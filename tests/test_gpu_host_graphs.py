@@ -23,3 +23,14 @@ def test_nothing_starts_before_an_import_has_ended(lg):
             edges.append(g.L.lg_debug_import_edges(g.model, early))
             assert early[0] == 0
         assert edges == [1, 2, 3, 4, 5]                          # every one of them began with an import
+
+
+@pytest.mark.parametrize("family", ["hybrid", "latent"])
+def test_nothing_starts_before_an_import_has_ended_in_plan_models(lg, family):
+    from tests import hybrid_models, latent_models
+    shape, _, path = hybrid_models.model("deep") if family == "hybrid" else latent_models.model("mixed")
+    toks = synth_module().prompt_ids(8, shape.vocab, seed=72)
+    early = np.full(1, -1, dtype=np.int32)
+    with lg.Session(path, None, 64, mtp_n=4) as g:
+        g.forward(int(toks[0]), 0), g.next(int(toks[1]), 1), g.spec(toks[2:6], 2)
+        assert g.L.lg_debug_import_edges(g.model, early) == 3 and early[0] == 0
